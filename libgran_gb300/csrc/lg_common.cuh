@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/libgran_gb300.h"
+#include "lg_exact_div.cuh"
 
 namespace lg {
 
@@ -29,14 +30,37 @@ __host__ __device__ __forceinline__ d3 mk3(double x, double y, double z) { retur
 __host__ __device__ __forceinline__ d3 add(d3 a, d3 b) { return mk3(a.x + b.x, a.y + b.y, a.z + b.z); }
 __host__ __device__ __forceinline__ d3 sub(d3 a, d3 b) { return mk3(a.x - b.x, a.y - b.y, a.z - b.z); }
 __host__ __device__ __forceinline__ d3 scl(double s, d3 a) { return mk3(s * a.x, s * a.y, s * a.z); }
-__host__ __device__ __forceinline__ d3 dvs(d3 a, double s) { return mk3(a.x / s, a.y / s, a.z / s); }
+// Correctly rounded quotient and root: on the device by lg_exact_div.cuh (integer pipes, the same
+// bits as the FP64 pipe's operations), on the host by the compiler's.
+__host__ __device__ __forceinline__ double ddiv(double a, double b) {
+#ifdef __CUDA_ARCH__
+    return xd::div(a, b);
+#else
+    return a / b;
+#endif
+}
+__host__ __device__ __forceinline__ double droot(double z) {
+#ifdef __CUDA_ARCH__
+    return xd::root(z);
+#else
+    return sqrt(z);
+#endif
+}
+__host__ __device__ __forceinline__ d3 dvs(d3 a, double s) {
+#ifdef __CUDA_ARCH__
+    const xd::Divisor d = xd::divisor(s);  // one reciprocal for the three quotients
+    return mk3(xd::quotient(a.x, d), xd::quotient(a.y, d), xd::quotient(a.z, d));
+#else
+    return mk3(a.x / s, a.y / s, a.z / s);
+#endif
+}
 __host__ __device__ __forceinline__ d3 neg(d3 a) { return mk3(-a.x, -a.y, -a.z); }
 __host__ __device__ __forceinline__ double dot(d3 a, d3 b) { return (a.x * b.x + a.y * b.y) + a.z * b.z; }
 __host__ __device__ __forceinline__ double sqn(d3 a) { return (a.x * a.x + a.y * a.y) + a.z * a.z; }
-__host__ __device__ __forceinline__ double nrm(d3 a) { return sqrt(sqn(a)); }
+__host__ __device__ __forceinline__ double nrm(d3 a) { return droot(sqn(a)); }
 __host__ __device__ __forceinline__ d3 nrmz(d3 a) {
     double z = sqn(a);
-    if (z > 0.0) return dvs(a, sqrt(z));
+    if (z > 0.0) return dvs(a, droot(z));
     return a;
 }
 __host__ __device__ __forceinline__ d3 crs(d3 a, d3 b) {
@@ -221,7 +245,7 @@ struct StateView {
 template <bool FAST>
 __device__ __forceinline__ d3 dvs_t(d3 a, double s) {
     if (FAST) {
-        const double r = 1.0 / s;
+        const double r = ddiv(1.0, s);
         return mk3(a.x * r, a.y * r, a.z * r);
     }
     return dvs(a, s);
@@ -229,7 +253,7 @@ __device__ __forceinline__ d3 dvs_t(d3 a, double s) {
 template <bool FAST>
 __device__ __forceinline__ d3 nrmz_t(d3 a) {
     const double z = sqn(a);
-    return z > 0.0 ? dvs_t<FAST>(a, sqrt(z)) : a;
+    return z > 0.0 ? dvs_t<FAST>(a, droot(z)) : a;
 }
 
 // contact_force.h:105-147
@@ -238,24 +262,23 @@ __device__ __forceinline__ d3 shear_coulomb(d3 &xi, d3 n, double stiffness, doub
                                             double mu_static, double phi_dynamic, d3 rel, double dt) {
     double mu_dynamic = mu_static * phi_dynamic;
     d3 xi_new = sub(xi, scl(dot(xi, n), n));
-    if (nrm(xi_new) > 0.0) {
-        double z = sqn(xi_new);
-        if (z > 0.0) xi_new = dvs_t<FAST>(xi_new, sqrt(z));
-        double old = nrm(xi);
-        xi_new = scl(old, xi_new);
+    const double z = sqn(xi_new);
+    if (z > 0.0) {  // (so is its root)
+        xi_new = dvs_t<FAST>(xi_new, droot(z));
+        xi_new = scl(nrm(xi), xi_new);
     }
     xi = xi_new;
     d3 f0 = sub(scl(-stiffness, xi), scl(damping, rel));
     double static_friction = mu_static * normal_force;
     double dynamic_friction = mu_dynamic * normal_force;
     double f0n = nrm(f0);
-    d3 t = (f0n > 0.0) ? (FAST ? dvs_t<true>(f0, f0n) : nrmz(f0)) : zero3();
+    d3 t = (f0n > 0.0) ? dvs_t<FAST>(f0, f0n) : zero3();
     double f_selected;
     if (f0n <= static_friction) {
         xi = add(xi, scl(dt, rel));
         f_selected = static_friction;
     } else {
-        xi = scl(-1.0 / stiffness, add(scl(dynamic_friction, t), scl(damping, rel)));
+        xi = scl(ddiv(-1.0, stiffness), add(scl(dynamic_friction, t), scl(damping, rel)));
         f_selected = dynamic_friction;
     }
     double m = (f0n < f_selected) ? f0n : f_selected;
@@ -266,11 +289,10 @@ __device__ __forceinline__ d3 shear_coulomb(d3 &xi, d3 n, double stiffness, doub
 template <bool FAST = false>
 __device__ __forceinline__ d3 shear_bond(d3 &xi, d3 n, double stiffness, double damping, d3 rel, double dt) {
     d3 xi_new = sub(xi, scl(dot(xi, n), n));
-    if (nrm(xi_new) > 0.0) {
-        double z = sqn(xi_new);
-        if (z > 0.0) xi_new = dvs_t<FAST>(xi_new, sqrt(z));
-        double old = nrm(xi);
-        xi_new = scl(old, xi_new);
+    const double z = sqn(xi_new);
+    if (z > 0.0) {  // (so is its root)
+        xi_new = dvs_t<FAST>(xi_new, droot(z));
+        xi_new = scl(nrm(xi), xi_new);
     }
     xi = xi_new;
     d3 f0 = sub(scl(-stiffness, xi), scl(damping, rel));
@@ -374,23 +396,8 @@ __device__ __forceinline__ double sq_(double x) { return x * x; }
 __device__ __forceinline__ double cb_(double x) { return x * x * x; }
 
 // hamaker_force.h:28-43 / limited_range_hamaker_force.h:33-45 / simplified_hamaker_force.h:23-29.
-// r = x_j - x_i. Angular part is zero. The limited variant's cutoff test is done by the caller.
-__device__ __forceinline__ d3 hamaker_accel(int mode, const lg_hamaker_params &p, d3 r) {
-    double h = nrm(r) - 2.0 * p.r_part;
-    if (h < p.h0) h = p.h0;
-    double rp = p.r_part;
-    double s;
-    if (mode == LG_HAMAKER_SIMPLIFIED) {
-        s = 2.0 * p.A * rp / sq_(h);
-    } else {
-        double br = (4.0 * rp + 2.0 * h) / (4.0 * rp + h) / h - 2.0 / (2.0 * rp + h) - 4.0 * sq_(rp) / cb_(2.0 * rp + h) -
-                    2.0 * sq_(rp) * (4.0 * rp + 2.0 * h) / sq_(4.0 * rp + h) / sq_(h);
-        s = -p.A / 6.0 * br;
-    }
-    return dvs(scl(s, nrmz(r)), p.mass);
-}
-
-// As hamaker_accel, with rn = nrm(r) already computed (the same value nrm() and nrmz() would compute).
+// r = x_j - x_i, rn = nrm(r) (which serves the cutoff test, h and the unit vector). Angular part is
+// zero. The limited variant's cutoff test is done by the caller.
 // FAST: the bracket over one common denominator, D = (4r + h) h (2r + h), with u = 1 / ((4r + h) h)
 // = (2r + h) / D and w = 1 / (2r + h) = (4r + h) h / D:
 //   (4r+2h) u - 2 w - 4 r^2 w^3 - 2 r^2 (4r+2h) u^2,
@@ -403,20 +410,21 @@ __device__ __forceinline__ d3 hamaker_accel_n(int mode, const lg_hamaker_params 
     double s;
     if (FAST && mode != LG_HAMAKER_SIMPLIFIED) {
         const double q = 4.0 * rp + h, w0 = 2.0 * rp + h, a = 4.0 * rp + 2.0 * h;
-        const double inv = 1.0 / (q * h * w0);
+        const double inv = ddiv(1.0, q * h * w0);
         const double u = w0 * inv, w = q * h * inv;
         const double br = a * u - 2.0 * w - 4.0 * sq_(rp) * (w * w * w) - 2.0 * sq_(rp) * a * (u * u);
-        s = -p.A / 6.0 * br;
-        return rn > 0.0 ? scl(s / (rn * p.mass), r) : dvs_t<true>(scl(s, r), p.mass);
+        s = ddiv(-p.A, 6.0) * br;
+        return rn > 0.0 ? scl(ddiv(s, rn * p.mass), r) : dvs_t<true>(scl(s, r), p.mass);
     }
     if (mode == LG_HAMAKER_SIMPLIFIED) {
-        s = 2.0 * p.A * rp / sq_(h);
+        s = ddiv(2.0 * p.A * rp, sq_(h));
     } else {
-        double br = (4.0 * rp + 2.0 * h) / (4.0 * rp + h) / h - 2.0 / (2.0 * rp + h) - 4.0 * sq_(rp) / cb_(2.0 * rp + h) -
-                    2.0 * sq_(rp) * (4.0 * rp + 2.0 * h) / sq_(4.0 * rp + h) / sq_(h);
-        s = -p.A / 6.0 * br;
+        const double a = 4.0 * rp + 2.0 * h, q = 4.0 * rp + h, w = 2.0 * rp + h;
+        double br = ddiv(ddiv(a, q), h) - ddiv(2.0, w) - ddiv(4.0 * sq_(rp), cb_(w)) -
+                    ddiv(ddiv(2.0 * sq_(rp) * a, sq_(q)), sq_(h));
+        s = ddiv(-p.A, 6.0) * br;
     }
-    if (FAST) return rn > 0.0 ? scl(s / (rn * p.mass), r) : dvs_t<true>(scl(s, r), p.mass);
+    if (FAST) return rn > 0.0 ? scl(ddiv(s, rn * p.mass), r) : dvs_t<true>(scl(s, r), p.mass);
     d3 u = (rn > 0.0) ? dvs(r, rn) : r;  // nrmz(r)
     return dvs(scl(s, u), p.mass);
 }
@@ -494,7 +502,7 @@ __device__ __forceinline__ d3 surface_hamaker(const lg_hamaker_params &p, d3 xf,
     d3 r = sub(xf, xi_);
     double h = nrm(r) - p.r_part;
     if (h < p.h0) h = p.h0;
-    double s = 2.0 * p.A / 3.0 * (cb_(p.r_part) / sq_(h) / sq_(h + 2.0 * p.r_part));
+    double s = ddiv(2.0 * p.A, 3.0) * ddiv(ddiv(cb_(p.r_part), sq_(h)), sq_(h + 2.0 * p.r_part));
     return dvs(scl(s, nrmz(r)), p.mass);
 }
 

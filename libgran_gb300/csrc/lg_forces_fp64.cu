@@ -166,10 +166,12 @@ __device__ __forceinline__ d3 slot_hamaker_fp64(const Params &P, const StateView
     const d3 xj = ld4(S.x, j);
     const d3 dx = sub(xi_, xj);
     d3 ha = zero3();
-    bool on = true;
-    if (hm == LG_HAMAKER_LIMITED) on = !(sqn(dx) > P.hamaker_skip_d2) && !(nrm(dx) > P.hamaker.r_cutoff);
-    if (on) ha = hamaker_accel(hm, P.hamaker, sub(xj, xi_));
-    return ha;
+    // |x_i - x_j| and |x_j - x_i| are the same value (the squares of negated differences are equal)
+    const double d2 = sqn(dx);
+    if (hm == LG_HAMAKER_LIMITED && d2 > P.hamaker_skip_d2) return ha;
+    const double rn = droot(d2);
+    if (hm == LG_HAMAKER_LIMITED && rn > P.hamaker.r_cutoff) return ha;
+    return hamaker_accel_n(hm, P.hamaker, sub(xj, xi_), rn);
 }
 
 // The pair value of a slot: binary + Hamaker as the reference's container adds them.
