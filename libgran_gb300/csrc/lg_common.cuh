@@ -285,21 +285,6 @@ __device__ __forceinline__ d3 shear_coulomb(d3 &xi, d3 n, double stiffness, doub
     return scl(m, t);
 }
 
-// alt_sinter_bridge.h:137-156
-template <bool FAST = false>
-__device__ __forceinline__ d3 shear_bond(d3 &xi, d3 n, double stiffness, double damping, d3 rel, double dt) {
-    d3 xi_new = sub(xi, scl(dot(xi, n), n));
-    const double z = sqn(xi_new);
-    if (z > 0.0) {  // (so is its root)
-        xi_new = dvs_t<FAST>(xi_new, droot(z));
-        xi_new = scl(nrm(xi), xi_new);
-    }
-    xi = xi_new;
-    d3 f0 = sub(scl(-stiffness, xi), scl(damping, rel));
-    xi = add(xi, scl(dt, rel));
-    return f0;
-}
-
 // FP64 overlap of a contact pair exactly as the FP64 path computes it (contact_force.h:65-66:
 // n = dx / |dx|, overlap = 2r - dx.n with dx = x_i - x_j), every operation rounded on its own.
 __device__ __forceinline__ double overlap_fp64(const dbl4 *x, int64_t i, int64_t j, double r) {
@@ -311,60 +296,6 @@ __device__ __forceinline__ double overlap_fp64(const dbl4 *x, int64_t i, int64_t
     const double nx = __ddiv_rn(dx, s), ny = __ddiv_rn(dy, s), nz = __ddiv_rn(dz, s);
     const double d = __dadd_rn(__dadd_rn(__dmul_rn(dx, nx), __dmul_rn(dy, ny)), __dmul_rn(dz, nz));
     return __dsub_rn(__dmul_rn(2.0, r), d);
-}
-
-// contact_force.h:57-96 -- the in-contact branch (caller has established overlap > 0 with the
-// reference's own arithmetic, n and overlap are passed in).
-template <bool FAST = false>
-__device__ __forceinline__ void contact_touching(const lg_contact_params &p, d3 n, double overlap, d3 vi, d3 vj,
-                                                 d3 wi, d3 wj, d3 *s, d3 &oa, d3 &oal) {
-    double rp = p.r_part - overlap / 2.0;
-    double v_n = -dot(sub(vi, vj), n);
-    double f_n = p.k * overlap + p.gamma_n * v_n;
-    d3 nwi = crs(n, wi), nwj = crs(n, wj);
-    d3 v_ij = add(add(sub(vi, vj), scl(rp, nwi)), scl(rp, nwj));
-    d3 v_t = sub(v_ij, scl(dot(v_ij, n), n));
-    d3 v_r = scl(-rp, sub(nwi, nwj));
-    d3 v_o = scl(p.r_part * (dot(n, wi) - dot(n, wj)), n);
-    d3 f_t = shear_coulomb<FAST>(s[0], n, p.k_t, p.gamma_t, f_n, p.mu_s, p.phi_d, v_t, p.dt);
-    d3 f_r = shear_coulomb<FAST>(s[1], n, p.k_r, p.gamma_r, f_n, p.mu_r, p.phi_r, v_r, p.dt);
-    d3 f_o = shear_coulomb<FAST>(s[2], n, p.k_o, p.gamma_o, f_n, p.mu_o, p.phi_o, v_o, p.dt);
-    d3 tau_t = scl(rp, crs(n, f_t));
-    d3 tau_r = scl(p.r_part, crs(n, f_r));
-    d3 tau_o = scl(p.r_part, f_o);
-    oa = dvs_t<FAST>(add(scl(f_n, n), f_t), p.mass);
-    oal = dvs_t<FAST>(add(add(neg(tau_t), tau_r), tau_o), p.inertia);
-}
-
-// alt_sinter_bridge.h:103-128 / alt_breaking_sinter_bridge.h:89-121. Returns true when the
-// breaking variant breaks the (i, j) bond (|f_tot| > strength, alt_breaking_sinter_bridge.h:118).
-template <bool FAST = false>
-__device__ __forceinline__ bool bond_force(const lg_sinter_params &p, d3 dx, d3 vi, d3 vj, d3 wi, d3 wj, d3 *s,
-                                           bool breaking, double strength, d3 &oa, d3 &oal) {
-    // the normal keeps the reference's division even in FAST: the overlap 2r - dx.n of a bonded pair
-    // is a small difference of large numbers, so an ulp of n is a large part of it
-    d3 n = nrmz(dx);
-    double overlap = 2.0 * p.r_part - dot(dx, n);
-    double rp = p.r_part - overlap / 2.0;
-    double v_n = -dot(sub(vi, vj), n);
-    double f_n = p.k * overlap + p.gamma_n * v_n;
-    d3 nwi = crs(n, wi), nwj = crs(n, wj);
-    d3 v_ij = add(add(sub(vi, vj), scl(rp, nwi)), scl(rp, nwj));
-    d3 v_t = sub(v_ij, scl(dot(v_ij, n), n));
-    d3 v_r = scl(-rp, sub(nwi, nwj));
-    d3 v_o = scl(p.r_part * (dot(n, wi) - dot(n, wj)), n);
-    d3 f_t = shear_bond<FAST>(s[0], n, p.k_t, p.gamma_t, v_t, p.dt);
-    d3 f_r = shear_bond<FAST>(s[1], n, p.k_r, p.gamma_r, v_r, p.dt);
-    d3 f_o = shear_bond<FAST>(s[2], n, p.k_o, p.gamma_o, v_o, p.dt);
-    d3 tau_t = scl(rp, crs(n, f_t));
-    d3 tau_r = scl(p.r_part, crs(n, f_r));
-    d3 tau_o = scl(p.r_part, f_o);
-    d3 f_tot = add(scl(f_n, n), f_t);
-    d3 tau_tot = add(add(neg(tau_t), tau_r), tau_o);
-    bool brk = breaking && (nrm(f_tot) > strength);
-    oa = dvs_t<FAST>(f_tot, p.mass);
-    oal = dvs_t<FAST>(tau_tot, p.inertia);
-    return brk;
 }
 
 // sinter_functor::bonded_contact_accelerations (sinter_bridge.h:238-266): five connector springs

@@ -12,13 +12,6 @@ namespace compact {
 constexpr int kWin = 4;           // slots per window (classified per memory round trip)
 constexpr int kHCap = 32 * kWin;  // Hamaker queue capacity per window
 
-// Slicing: the windows of a 32-row group may be split over SL warps (window w of a row goes to
-// warp w % SL); virtual slot v of slice sl (its windows sl, sl + SL, ...) -> slot of the row.
-template <int SL>
-__device__ __forceinline__ int64_t slot_of(int64_t v, int sl) {
-    return ((v / kWin) * SL + sl) * kWin + (v % kWin);
-}
-
 // Facet auto-move: the vertices one step ahead, written once per launch into the second vertex
 // buffer; the engine swaps the two buffers after the step.
 __device__ __forceinline__ void move_facets(const Params &P, const StateView &S, double dt) {

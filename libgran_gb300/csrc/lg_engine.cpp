@@ -379,11 +379,9 @@ int lg_system::alloc(U **p, size_t count) {
     return LG_OK;
 }
 
-// Pair slots up to which an FP64 system keeps the pair-parallel kernel's scratch (48 bytes a slot),
-// and up to which the automatic choice takes that kernel. Measured on GB300 (sinter + limited
-// Hamaker, FP64, graph-replayed steps): it leads the row-group and compacted kernels from 19
-// particles (37 vs 96 us a step) up to 8000 particles in Verlet mode (295 vs 313 us); the compacted
-// kernel keeps the large systems, where full warps and no divergence decide.
+// Pair slots up to which LG_FORCE_KERNEL_PAIRS may be asked for, and up to which the automatic choice
+// reports it. In FP64 it and LG_FORCE_KERNEL_COMPACT name the same pair kernels (lg_forces_pairs.cu),
+// whose block shape follows the size; both lead the row-group kernel at every size measured.
 constexpr int64_t kPairsMaxSlots = (int64_t)1 << 21;
 constexpr int64_t kPairsAutoSlots = (int64_t)1 << 19;
 
@@ -391,15 +389,14 @@ static int choose_kernel(const lg_system *s, int requested) {
     if (requested == LG_FORCE_KERNEL_ROWGROUP || requested == LG_FORCE_KERNEL_COMPACT) return requested;
     if (requested == LG_FORCE_KERNEL_PERSISTENT) return s->precision == LG_PRECISION_MIXED ? requested : -1;
     if (requested == LG_FORCE_KERNEL_FP64_FAST) return s->precision == LG_PRECISION_FP64 ? requested : -1;
-    if (requested == LG_FORCE_KERNEL_PAIRS) return s->pres ? requested : -1;
+    const bool pairs_ok = s->precision == LG_PRECISION_FP64 && (int64_t)s->pv[0].cap * s->P.n <= kPairsMaxSlots;
+    if (requested == LG_FORCE_KERNEL_PAIRS) return pairs_ok ? requested : -1;
     const int64_t n = s->P.n;
     // mixed precision: the compacted kernels at every size (their float-float completion and fused
     // runs of steps also make small systems fastest: 19 particles 13.7 against 36.9 us a step, 1000
     // particles 15.4 against 47.7 us, on GB300 with the row-group kernel)
     if (s->precision == LG_PRECISION_MIXED) return LG_FORCE_KERNEL_COMPACT;
-    if (s->pres && (int64_t)s->pv[0].cap * n <= kPairsAutoSlots) return LG_FORCE_KERNEL_PAIRS;
-    if (s->P.pairs == LG_PAIRS_VERLET ? n >= 1024 : n >= 4096) return LG_FORCE_KERNEL_COMPACT;
-    return LG_FORCE_KERNEL_ROWGROUP;
+    return (int64_t)s->pv[0].cap * n <= kPairsAutoSlots ? LG_FORCE_KERNEL_PAIRS : LG_FORCE_KERNEL_COMPACT;
 }
 
 static int choose_threads_per_row(const lg_system *s) {
@@ -410,6 +407,30 @@ static int choose_threads_per_row(const lg_system *s) {
     const int64_t len = s->P.pairs == LG_PAIRS_VERLET ? 32 : n - 1;
     while (T > 1 && T * 2 > len) T /= 2;
     return T;
+}
+
+// Scratch of the FP64 pair kernels (rec null: there is none).
+static PairScratch pair_scratch(const lg_system *s) {
+    PairScratch R{};
+    const int64_t slots = s->pv[0].cap * s->P.n;
+    double *base = s->P.pairs == LG_PAIRS_VERLET ? s->pv[1 - s->pcur].xi : s->pres;
+    if (!base) return R;
+    R.rec = reinterpret_cast<dbl4 *>(base);
+    R.tq = reinterpret_cast<dbl4 *>(base + 4 * slots);
+    R.q_n = s->d_queue_n;
+    if (s->P.pairs == LG_PAIRS_VERLET) {
+        // the list that is not current: 9 doubles a slot hold two records and an owner entry, its partner
+        // and flag arrays the contact queue
+        R.own = reinterpret_cast<uint2 *>(base + 8 * slots);
+        R.own_n = s->own_n;
+        R.rb = pair_block_rows(s->P.n);
+        R.q_i = s->pv[1 - s->pcur].nbr;
+        R.q_k = reinterpret_cast<int32_t *>(s->pv[1 - s->pcur].flags);
+    } else {
+        R.q_i = reinterpret_cast<int32_t *>(base + 8 * slots);
+        R.q_k = R.q_i + slots;
+    }
+    return R;
 }
 
 static int rebuild_list(lg_system *s) {
@@ -423,6 +444,10 @@ static int rebuild_list(lg_system *s) {
     s->launches += 9;
     s->pcur = 1 - s->pcur;
     s->list_built = true;
+    if (s->own_n) {
+        launch_pair_owners(s->P.n, s->pv[s->pcur], pair_scratch(s), s->stream);
+        s->launches += 1;
+    }
     LG_CUDA(cudaGetLastError());
     return LG_OK;
 }
@@ -449,6 +474,12 @@ static int ensure_step_buffers(lg_system *s) {
     s->step_slices = sl;
     s->fstep = 0;
     return LG_OK;
+}
+
+// Whether the handle's FP64 evaluations run the pair kernels.
+static bool pair_kernel(const lg_system *s) {
+    return s->precision == LG_PRECISION_FP64 && s->kernel != LG_FORCE_KERNEL_ROWGROUP &&
+           (s->P.pairs == LG_PAIRS_VERLET || s->pres);
 }
 
 static StateView state_view(lg_system *s, bool half_step_inputs) {
@@ -547,14 +578,12 @@ static int launch_forces(lg_system *s, double hdt, double dt, int move_facets, b
         else
             launch_forces_mixed(s->T, s->P, S, s->pv[s->pcur], s->bv, hdt, dt, move_facets, s->mx, s->stream);
     } else {
-        if (s->kernel == LG_FORCE_KERNEL_PAIRS)
-            kernels = launch_forces_pairs_fp64(s->P, S, s->pv[s->pcur], s->bv, s->pres, hdt, dt, move_facets,
-                                               fuse_kick, s->stream);
-        else if (compact || s->kernel == LG_FORCE_KERNEL_FP64_FAST)
-            launch_forces_compact_fp64(s->P, S, s->pv[s->pcur], s->bv, hdt, dt, move_facets, s->stream,
-                                       s->kernel == LG_FORCE_KERNEL_FP64_FAST);
-        else
-            launch_forces_fp64(s->T, s->P, S, s->pv[s->pcur], s->bv, hdt, dt, move_facets, s->stream);
+        if (pair_kernel(s))
+            kernels = launch_forces_pairs_fp64(s->P, S, s->pv[s->pcur], s->bv, pair_scratch(s), hdt, dt, move_facets,
+                                               fuse_kick, s->kernel == LG_FORCE_KERNEL_FP64_FAST, s->stream);
+        else  // (one lane per row where the pair kernels' scratch did not fit: the same bits)
+            launch_forces_fp64(s->kernel == LG_FORCE_KERNEL_ROWGROUP ? s->T : 1, s->P, S, s->pv[s->pcur], s->bv, hdt,
+                               dt, move_facets, s->stream);
     }
     s->launches += kernels;
     LG_CUDA(cudaGetLastError());
@@ -582,7 +611,7 @@ static int step_once(lg_system *s, double dt, int64_t rebuild_every, bool fuse_n
     const int mv = (s->facet_auto_move && s->P.n_facets > 0) ? 1 : 0;
     const bool fuse = fuse_next && ((s->precision == LG_PRECISION_MIXED && (s->kernel == LG_FORCE_KERNEL_COMPACT ||
                                                                             s->kernel == LG_FORCE_KERNEL_PERSISTENT)) ||
-                                    (s->precision == LG_PRECISION_FP64 && s->kernel == LG_FORCE_KERNEL_PAIRS));
+                                    pair_kernel(s));
     LG_TRY(launch_forces(s, hdt, dt, mv, fuse, prev_fused));
     s->kick_done = fuse;
     s->vcur = 1 - s->vcur;
@@ -1057,6 +1086,7 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
         LG_TRY(s->alloc(&s->ls.tile, (size_t)(s->max_cells / 4096 + 1)));
         LG_TRY(s->alloc(&s->ls.x32, (size_t)n));
         LG_TRY(s->alloc(&s->ls.max_row, 1));
+        if (s->precision == LG_PRECISION_FP64) LG_TRY(s->alloc(&s->own_n, (size_t)n / 4 + 1));
         LG_CUDA(cudaMemset(s->ls.max_row, 0, sizeof(int32_t)));
         LG_TRY(rebuild_list(s));
         // without an explicit max_neighbors the row capacity follows the initial state: rows get
@@ -1082,9 +1112,14 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
             LG_TRY(rebuild_list(s));
         }
     }
-    if (s->precision == LG_PRECISION_FP64 && (int64_t)s->pv[0].cap * n <= kPairsMaxSlots)
-        LG_TRY(s->alloc(&s->pres, 6 * (size_t)(s->pv[0].cap * n)));
+    if (s->precision == LG_PRECISION_FP64 && d->pairs == LG_PAIRS_ALL &&
+        s->alloc(&s->pres, 9 * (size_t)(s->pv[0].cap * n)) != LG_OK)
+        s->pres = nullptr;  // the row kernel then evaluates the pairs
     LG_TRY(s->alloc(&s->obs_scratch, (size_t)obs_scratch_doubles(n)));
+    if (s->precision == LG_PRECISION_FP64) {
+        LG_TRY(s->alloc(&s->d_queue_n, 1));
+        LG_CUDA(cudaMemset(s->d_queue_n, 0, sizeof(int32_t)));
+    }
     LG_TRY(s->alloc(&s->d_ticket, 1));
     LG_CUDA(cudaMemset(s->d_ticket, 0, sizeof(unsigned)));
     if (s->pooled) {  // plain host memory: freeing pinned memory can synchronise the device
@@ -2189,7 +2224,7 @@ static int apply_tuning(lg_system *s, const lg_tuning &t) {
     s->step_min_blocks = t.step_min_blocks;
     s->step_slices = t.step_slices;
     s->step_assign = t.step_assign;
-    if (t.force_kernel == LG_FORCE_KERNEL_PAIRS && !s->pres) return lg_fail(LG_E_INVALID, "tuning: no pair-parallel scratch");
+    if (t.force_kernel == LG_FORCE_KERNEL_PAIRS && choose_kernel(s, LG_FORCE_KERNEL_PAIRS) < 0) return lg_fail(LG_E_INVALID, "tuning: no pair-parallel scratch");
     s->kernel = t.force_kernel;
     if (compact_mixed(s, t.force_kernel))
         s->contact_lanes = t.threads_per_row == 1 ? 1 : 2;
@@ -2395,7 +2430,7 @@ extern "C" int lg_autotune(lg_system *s, double dt, int64_t probe_steps, int64_t
     const int sl0 = mixed_hamaker_slices(s->P.n);
     add(LG_FORCE_KERNEL_COMPACT, s->precision == LG_PRECISION_MIXED ? 2 : 1, 4, sl0, 0);
     if (s->precision == LG_PRECISION_MIXED) add(LG_FORCE_KERNEL_COMPACT, 1, 4, sl0, 0);  // one contact lane per row
-    if (s->pres) add(LG_FORCE_KERNEL_PAIRS, 1, 4, sl0, 0);
+    if (choose_kernel(s, LG_FORCE_KERNEL_PAIRS) > 0) add(LG_FORCE_KERNEL_PAIRS, 1, 4, sl0, 0);
     for (int T = 1; T <= 32; T *= 2) add(LG_FORCE_KERNEL_ROWGROUP, T, 4, sl0, 0);
     if (s->precision == LG_PRECISION_MIXED)
         for (int mb = 4; mb <= 6; ++mb)

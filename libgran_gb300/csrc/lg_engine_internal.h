@@ -67,7 +67,12 @@ struct lg_system {
     float4 *csum = nullptr;    // mixed: [3n] contact sums (float-float)
     float4 *hsum = nullptr;    // mixed: [2n] Hamaker sums (float-float)
     int32_t *d_flag = nullptr;  // mixed: device flag of the float-float copy check
-    double *pres = nullptr;     // FP64 pair-parallel kernel: per-slot pair values [6][cap * n]
+    // FP64 pair kernels. All pairs: per-slot records and the contact queue, 9 doubles a slot (null when
+    // they did not fit the device: the row kernel takes over). Verlet mode keeps them and the owned slots
+    // in the buffers of the list that is not current, which nothing reads between two list builds.
+    double *pres = nullptr;
+    int32_t *d_queue_n = nullptr;  // length of the contact queue (zero between evaluations)
+    int32_t *own_n = nullptr;   // Verlet: owned slots per block of rows
     unsigned *d_ticket = nullptr;  // zeroed counter of the reductions' last-block combine
     double *h_pin = nullptr;       // pinned host buffer (64 doubles) for small results read back
     uint8_t *d_hold = nullptr;  // [n] LG_HOLD_* bits (allocated on first use)

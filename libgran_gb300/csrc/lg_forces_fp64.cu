@@ -10,6 +10,7 @@
 // by one row group, so results are deterministic run to run.
 #include "lg_compact.cuh"
 #include "lg_kernels.h"
+#include "lg_pair_fp64.cuh"
 
 namespace lg {
 
@@ -17,38 +18,6 @@ namespace lg {
 // Kick + drift (first half of the rotational velocity-Verlet step):
 //   v += a*(dt/2); w += al*(dt/2); x += v*dt; th += w*dt
 // ------------------------------------------------------------------------------------------------
-// With connectors (BV.cn): the drift is sinter_step_handler's increment_x then increment_theta
-// (sinter_bridge.h:24-42, 55-75): the particle's connectors move with it by dx, then turn by
-// dtheta about its moved centre.
-// Drift of particle i with kicked velocities vi, wi (stored by the caller).
-// A held increment (LG_HOLD_X, LG_HOLD_THETA in `h`) is skipped together with its connector update.
-__device__ __forceinline__ void drift_one(int64_t n, int64_t i, dbl4 *__restrict__ x, dbl4 *__restrict__ th, d3 vi,
-                                          d3 wi, double dt, const BondView &BV, uint32_t h) {
-    const bool hx = h & LG_HOLD_X, hth = h & LG_HOLD_THETA;
-    const d3 dx = scl(dt, vi);
-    const d3 xn = hx ? ld4(x, i) : add(ld4(x, i), dx);
-    if (!hx) st4(x, i, xn);
-    const d3 dth = scl(dt, wi);
-    if (!hth) st4(th, i, add(ld4(th, i), dth));
-    if (BV.cn && !(hx && hth)) {
-        const int64_t bs = (int64_t)BV.bcap * n;
-        for (int b = 0; b < BV.bcap; ++b) {
-            const int64_t e = (int64_t)b * n + i;
-            if (BV.j[e] < 0) continue;
-#pragma unroll
-            for (int k = 0; k < 5; ++k) {
-                double *cx = BV.cn + (3 * k) * bs + e, *cy = BV.cn + (3 * k + 1) * bs + e, *cz = BV.cn + (3 * k + 2) * bs + e;
-                d3 c = mk3(*cx, *cy, *cz);
-                if (!hx) c = add(c, dx);
-                if (!hth) c = add(c, crs(dth, sub(c, xn)));
-                *cx = c.x;
-                *cy = c.y;
-                *cz = c.z;
-            }
-        }
-    }
-}
-
 __global__ void kick_drift_fp64(int64_t n, dbl4 *__restrict__ x, dbl4 *__restrict__ v,
                                 dbl4 *__restrict__ th, dbl4 *__restrict__ w, const dbl4 *__restrict__ a,
                                 const dbl4 *__restrict__ al, double dt, double hdt, BondView BV,
@@ -85,121 +54,6 @@ __device__ __forceinline__ double group_sum(double v) {
 #pragma unroll
     for (int o = T / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
-}
-
-// The binary functor's value for slot e of row i (P.binary_model != LG_BINARY_NONE); pair state
-// (springs, bond state, flags) of slot e is read and written here and nowhere else.
-__device__ __forceinline__ void slot_binary_fp64(const Params &P, const StateView &S, const PairView &PV,
-                                                 const BondView &BV, int64_t n, int64_t i, int64_t e, int64_t j,
-                                                 const d3 xi_, const d3 vi, const d3 wi, d3 &pa, d3 &pal) {
-    const int bm = P.binary_model;
-    const bool breaking = bm == LG_BINARY_BREAKING_SINTER;
-    const uint32_t fl = PV.flags[e];
-    const d3 xj = ld4(S.x, j);
-    const d3 dx = sub(xi_, xj);
-    pa = zero3();
-    pal = zero3();
-    {
-        if ((fl & kBonded) && BV.cn) {  // 5-connector model
-            const int64_t be = (int64_t)bond_slot_of(fl) * n + i;
-            const d3 vj = ld4(S.v, j), wj = ld4(S.w, j);
-            connector_force(P.connector, P.contact.r_part, P.contact.mass, P.contact.inertia, xi_, xj, vi, vj,
-                            wi, wj, BV.cn, (int64_t)BV.bcap * n, be, (int64_t)BV.rev[be] * n + j, pa, pal);
-        } else if (fl & kBonded) {
-            const int b = (int)bond_slot_of(fl);
-            const int64_t be = (int64_t)b * n + i;
-            const int64_t bs = (int64_t)BV.bcap * n;
-            d3 s[3];
-#pragma unroll
-            for (int q = 0; q < 3; ++q)
-                s[q] = mk3(BV.xi[(3 * q) * bs + be], BV.xi[(3 * q + 1) * bs + be], BV.xi[(3 * q + 2) * bs + be]);
-            const d3 vj = ld4(S.v, j), wj = ld4(S.w, j);
-            bool brk = bond_force(P.sinter, dx, vi, vj, wi, wj, s, breaking, breaking ? BV.strength[be] : 0.0, pa,
-                                  pal);
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                BV.xi[(3 * q) * bs + be] = s[q].x;
-                BV.xi[(3 * q + 1) * bs + be] = s[q].y;
-                BV.xi[(3 * q + 2) * bs + be] = s[q].z;
-            }
-            if (brk) {
-                BV.intact[be] = 0;
-                PV.flags[e] = fl & ~(kBonded | (0xffu << 8));
-            }
-        } else {
-            const int64_t xs = PV.cap * n;
-            bool touching = false;
-            d3 nn = zero3();
-            double overlap = 0.0;
-            if (!(sqn(dx) > P.contact_skip_d2)) {
-                nn = nrmz(dx);
-                overlap = 2.0 * P.contact.r_part - dot(dx, nn);
-                touching = !(overlap <= 0);
-            }
-            if (touching) {
-                d3 s[3] = {zero3(), zero3(), zero3()};  // springs of a slot that is not live are zero
-                if (fl & kXiLive)
-#pragma unroll
-                    for (int q = 0; q < 3; ++q)
-                        s[q] = mk3(PV.xi[(3 * q) * xs + e], PV.xi[(3 * q + 1) * xs + e], PV.xi[(3 * q + 2) * xs + e]);
-                const d3 vj = ld4(S.v, j), wj = ld4(S.w, j);
-                contact_touching(P.contact, nn, overlap, vi, vj, wi, wj, s, pa, pal);
-#pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    PV.xi[(3 * q) * xs + e] = s[q].x;
-                    PV.xi[(3 * q + 1) * xs + e] = s[q].y;
-                    PV.xi[(3 * q + 2) * xs + e] = s[q].z;
-                }
-                if (!(fl & kXiLive)) PV.flags[e] = fl | kXiLive;
-            } else if (fl & kXiLive) {  // reset_springs (contact_force.h:69,99-101)
-#pragma unroll
-                for (int q = 0; q < 9; ++q) PV.xi[q * xs + e] = 0.0;
-                PV.flags[e] = fl & ~kXiLive;
-            }
-        }
-    }
-}
-
-// The Hamaker term of the pair (i, j) (P.hamaker_model != LG_HAMAKER_NONE).
-__device__ __forceinline__ d3 slot_hamaker_fp64(const Params &P, const StateView &S, int64_t j, const d3 xi_) {
-    const int hm = P.hamaker_model;
-    const d3 xj = ld4(S.x, j);
-    const d3 dx = sub(xi_, xj);
-    d3 ha = zero3();
-    // |x_i - x_j| and |x_j - x_i| are the same value (the squares of negated differences are equal)
-    const double d2 = sqn(dx);
-    if (hm == LG_HAMAKER_LIMITED && d2 > P.hamaker_skip_d2) return ha;
-    const double rn = droot(d2);
-    if (hm == LG_HAMAKER_LIMITED && rn > P.hamaker.r_cutoff) return ha;
-    return hamaker_accel_n(hm, P.hamaker, sub(xj, xi_), rn);
-}
-
-// The pair value of a slot: binary + Hamaker as the reference's container adds them.
-__device__ __forceinline__ void combine_pair_fp64(bool have_binary, bool have_hamaker, const d3 &pb, const d3 &pbl,
-                                                  const d3 &ha, d3 &pa, d3 &pal) {
-    pa = pb;
-    pal = pbl;
-    if (have_hamaker) {
-        if (have_binary) {
-            pa = add(pa, ha);
-            pal = add(pal, zero3());
-        } else {
-            pa = ha;
-            pal = zero3();
-        }
-    }
-}
-
-// One slot of row i: the binary functor's pair value plus the Hamaker term, in that order (the
-// reference's container returns binary + hamaker for each pair, operator_overloads.h:16-20).
-__device__ __forceinline__ void slot_pair_fp64(const Params &P, const StateView &S, const PairView &PV,
-                                               const BondView &BV, int64_t n, int64_t i, int64_t e, int64_t j,
-                                               const d3 xi_, const d3 vi, const d3 wi, d3 &pa_out, d3 &pal_out) {
-    const bool hb = P.binary_model != LG_BINARY_NONE, hh = P.hamaker_model != LG_HAMAKER_NONE;
-    d3 pb = zero3(), pbl = zero3(), ha = zero3();
-    if (hb) slot_binary_fp64(P, S, PV, BV, n, i, e, j, xi_, vi, wi, pb, pbl);
-    if (hh) ha = slot_hamaker_fp64(P, S, j, xi_);
-    combine_pair_fp64(hb, hh, pb, pbl, ha, pa_out, pal_out);
 }
 
 template <int T, bool VERLET>
@@ -243,127 +97,6 @@ __global__ void __launch_bounds__(256) forces_fp64(Params P, StateView S, PairVi
     }
     if (!active || lane != 0) return;
     compact::finish_row(P, S, i, n, acc, accw, vi, wi, hdt);
-}
-
-// ------------------------------------------------------------------------------------------------
-// Pair-parallel evaluation for small systems (latency path)
-// ------------------------------------------------------------------------------------------------
-// A GB300 SM retires few FP64 instructions per clock, so a small system whose rows all sit on one
-// or two SMs spends its step waiting on those SMs' FP64 pipes while the rest of the GPU idles. Here
-// every slot (i, k) gets its own thread, in one-warp blocks that the block scheduler spreads over
-// all SMs; each thread writes its pair value (a, alpha: 6 doubles) to a slot-major scratch array.
-// A second kernel then adds each row's values in ascending slot order, exactly as the sequential
-// row loop adds them (so results match the T = 1 row kernel bit for bit), runs the facet terms
-// and the closing half kick and, when another step follows, the next step's kick and drift.
-constexpr int kPairBlock = 32;
-constexpr int kFoldBlock = 32;
-constexpr int kFoldRows = 5;    // rows per warp of the fold (six lanes each)
-constexpr int kFoldAhead = 8;   // slots whose pair terms a lane of the fold loads at once
-
-template <bool VERLET>
-__global__ void __launch_bounds__(kPairBlock) forces_pairs_fp64(Params P, StateView S, PairView PV, BondView BV,
-                                                                double *__restrict__ pres, int64_t ps, int64_t total) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= total) return;
-    const int64_t n = P.n;
-    const int64_t k = t / n, i = t - k * n;  // slot t = k * n + i
-    if (VERLET && k >= (int64_t)PV.row_len[i]) return;
-    const int64_t j = VERLET ? (int64_t)PV.nbr[t] : (k < i ? k : k + 1);
-    d3 pa, pal;
-    slot_pair_fp64(P, S, PV, BV, n, i, t, j, ld4(S.x, i), ld4(S.v, i), ld4(S.w, i), pa, pal);
-    pres[t] = pa.x;
-    pres[ps + t] = pa.y;
-    pres[2 * ps + t] = pa.z;
-    pres[3 * ps + t] = pal.x;
-    pres[4 * ps + t] = pal.y;
-    pres[5 * ps + t] = pal.z;
-}
-
-// The same slots with the binary functor and the Hamaker term in two warps of one block (warp 0:
-// binary, warp 1: Hamaker, 32 slots each): each warp issues only its own part's FP64 instructions,
-// which halves the longest instruction sequence a small system waits for. Warp 1 then adds the two
-// parts exactly as slot_pair_fp64 does.
-template <bool VERLET>
-__global__ void __launch_bounds__(2 * kPairBlock) forces_pairs_split_fp64(Params P, StateView S, PairView PV,
-                                                                          BondView BV, double *__restrict__ pres,
-                                                                          int64_t ps, int64_t total) {
-    __shared__ double part[6][kPairBlock];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t t = blockIdx.x * (int64_t)kPairBlock + lane;
-    const int64_t n = P.n;
-    const int64_t k = t / n, i = t - k * n;  // slot t = k * n + i
-    const bool live = t < total && (!VERLET || k < (int64_t)PV.row_len[i]);
-    const int64_t j = !live ? 0 : VERLET ? (int64_t)PV.nbr[t] : (k < i ? k : k + 1);
-    d3 pb = zero3(), pbl = zero3();
-    if (warp == 0) {
-        if (live) slot_binary_fp64(P, S, PV, BV, n, i, t, j, ld4(S.x, i), ld4(S.v, i), ld4(S.w, i), pb, pbl);
-        part[0][lane] = pb.x;
-        part[1][lane] = pb.y;
-        part[2][lane] = pb.z;
-        part[3][lane] = pbl.x;
-        part[4][lane] = pbl.y;
-        part[5][lane] = pbl.z;
-    }
-    d3 ha = zero3();
-    if (warp == 1 && live) ha = slot_hamaker_fp64(P, S, j, ld4(S.x, i));
-    __syncthreads();
-    if (warp != 1 || !live) return;
-    pb = mk3(part[0][lane], part[1][lane], part[2][lane]);
-    pbl = mk3(part[3][lane], part[4][lane], part[5][lane]);
-    d3 pa, pal;
-    combine_pair_fp64(true, true, pb, pbl, ha, pa, pal);
-    pres[t] = pa.x;
-    pres[ps + t] = pa.y;
-    pres[2 * ps + t] = pa.z;
-    pres[3 * ps + t] = pal.x;
-    pres[4 * ps + t] = pal.y;
-    pres[5 * ps + t] = pal.z;
-}
-
-template <bool VERLET, bool FACETS>
-__global__ void __launch_bounds__(kFoldBlock) fold_pairs_fp64(Params P, StateView S, PairView PV, BondView BV,
-                                                              const double *__restrict__ pres, int64_t ps, double hdt,
-                                                              double dt, int move_facets, int kick) {
-    const int64_t n = P.n;
-    if (move_facets && blockIdx.x == 0 && threadIdx.x == 0) compact::move_facets(P, S, dt);
-    // lane 6 r + c of a warp sums component c (force x, y, z, torque x, y, z) of the warp's row r:
-    // each component's terms in slot order, as one dependent chain per lane, so that a warp's FP64
-    // instructions each advance six chains of a row instead of one (FP64 issues slowly on this GPU).
-    // The loads of kFoldAhead slots are issued before their additions.
-    const int lane = threadIdx.x & 31;
-    const int64_t wg = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int r = lane / 6, c = lane % 6;
-    const int64_t i = wg * kFoldRows + r;
-    const bool mine = r < kFoldRows && i < n;
-    double sum = 0.0;
-    if (mine) {
-        const int64_t len = VERLET ? (int64_t)PV.row_len[i] : n - 1;
-        const double *col = pres + (int64_t)c * ps + i;
-        for (int64_t k = 0; k < len; k += kFoldAhead) {
-            double t[kFoldAhead];
-#pragma unroll
-            for (int u = 0; u < kFoldAhead; ++u) t[u] = k + u < len ? col[(k + u) * n] : 0.0;
-#pragma unroll
-            for (int u = 0; u < kFoldAhead; ++u)
-                if (k + u < len) sum += t[u];  // (adding a padding zero could turn -0 into +0)
-        }
-    }
-    double f[6];
-    const int src = r < kFoldRows ? 6 * r : 0;
-#pragma unroll
-    for (int q = 0; q < 6; ++q) f[q] = __shfl_sync(0xffffffffu, sum, src + q);
-    if (!mine || c != 0) return;
-    d3 acc = mk3(f[0], f[1], f[2]), accw = mk3(f[3], f[4], f[5]);
-    const d3 vi = ld4(S.v, i), wi = ld4(S.w, i);
-    compact::finish_row<FACETS>(P, S, i, n, acc, accw, vi, wi, hdt);
-    if (kick) {  // the next step's opening half kick and drift, as kick_drift_fp64
-        const uint32_t h = hold_of(P.hold, i);
-        const d3 v2 = kick_unless(kick_unless(vi, hdt, acc, h & LG_HOLD_V), hdt, acc, h & LG_HOLD_V);
-        const d3 w2 = kick_unless(kick_unless(wi, hdt, accw, h & LG_HOLD_OMEGA), hdt, accw, h & LG_HOLD_OMEGA);
-        st4(S.v_out, i, v2);
-        st4(S.w_out, i, w2);
-        drift_one(n, i, S.x, S.th, v2, w2, dt, BV, h);
-    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -944,41 +677,6 @@ void launch_forces_fp64(int T, const Params &P, const StateView &S, const PairVi
             launch_forces_t<1, false>(P, S, PV, BV, hdt, dt, move_facets, st);
     }
 #undef LG_CASE
-}
-
-int launch_forces_pairs_fp64(const Params &P, const StateView &S, const PairView &PV, const BondView &BV,
-                             double *pres, double hdt, double dt, int move_facets, bool kick, cudaStream_t st) {
-    const int64_t n = P.n;
-    const bool verlet = P.pairs == LG_PAIRS_VERLET;
-    const int64_t ps = (int64_t)PV.cap * n;
-    const int64_t total = (verlet ? (int64_t)PV.cap : n - 1) * n;
-    if (total > 0) {
-        const int64_t blocks = (total + kPairBlock - 1) / kPairBlock;
-        const bool split = P.binary_model != LG_BINARY_NONE && P.hamaker_model != LG_HAMAKER_NONE;
-        if (split && verlet)
-            forces_pairs_split_fp64<true><<<(unsigned)blocks, 2 * kPairBlock, 0, st>>>(P, S, PV, BV, pres, ps, total);
-        else if (split)
-            forces_pairs_split_fp64<false><<<(unsigned)blocks, 2 * kPairBlock, 0, st>>>(P, S, PV, BV, pres, ps, total);
-        else if (verlet)
-            forces_pairs_fp64<true><<<(unsigned)blocks, kPairBlock, 0, st>>>(P, S, PV, BV, pres, ps, total);
-        else
-            forces_pairs_fp64<false><<<(unsigned)blocks, kPairBlock, 0, st>>>(P, S, PV, BV, pres, ps, total);
-    }
-    const unsigned fb = (unsigned)((n + kFoldRows - 1) / kFoldRows);  // one warp per kFoldRows rows
-    const int kk = kick ? 1 : 0;
-    const bool unary = P.n_facets > 0 || P.ext_a;
-    if (verlet) {
-        if (unary)
-            fold_pairs_fp64<true, true><<<fb, kFoldBlock, 0, st>>>(P, S, PV, BV, pres, ps, hdt, dt, move_facets, kk);
-        else
-            fold_pairs_fp64<true, false><<<fb, kFoldBlock, 0, st>>>(P, S, PV, BV, pres, ps, hdt, dt, move_facets, kk);
-    } else {
-        if (unary)
-            fold_pairs_fp64<false, true><<<fb, kFoldBlock, 0, st>>>(P, S, PV, BV, pres, ps, hdt, dt, move_facets, kk);
-        else
-            fold_pairs_fp64<false, false><<<fb, kFoldBlock, 0, st>>>(P, S, PV, BV, pres, ps, hdt, dt, move_facets, kk);
-    }
-    return total > 0 ? 2 : 1;
 }
 
 void launch_body_central(int64_t n, const dbl4 *x, const int32_t *agg, const double *centre, double kam, dbl4 *ea,

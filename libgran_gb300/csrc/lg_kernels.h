@@ -41,11 +41,26 @@ struct ListScratch {
 // FP64 path (lg_forces_fp64.cu, compiled with --fmad=false)
 void launch_forces_fp64(int T, const Params &P, const StateView &S, const PairView &PV, const BondView &BV, double hdt,
                         double dt, int move_facets, cudaStream_t st);
-// Pair-parallel FP64 evaluation for small systems: per-slot pair values into pres [6][PV.cap * n],
-// then an ordered per-row fold; kick: also runs the next step's half kick and drift. Returns the
-// number of kernels launched.
+// FP64 evaluation over unordered pairs (lg_forces_pairs.cu): scratch of the pair kernels.
+struct PairScratch {
+    dbl4 *rec;       // [cap * n] per slot: force part of the pair value, w: 1 when it has a torque part
+    dbl4 *tq;        // [cap * n] per slot: torque part (written where rec's w is 1)
+    uint2 *own;      // Verlet: [cap * n] owned slots of each block of rb rows (the block's from row0 * cap on)
+    int32_t *own_n;  // Verlet: [ceil(n / rb)] owned slots per block
+    int32_t rb;      // rows per block of owned slots
+    // contact queue: slots (row, slot in the row) to evaluate, and their number (zero between evaluations)
+    int32_t *q_i, *q_k;  // [cap * n]
+    int32_t *q_n;
+};
+int32_t pair_block_rows(int64_t n);
+// Lists the owned slots of every block (Verlet mode; after each list build).
+void launch_pair_owners(int64_t n, const PairView &PV, const PairScratch &R, cudaStream_t st);
+// Per-slot pair values into the scratch, then an ordered per-row fold; kick: also runs the next step's
+// half kick and drift; fast: LG_FORCE_KERNEL_FP64_FAST (reciprocals instead of repeated divisions;
+// within 1e-12). Returns the number of kernels launched.
 int launch_forces_pairs_fp64(const Params &P, const StateView &S, const PairView &PV, const BondView &BV,
-                             double *pres, double hdt, double dt, int move_facets, bool kick, cudaStream_t st);
+                             const PairScratch &R, double hdt, double dt, int move_facets, bool kick, bool fast,
+                             cudaStream_t st);
 // With connectors (BV.cn non-null) the drift also carries the 5-connector model's connectors.
 // hold: per-particle LG_HOLD_* bits (null: none).
 void launch_kick_drift_fp64(int64_t n, dbl4 *x, dbl4 *v, dbl4 *th, dbl4 *w, const dbl4 *a,
@@ -154,11 +169,7 @@ int launch_step_mixed(const Params &P, const StateView &S, const PairView &PV, c
                       const MixedExtra &MX, const StepArgs &A, cudaStream_t st, cudaStream_t side = nullptr,
                       cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr);
 
-// Warp-compacted force kernels (lg_forces_compact.cu, compiled once per precision)
-// fast: LG_FORCE_KERNEL_FP64_FAST (reciprocals instead of repeated divisions; within 1e-12).
-void launch_forces_compact_fp64(const Params &P, const StateView &S, const PairView &PV, const BondView &BV, double hdt,
-                                double dt, int move_facets, cudaStream_t st, bool fast = false);
-// Mixed precision: the contact/bond kernel (if the system has a binary model) on `side`, beside the
+// Warp-compacted mixed-precision kernels (lg_forces_compact_mixed.cu): the contact/bond kernel (if the system has a binary model) on `side`, beside the
 // Hamaker kernel on `st` (fork / join through the two events), then the completion kernel on `st`;
 // returns the number of kernels launched.
 // With `kick`, the completion kernel goes on to the next step's opening half kick and drift (and the
