@@ -196,21 +196,21 @@ typedef struct lg_system_desc {
     void *unary_hook_user;
 } lg_system_desc;
 
-/* Force kernels. Both give deterministic sums; in FP64 both add each row in ascending j, and the
- * compacted kernel and the row-group kernel with one lane per row are bit-identical to a
- * sequential evaluation of libgran's functors. */
-#define LG_FORCE_KERNEL_AUTO 0       /* mixed: compacted; FP64: pair-parallel for small systems, compacted
-                                       for large ones */
+/* Force kernels. All give deterministic sums; in FP64 the pair kernels and the row-group kernel with one
+ * lane per row add each row in ascending j and are bit-identical to a sequential evaluation of libgran's
+ * functors. */
+#define LG_FORCE_KERNEL_AUTO 0       /* mixed: compacted; FP64: the pair kernels */
 #define LG_FORCE_KERNEL_ROWGROUP 1   /* T lanes per row (threads_per_row), fixed butterfly combine */
-#define LG_FORCE_KERNEL_COMPACT 2    /* one row per lane, warp-compacted pair queues (see csrc) */
-#define LG_FORCE_KERNEL_PAIRS 3      /* FP64, small systems: one thread per pair slot spread over all SMs,
-                                       then an ordered per-row fold (the reference's summation order) */
+#define LG_FORCE_KERNEL_COMPACT 2    /* mixed: one row per lane, warp-compacted pair queues; FP64: the pair
+                                       kernels (every unordered pair once, queued contacts, then an ordered
+                                       per-row fold in the reference's summation order) */
+#define LG_FORCE_KERNEL_PAIRS 3      /* FP64: the pair kernels, for systems of at most 2^21 pair slots */
 #define LG_FORCE_KERNEL_PERSISTENT 4 /* mixed: every step inside a run of steps (no facets, body terms or
                                        held particles) is one persistent launch whose warps pull contact
                                        and Hamaker work items of 32-row groups from a device queue and
                                        complete each group when its last item finishes; the same bits as
                                        the compacted kernels. Other steps use the compacted kernels. */
-#define LG_FORCE_KERNEL_FP64_FAST 5  /* FP64: the compacted kernel with one reciprocal where libgran divides a
+#define LG_FORCE_KERNEL_FP64_FAST 5  /* FP64: the pair kernels with one reciprocal where libgran divides a
                                        vector by a scalar, and the Hamaker bracket over one common
                                        denominator (2 divisions per Hamaker pair instead of 12, 2 per
                                        contact scaling instead of 6); contact is decided by the reference's

@@ -49,7 +49,10 @@ __host__ __device__ __forceinline__ double droot(double z) {
 __host__ __device__ __forceinline__ d3 dvs(d3 a, double s) {
 #ifdef __CUDA_ARCH__
     const xd::Divisor d = xd::divisor(s);  // one reciprocal for the three quotients
-    return mk3(xd::quotient(a.x, d), xd::quotient(a.y, d), xd::quotient(a.z, d));
+    bool ok = true;
+    const d3 q = mk3(xd::quotient(a.x, d, ok), xd::quotient(a.y, d, ok), xd::quotient(a.z, d, ok));
+    if (ok) return q;
+    return mk3(xd::slow_div(a.x, s), xd::slow_div(a.y, s), xd::slow_div(a.z, s));
 #else
     return mk3(a.x / s, a.y / s, a.z / s);
 #endif
@@ -145,6 +148,12 @@ struct FacetDev {
     lg_hamaker_params hamaker;
 };
 
+// Values of the Hamaker functor that do not depend on the pair, each formed as the functor forms it.
+struct HamakerConst {
+    double two_r, four_r, four_r2, two_r2, a6, a2r;  // 2r, 4r, 4 r^2, 2 r^2, -A / 6, 2 A r
+    xd::Divisor mass;
+};
+
 struct Params {
     int64_t n;
     int32_t binary_model, hamaker_model, neck_mode, pairs;
@@ -154,8 +163,10 @@ struct Params {
     double r_verlet;
     int32_t n_facets;
     FacetDev facets[kMaxFacets];
-    double contact_skip_d2;  // squared centre distance above which overlap <= 0 is certain
-    double hamaker_skip_d2;  // squared centre distance above which the limited Hamaker is zero
+    // bounds as above() takes them: squared centre distance above which overlap <= 0 is certain, squared
+    // distance above which the limited Hamaker is zero, and its cutoff
+    int64_t contact_skip_d2, hamaker_skip_d2, hamaker_cut;
+    HamakerConst hc;
     int32_t springs_ff;      // pair and bond springs held as float-float pairs (mixed precision)
     lg_connector_params connector;  // 5-connector sinter model
     const uint8_t *hold;     // [n] LG_HOLD_* bits of the increments the integrator skips; null: none
@@ -334,30 +345,34 @@ __device__ __forceinline__ double cb_(double x) { return x * x * x; }
 //   (4r+2h) u - 2 w - 4 r^2 w^3 - 2 r^2 (4r+2h) u^2,
 // and the scaling by 1 / (|r| m) as one factor: two divisions per pair instead of twelve.
 template <bool FAST = false>
-__device__ __forceinline__ d3 hamaker_accel_n(int mode, const lg_hamaker_params &p, d3 r, double rn) {
-    double h = rn - 2.0 * p.r_part;
+__device__ __forceinline__ d3 hamaker_accel_n(int mode, const lg_hamaker_params &p, const HamakerConst &C, d3 r,
+                                              double rn) {
+    double h = rn - C.two_r;
     if (h < p.h0) h = p.h0;
-    double rp = p.r_part;
     double s;
     if (FAST && mode != LG_HAMAKER_SIMPLIFIED) {
-        const double q = 4.0 * rp + h, w0 = 2.0 * rp + h, a = 4.0 * rp + 2.0 * h;
+        const double q = C.four_r + h, w0 = C.two_r + h, a = __fma_rn(2.0, h, C.four_r);
         const double inv = ddiv(1.0, q * h * w0);
         const double u = w0 * inv, w = q * h * inv;
-        const double br = a * u - 2.0 * w - 4.0 * sq_(rp) * (w * w * w) - 2.0 * sq_(rp) * a * (u * u);
-        s = ddiv(-p.A, 6.0) * br;
+        const double br = a * u - 2.0 * w - C.four_r2 * (w * w * w) - C.two_r2 * a * (u * u);
+        s = C.a6 * br;
         return rn > 0.0 ? scl(ddiv(s, rn * p.mass), r) : dvs_t<true>(scl(s, r), p.mass);
     }
     if (mode == LG_HAMAKER_SIMPLIFIED) {
-        s = ddiv(2.0 * p.A * rp, sq_(h));
-    } else {
-        const double a = 4.0 * rp + 2.0 * h, q = 4.0 * rp + h, w = 2.0 * rp + h;
-        double br = ddiv(ddiv(a, q), h) - ddiv(2.0, w) - ddiv(4.0 * sq_(rp), cb_(w)) -
-                    ddiv(ddiv(2.0 * sq_(rp) * a, sq_(q)), sq_(h));
-        s = ddiv(-p.A, 6.0) * br;
+        s = ddiv(C.a2r, sq_(h));
+    } else {  // (2 h is exact, so the fused 2 h + 4 r rounds as their sum)
+        const double a = __fma_rn(2.0, h, C.four_r), q = C.four_r + h, w = C.two_r + h;
+        double br = ddiv(ddiv(a, q), h) - ddiv(2.0, w) - ddiv(C.four_r2, cb_(w)) -
+                    ddiv(ddiv(C.two_r2 * a, sq_(q)), sq_(h));
+        s = C.a6 * br;
     }
     if (FAST) return rn > 0.0 ? scl(ddiv(s, rn * p.mass), r) : dvs_t<true>(scl(s, r), p.mass);
-    d3 u = (rn > 0.0) ? dvs(r, rn) : r;  // nrmz(r)
-    return dvs(scl(s, u), p.mass);
+    const int64_t ir = __double_as_longlong(rn);
+    const d3 u = ir > 0 && ir <= 0x7ff0000000000000ll ? dvs(r, rn) : r;  // nrmz(r)
+    const d3 su = scl(s, u);
+    bool ok = true;
+    const d3 a = mk3(xd::quotient(su.x, C.mass, ok), xd::quotient(su.y, C.mass, ok), xd::quotient(su.z, C.mass, ok));
+    return ok ? a : dvs(su, p.mass);
 }
 
 // triangular_facet.h:73-137

@@ -725,6 +725,17 @@ static int apply_unary(lg_system *s, const lg_body_force *body, lg_unary_hook ho
     return LG_OK;
 }
 
+// A bound as the kernels' integer comparison takes it: a > b for every nonnegative a (NaN excepted) when
+// the bits of a exceed it.
+static int64_t above_bound(double b) {
+    if (std::isnan(b)) return INT64_MAX;  // never above
+    if (b < 0) return -1;                 // always above
+    const double z = std::fabs(b);
+    int64_t bits;
+    std::memcpy(&bits, &z, sizeof(bits));
+    return bits;
+}
+
 // A serving arena (lg_arena_create): a batch whose systems are slots that start empty -- every
 // particle inactive, no bonds -- on a lattice of the given spacing, with bond capacity bcap per
 // particle and float-float extents allowed up to ext.
@@ -778,8 +789,17 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
     P.r_verlet = d->r_verlet;
     P.n_facets = d->n_facets;
     const double cr = 2.0 * d->contact.r_part;
-    P.contact_skip_d2 = cr * cr * (1.0 + 1e-9);
-    P.hamaker_skip_d2 = d->hamaker.r_cutoff * d->hamaker.r_cutoff * (1.0 + 1e-9);
+    P.contact_skip_d2 = above_bound(cr * cr * (1.0 + 1e-9));
+    P.hamaker_skip_d2 = above_bound(d->hamaker.r_cutoff * d->hamaker.r_cutoff * (1.0 + 1e-9));
+    P.hamaker_cut = above_bound(d->hamaker.r_cutoff);
+    const double hr = d->hamaker.r_part;  // as the functor forms them (hamaker_force.h:36-40)
+    P.hc.two_r = 2.0 * hr;
+    P.hc.four_r = 4.0 * hr;
+    P.hc.four_r2 = 4.0 * (hr * hr);
+    P.hc.two_r2 = 2.0 * (hr * hr);
+    P.hc.a6 = -d->hamaker.A / 6.0;
+    P.hc.a2r = 2.0 * d->hamaker.A * hr;
+    P.hc.mass = xd::divisor(d->hamaker.mass);
     P.springs_ff = d->precision == LG_PRECISION_MIXED ? 1 : 0;
     P.connector = d->connector;
     for (int f = 0; f < d->n_facets; ++f) {

@@ -5,13 +5,13 @@
 // much issue time as several hundred integer instructions. Here both operations run in fixed point:
 //   reciprocal  a 22-bit estimate (MUFU), two Newton steps y <- y + y (1 - b y) on the 64-bit
 //               significand: y = 2^64 / b' to a few units, never above it;
-//   quotient    the high half of a' y: the quotient to about 60 bits, never above it. Where its low
-//               bits leave the rounding open (it lies within kQMargin units below a midpoint, about
-//               1 % of all quotients), the sign of the exact remainder a - m b of the midpoint m decides:
-//               it is small, so 64-bit wrap-around arithmetic holds it exactly. (A quotient of two
-//               53-bit significands is never a midpoint itself.)
+//   quotient    the high half of a' y: the quotient to about 60 bits, never above it, cut to 53 bits;
+//               the sign of the exact remainder a - m b of the midpoint m above it decides the rounding
+//               (the remainder is smaller than b, so 64-bit wrap-around arithmetic holds it; a quotient
+//               of two 53-bit significands is never a midpoint itself);
 //   root        the same with an inverse-root estimate, one Newton step, s = z y, one correction
 //               s + (z - s^2) y / 2, and the sign of z - m^2.
+// No step branches on the values, so independent quotients overlap.
 // So results are RN(a / b) and RN(sqrt(z)), bit for bit what IEEE arithmetic gives. Long division
 // with a quotient estimate and an exact remainder test is Knuth's (The Art of Computer Programming,
 // vol. 2, 4.3.1); Newton iterations with a final remainder test are described in Muller et al.,
@@ -94,11 +94,21 @@ float rcp_estimate(float f);
 float rsqrt_estimate(float f);
 #endif
 
+// 2^32 f for an estimate f of about [0.5, 1], kept within [2^31, 2^32 - 2^8]: from the float's bits, since
+// a conversion instruction would go through the same slow path as the FP64 operations
+LG_XD uint32_t fixed32(float f) {
+#ifdef __CUDACC__
+    int32_t u = __float_as_int(f);
+#else
+    int32_t u;
+    std::memcpy(&u, &f, 4);
+#endif
+    u = u < 0x3f000000 ? 0x3f000000 : u > 0x3f7fffff ? 0x3f7fffff : u;
+    return ((uint32_t)u << 8) | 0x80000000u;
+}
+
 constexpr uint64_t kFrac = 0xfffffffffffffull;  // 52 fraction bits
 constexpr uint64_t kOne = 0x10000000000000ull;  // the implicit bit
-constexpr uint32_t kQMargin = 32;  // units (2^-63 of the quotient's scale) a quotient may lie low
-constexpr uint32_t kSMargin = 16;  // the same for a root (2^-62 of its scale)
-
 LG_XD_SLOW double slow_div(double a, double b) { return a / b; }
 LG_XD_SLOW double slow_sqrt(double z) { return ::sqrt(z); }
 
@@ -106,18 +116,16 @@ LG_XD_SLOW double slow_sqrt(double z) { return ::sqrt(z); }
 struct Divisor {
     uint64_t y, m;  // reciprocal, 53-bit significand
     uint32_t top;   // sign and exponent field (bits 52..63 of b)
-    double b;
 };
 
 LG_XD Divisor divisor(double b) {
     const uint64_t u = bits_of(b);
     Divisor d;
-    d.b = b;
     d.top = (uint32_t)(u >> 52);
     d.m = (u & kFrac) | kOne;
     const uint64_t bn = d.m << 11;  // b' 2^63
     const float r = rcp_estimate(float_of(0x3f800000u | ((uint32_t)(u >> 29) & 0x7fffffu)));
-    const uint32_t y0 = (uint32_t)(r * 4294967040.0f);  // 2^32 y0, just below 2^32 for y0 = 1
+    const uint32_t y0 = fixed32(r);
     // e = 1 - b' y0 (2^63 units, |e| < 2^-20), y1 = y0 + y0 e
     const uint64_t t0 = mul_wide((uint32_t)(bn >> 32), y0) + (mul_wide((uint32_t)bn, y0) >> 32);
     const int32_t e0 = (int32_t)((int64_t)(0x8000000000000000ull - t0) >> 12);
@@ -128,33 +136,30 @@ LG_XD Divisor divisor(double b) {
     return d;
 }
 
-// RN(a / d.b)
-LG_XD double quotient(double a, const Divisor &d) {
+// RN(a / b) for the divisor b where `ok` stays true: a zero or normal, b and the quotient normal
+LG_XD double quotient(double a, const Divisor &d, bool &ok) {
     const uint64_t u = bits_of(a);
     const uint32_t top = (uint32_t)(u >> 52), ea = top & 0x7ffu, eb = d.top & 0x7ffu;
     const uint64_t sign = (uint64_t)((top ^ d.top) & 0x800u) << 52;
     const uint64_t m = (u & kFrac) | kOne;
     uint64_t q = mul_hi(m << 11, d.y);  // a' / b' 2^63, in (2^62, 2^64)
     const bool ge1 = (int64_t)q < 0;
-    const int32_t er = (int32_t)ea - (int32_t)eb + (ge1 ? 1023 : 1022);  // exponent field of the quotient
+    const int32_t er = (int32_t)ea - (int32_t)eb + (ge1 ? 1022 : 1021);  // exponent field of the quotient, less 1
     if (!ge1) q += q;
-    const uint32_t f = (uint32_t)q & 0x7ffu;
     const uint64_t s = q >> 11;  // the quotient's 53-bit significand, truncated
-    bool up = f >= 0x400u;
-    if (0x3ffu - f < kQMargin) {  // up to kQMargin below a midpoint: the remainder decides
-        const uint64_t rem = (m << (ge1 ? 53 : 54)) - (2u * s + 1u) * d.m;
-        up = (int64_t)rem > 0;
-    }
-    const double r = of_bits(sign | (((uint64_t)(uint32_t)(er - 1) << 52) + s + (up ? 1u : 0u)));
-    const bool fast = (ea - 1u) < 0x7feu && (eb - 1u) < 0x7feu && (uint32_t)(er - 1) < 0x7fdu;
-    if (!fast) {
-        if ((u << 1) == 0 && (eb - 1u) < 0x7feu) return of_bits(sign);  // zero over a normal number
-        return slow_div(a, d.b);
-    }
-    return r;
+    // (a' 2^53 or 2^54) - (2 s + 1) b': the sign of quotient - midpoint
+    const uint64_t rem = (m << (ge1 ? 53 : 54)) - (2u * s + 1u) * d.m;
+    const double r = of_bits(sign | (((uint64_t)(uint32_t)er << 52) + s + ((int64_t)rem > 0 ? 1u : 0u)));
+    const bool zero = (u << 1) == 0;
+    ok = ok && (eb - 1u) < 0x7feu && (zero || ((ea - 1u) < 0x7feu && (uint32_t)er < 0x7fdu));
+    return zero ? of_bits(sign) : r;
 }
 
-LG_XD double div(double a, double b) { return quotient(a, divisor(b)); }
+LG_XD double div(double a, double b) {
+    bool ok = true;
+    const double r = quotient(a, divisor(b), ok);
+    return ok ? r : slow_div(a, b);
+}
 
 // RN(sqrt(z))
 LG_XD double root(double z) {
@@ -164,7 +169,7 @@ LG_XD double root(double z) {
     const uint64_t m = (u & kFrac) | kOne;
     const uint64_t zn = m << (10 + odd);  // z' 2^62, z' in [1, 4)
     const float r = rsqrt_estimate(float_of(((127u + odd) << 23) | ((uint32_t)(u >> 29) & 0x7fffffu)));
-    const uint32_t y0 = (uint32_t)(r * 4294967040.0f);
+    const uint32_t y0 = fixed32(r);
     // e = 1 - z' y0^2 (2^62 units, |e| < 2^-19), y1 = y0 + y0 e / 2
     const int32_t e0 = (int32_t)((int64_t)(0x4000000000000000ull - mul_hi(zn, mul_wide(y0, y0))) >> 12);
     const uint64_t y1 = ((uint64_t)y0 << 32) + (uint64_t)(((int64_t)e0 * (int64_t)(uint64_t)y0) >> 19);
@@ -172,13 +177,9 @@ LG_XD double root(double z) {
     const uint64_t s1 = mul_hi(zn, y1);
     const int32_t e1 = (int32_t)(int64_t)((zn >> 2) - 1u - mul_hi(s1, s1));
     const uint64_t s = s1 + (uint64_t)(((int64_t)e1 * (int64_t)(y1 >> 32)) >> 31);
-    const uint32_t f = (uint32_t)s & 0x3ffu;
     const uint64_t t = s >> 10;  // 53-bit significand, truncated
-    bool up = f >= 0x200u;
-    if (0x1ffu - f < kSMargin) {
-        const uint64_t mid = 2u * t + 1u;
-        up = (int64_t)((m << (54 + odd)) - mid * mid) > 0;
-    }
+    const uint64_t mid = 2u * t + 1u;
+    const bool up = (int64_t)((m << (54 + odd)) - mid * mid) > 0;
     const uint32_t er = (top + 1023u - 1u + (odd ^ 1u)) >> 1;  // exponent field of the root
     const double v = of_bits(((uint64_t)(er - 1u) << 52) + t + (up ? 1u : 0u));
     if ((top - 1u) >= 0x7feu) return (u << 1) == 0 ? z : slow_sqrt(z);
