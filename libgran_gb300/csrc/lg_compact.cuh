@@ -10,7 +10,6 @@ namespace lg {
 namespace compact {
 
 constexpr int kWin = 4;           // slots per window (classified per memory round trip)
-constexpr int kHCap = 32 * kWin;  // Hamaker queue capacity per window
 
 // Facet auto-move: the vertices one step ahead, written once per launch into the second vertex
 // buffer; the engine swaps the two buffers after the step.

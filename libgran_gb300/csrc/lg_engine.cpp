@@ -433,6 +433,38 @@ static PairScratch pair_scratch(const lg_system *s) {
     return R;
 }
 
+// Scratch of the mixed contact kernel that evaluates each pair once, in the idle list's spring buffer (9
+// doubles a slot: two float4 of records, an owner entry). Neck strengths looked up by the reference's
+// indexing differ between a pair's two orders, so a breaking bond may then break in one order only: such
+// systems take the kernel that evaluates each order.
+static NearScratch near_scratch(const lg_system *s) {
+    NearScratch R{};
+    if (!s->own_n || s->precision != LG_PRECISION_MIXED || !s->pv[0].near_len) return R;
+    if (s->P.n < (getenv("LG_NM") ? atoi(getenv("LG_NM")) : 8192)) return R;
+    if (s->P.binary_model == LG_BINARY_BREAKING_SINTER && s->P.neck_mode == LG_NECK_REFERENCE_INDEXING) return R;
+    double *base = s->pv[1 - s->pcur].xi;
+    const int64_t slots = s->pv[0].cap * s->P.n;
+    R.rec = reinterpret_cast<float4 *>(base);
+    R.own = reinterpret_cast<uint4 *>(base + 4 * slots);
+    R.own_n = s->own_n;
+    R.rb = near_block_rows(s->P.n);
+    return R;
+}
+
+// The owned slots or contact candidates of the current list (after a build, and after a restore brings an
+// older list back).
+static void list_owners(lg_system *s) {
+    const NearScratch N = near_scratch(s);
+    if (N.rec) {
+        launch_near_owners(s->P.n, s->pv[s->pcur], N, s->stream);
+    } else if (s->own_n && s->precision == LG_PRECISION_FP64) {
+        launch_pair_owners(s->P.n, s->pv[s->pcur], pair_scratch(s), s->stream);
+    } else {
+        return;
+    }
+    s->launches += 1;
+}
+
 static int rebuild_list(lg_system *s) {
     PairView &oldv = s->pv[s->pcur];
     PairView &newv = s->pv[1 - s->pcur];
@@ -441,13 +473,10 @@ static int rebuild_list(lg_system *s) {
     BatchView B{s->d_agg, s->d_hoff, s->P.hold};
     launch_list_build(s->P.n, s->x, B, s->P.r_verlet, s->r_near, s->max_cells, s->ls, o, newv, s->bv, s->err,
                       s->stream);
-    s->launches += 9;
+    s->launches += 5;
     s->pcur = 1 - s->pcur;
     s->list_built = true;
-    if (s->own_n) {
-        launch_pair_owners(s->P.n, s->pv[s->pcur], pair_scratch(s), s->stream);
-        s->launches += 1;
-    }
+    list_owners(s);
     LG_CUDA(cudaGetLastError());
     return LG_OK;
 }
@@ -574,7 +603,7 @@ static int launch_forces(lg_system *s, double hdt, double dt, int move_facets, b
         if (compact || persistent)
             kernels = launch_forces_compact_mixed(s->P, S, s->pv[s->pcur], s->bv, hdt, dt, move_facets, fuse_kick,
                                                   prev_fused, s->mx, s->stream, s->side, s->fork_ev, s->join_ev,
-                                                  s->ham_slices, s->contact_lanes);
+                                                  s->ham_slices, s->contact_lanes, near_scratch(s));
         else
             launch_forces_mixed(s->T, s->P, S, s->pv[s->pcur], s->bv, hdt, dt, move_facets, s->mx, s->stream);
     } else {
@@ -1095,18 +1124,19 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
             const double per = (double)m * arena->lattice / d->r_verlet + 2.0;
             s->max_cells = std::max<int64_t>(s->max_cells, (int64_t)std::min(per * per * per, 33554432.0));
         }
-        s->ls.nparts = 256;
-        LG_TRY(s->alloc(&s->ls.part, 6 * 256));
+        s->ls.nparts = 608;
+        LG_TRY(s->alloc(&s->ls.part, 6 * 608));
         LG_TRY(s->alloc(&s->ls.grid, 1));
         LG_TRY(s->alloc(&s->ls.cell_of, (size_t)n));
         LG_TRY(s->alloc(&s->ls.count, (size_t)s->max_cells));
         LG_TRY(s->alloc(&s->ls.start, (size_t)s->max_cells));
-        LG_TRY(s->alloc(&s->ls.fill, (size_t)s->max_cells));
         LG_TRY(s->alloc(&s->ls.sorted, (size_t)n));
-        LG_TRY(s->alloc(&s->ls.tile, (size_t)(s->max_cells / 4096 + 1)));
+        LG_TRY(s->alloc(&s->ls.ticket, 1));
+        LG_TRY(s->alloc(&s->ls.cursor, 1));
+        LG_CUDA(cudaMemset(s->ls.ticket, 0, sizeof(unsigned)));
         LG_TRY(s->alloc(&s->ls.x32, (size_t)n));
         LG_TRY(s->alloc(&s->ls.max_row, 1));
-        if (s->precision == LG_PRECISION_FP64) LG_TRY(s->alloc(&s->own_n, (size_t)n / 4 + 1));
+        if (s->precision == LG_PRECISION_FP64 || s->r_near > 0) LG_TRY(s->alloc(&s->own_n, (size_t)n / 4 + 1));
         LG_CUDA(cudaMemset(s->ls.max_row, 0, sizeof(int32_t)));
         LG_TRY(rebuild_list(s));
         // without an explicit max_neighbors the row capacity follows the initial state: rows get
@@ -2396,6 +2426,8 @@ static int snapshot_restore(lg_system *s) {
     set_ff_buffers(s);
     s->step_index = s->snap_step;
     s->list_built = s->snap_built;
+    if (s->list_built) list_owners(s);
+    LG_CUDA(cudaGetLastError());
     return LG_OK;
 }
 

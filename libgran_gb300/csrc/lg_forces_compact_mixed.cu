@@ -34,6 +34,8 @@ using namespace mixed;
 
 namespace {
 
+constexpr uint32_t kNoPartner = 255u;  // the partner's row does not list the entry's row
+
 // ---- launch shapes of the two-stream kernels ----
 // Slices per row group of the Hamaker kernel: 0 chooses from the launch size (compile-time
 // override for tuning).
@@ -41,9 +43,7 @@ namespace {
 #define LG_MIXED_SLICES 0
 #endif
 constexpr int kCWarps = 2;   // warps per block
-#ifndef LG_HAMAKER_REGS
-#define LG_HAMAKER_REGS 96  // register budget of the Hamaker kernel (compile-time override for tuning)
-#endif
+constexpr int kHThreads = 128;  // threads per block of the Hamaker kernel
 // Resident blocks per SM the contact kernel is compiled for (its register budget): beside the Hamaker
 // kernel (two streams) a tighter budget lets more of both kernels' warps share an SM; alone, the
 // looser one avoids spills. Measured on the 32768-particle workload (graph-replayed steps): 12 blocks
@@ -55,14 +55,6 @@ constexpr int kCWarps = 2;   // warps per block
 #ifndef LG_CONTACT_MIN_BLOCKS_ALONE
 #define LG_CONTACT_MIN_BLOCKS_ALONE 8
 #endif
-template <int SL>
-struct ShapeH {
-    static constexpr int kSlices = SL;
-    static constexpr int kRowWarps = SL == 1 ? 2 : 1;  // 32-row groups per block
-    static constexpr int kWarps = kSlices * kRowWarps;
-    // blocks per SM that the register budget allows (shared memory allows as many)
-    static constexpr int kMinBlocks = 65536 / (kWarps * 32 * LG_HAMAKER_REGS);
-};
 }  // namespace
 
 // Contact and bond pairs of rows row0 .. row0 + 32/T - 1 per warp (contact_rows), csum receives the
@@ -77,46 +69,298 @@ __global__ void __launch_bounds__(kCWarps * 32, MINB)
     contact_rows<NEAR, T>(P, PV, BV, MX, W, ((int64_t)blockIdx.x * kCWarps + warp) * kRows, lane);
 }
 
-// Hamaker pairs of rows row0 .. row0 + 31; hsum receives the Hamaker part of the row's acceleration
-// as float-float pairs. With SL > 1 slices the row group's windows are spread over SL warps of the
-// block, whose partial sums are combined in slice order.
-template <bool VERLET, int SL>
-__global__ void __launch_bounds__(ShapeH<SL>::kWarps * 32, ShapeH<SL>::kMinBlocks)
-    forces_hamaker_mixed(Params P, PairView PV, MixedExtra MX) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int kSlices = ShapeH<SL>::kSlices, kRowWarps = ShapeH<SL>::kRowWarps;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    HamakerSmem *Wall = reinterpret_cast<HamakerSmem *>(smem_raw);
-    HamakerSmem &W = Wall[warp];
-    const int rw = warp / kSlices, sl = warp % kSlices;  // row group of the block, slice of it
-    const int64_t row0 = ((int64_t)blockIdx.x * kRowWarps + rw) * 32;
-    const int64_t i = row0 + lane;
-    const bool active = i < P.n;
-    ff acch[3];
-    hamaker_rows<VERLET>(P, PV, MX, W, row0, sl, kSlices, lane, acch);
-    if (kSlices > 1) {
-        // combine the slices' partial sums of each row in slice order (fixed, deterministic); each
-        // warp parks its partials in its own queue, which is no longer in use
-        float *mine = reinterpret_cast<float *>(W.hhi);
+// The owned contact candidates of each block of `rb` rows: of the two entries of a pair (i, j) the one in
+// row i when i < j and i + j is odd, or i > j and i + j is even; an entry that the partner's row does not
+// list is always owned. (j; local row, slot, slot in the partner's row; entry, entry in the partner's row.)
+__global__ void __launch_bounds__(512) near_owners(int64_t n, PairView PV, NearScratch R) {
+    __shared__ int32_t cnt;
+    if (threadIdx.x == 0) cnt = 0;
+    __syncthreads();
+    const int64_t row0 = (int64_t)blockIdx.x * R.rb;
+    uint4 *own = R.own + row0 * PV.cap;
+    const int per = blockDim.x / R.rb;  // lanes per row
+    const int r = threadIdx.x % R.rb;
+    const int64_t i = row0 + r;
+    const int len = i < n ? PV.near_len[i] : 0;
+    for (int m = threadIdx.x / R.rb; m < len; m += per) {
+        const int32_t j = PV.near_j[(int64_t)m * n + i];
+        const uint32_t k = PV.near_k[(int64_t)m * n + i];
+        const int lj = PV.near_len[j];
+        int m2 = 0;
+        while (m2 < lj && PV.near_j[(int64_t)m2 * n + j] != (int32_t)i) ++m2;
+        const bool both = m2 < lj;
+        if (both && !(((i + j) & 1) ? i < j : i > j)) continue;
+        const uint32_t k2 = both ? PV.near_k[(int64_t)m2 * n + j] : kNoPartner;
+        own[atomicAdd(&cnt, 1)] =
+            make_uint4((uint32_t)j, (uint32_t)r | (k << 8) | (k2 << 16), (uint32_t)m | ((uint32_t)m2 << 8), 0u);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) R.own_n[blockIdx.x] = cnt;
+}
+
+// Contact and bond pairs, each evaluated once for both of its rows (contact_pair): the block's owned
+// candidates are classified two per thread, those that can touch or are bonded are queued in shared memory and
+// evaluated 32 at a time. Each entry's accelerations go to its record (zero when apart), which the
+// completion adds per row in entry order; the springs of both slots are written.
+// What bounds it: instruction issue and the latency of its gathers.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 640 / THREADS)
+    mixed_contacts(Params P, PairView PV, BondView BV, MixedExtra MX, NearScratch R) {
+    struct Item {
+        int32_t i, j;
+        uint32_t kk, mm;  // slots (k | k2 << 8), entries (m | m2 << 8); k2 = kNoPartner: one-sided
+    };
+    __shared__ Item queue[4 * THREADS];
+    __shared__ int32_t qn;
+    const int tid = threadIdx.x;
+    const int64_t n = P.n;
+    const int count = R.own_n[blockIdx.x];
+    const int64_t row0 = (int64_t)blockIdx.x * R.rb;
+    const uint4 *own = R.own + row0 * PV.cap;
+    const int64_t xs = PV.cap * n, bs = (int64_t)BV.bcap * n;
+    auto put = [&](int64_t i, uint32_t m, float4 a, float4 b) {
+        R.rec[2 * ((int64_t)m * n + i)] = a;
+        R.rec[2 * ((int64_t)m * n + i) + 1] = b;
+    };
+    auto part = [&](int64_t i, uint32_t m, int64_t e, uint32_t fl) {  // reset_springs (contact_force.h:69,99-101)
+        put(i, m, make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f));
+        if (!(fl & kXiLive)) return;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            mine[(2 * c) * 32 + lane] = acch[c].hi;
-            mine[(2 * c + 1) * 32 + lane] = acch[c].lo;
+        for (int c = 0; c < 9; ++c) PV.xi[spring_at(PV.aos, c, e, xs)] = 0.0;
+        PV.flags[e] = fl & ~kXiLive;
+    };
+    for (int t0 = 0; t0 < count; t0 += 2 * THREADS) {
+        if (tid == 0) qn = 0;
+        __syncthreads();
+        uint4 o[2];
+        bool live[2];
+        float4 pi[2], pj[2];
+        uint32_t fl[2], fl2[2];
+        int64_t e[2], e2[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            live[u] = t0 + u * THREADS + tid < count;
+            o[u] = own[live[u] ? t0 + u * THREADS + tid : 0];
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int64_t j = o[u].x, i = row0 + (o[u].y & 0xffu);
+            const uint32_t k = (o[u].y >> 8) & 0xffu, k2 = (o[u].y >> 16) & 0xffu;
+            e[u] = (int64_t)k * n + i;
+            e2[u] = k2 != kNoPartner ? (int64_t)k2 * n + j : e[u];
+            pi[u] = MX.x32[2 * i];
+            pj[u] = MX.x32[2 * j];
+            fl[u] = PV.flags[e[u]];
+            fl2[u] = PV.flags[e2[u]];
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            if (!live[u]) continue;
+            const int64_t j = o[u].x, i = row0 + (o[u].y & 0xffu);
+            const uint32_t k = (o[u].y >> 8) & 0xffu, k2 = (o[u].y >> 16) & 0xffu, m = o[u].z & 0xffu, m2 = o[u].z >> 8;
+            const bool both = k2 != kNoPartner;
+            const float dx = pi[u].x - pj[u].x, dy = pi[u].y - pj[u].y, dz = pi[u].z - pj[u].z;
+            if (((fl[u] | fl2[u]) & kBonded) || fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= MX.contact2f) {
+                // the two orders' states agree, unless only one of them lost its bond or list place
+                const bool split = both && ((fl[u] ^ fl2[u]) & (kBonded | kXiLive));
+                const int q = atomicAdd(&qn, split ? 2 : 1);
+                queue[q] = Item{(int32_t)i, (int32_t)j, k | ((split ? kNoPartner : k2) << 8), m | (m2 << 8)};
+                if (split) queue[q + 1] = Item{(int32_t)j, (int32_t)i, k2 | (kNoPartner << 8), m2 | (m << 8)};
+            } else {
+                part(i, m, e[u], fl[u]);
+                if (both) part(j, m2, e2[u], fl2[u]);
+            }
         }
         __syncthreads();
-        if (sl != 0) return;
-        for (int q = 1; q < kSlices; ++q) {
-            const float *o = reinterpret_cast<const float *>(Wall[rw * kSlices + q].hhi);
+        const int total = qn;
+        for (int q = tid; q < total; q += THREADS) {
+            const Item it = queue[q];
+            const int64_t i = it.i, j = it.j;
+            const uint32_t k = it.kk & 0xffu, k2 = it.kk >> 8;
+            const bool both = k2 != kNoPartner;
+            const int64_t e = (int64_t)k * n + i, e2 = both ? (int64_t)k2 * n + j : e;
+            const uint32_t fl = PV.flags[e], fl2 = PV.flags[e2];
+            const bool bonded = (fl & kBonded) != 0;
+            // (mixed precision stores springs as one 9-component record per slot or bond)
+            const int64_t at = bonded ? (int64_t)bond_slot_of(fl) * n + i : e;
+            const int64_t at2 = bonded ? (int64_t)bond_slot_of(fl2) * n + j : e2;
+            float2 *store = reinterpret_cast<float2 *>(bonded ? BV.xi : PV.xi);
+            const int32_t aos = bonded ? BV.aos : PV.aos;
+            const int64_t stride = bonded ? bs : xs;
+            const Body bi = body_of(MX, n, i), bj = body_of(MX, n, j);
+            ff s[3][3] = {};  // springs of a slot that is not live are zero
+            if (fl & (kBonded | kXiLive))
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                ff_acc(acch[c], o[(2 * c) * 32 + lane]);
-                ff_acc(acch[c], o[(2 * c + 1) * 32 + lane]);
+                for (int c = 0; c < 9; ++c) {
+                    const float2 v = store[spring_at(aos, c, at, stride)];
+                    s[c / 3][c % 3] = ff{v.x, v.y};
+                }
+            ContactOut o;
+            if (!contact_pair(P, MX, bonded, i, j, bi, bj, s, o)) {
+                part(i, it.mm & 0xffu, e, fl);
+                if (both) part(j, it.mm >> 8, e2, fl2);
+                continue;
+            }
+            const bool breaks = bonded && P.binary_model == LG_BINARY_BREAKING_SINTER;
+            const float f2 = fdot(o.force, o.force);
+            float sgn = 1.0f;
+            const int sides = both ? 2 : 1;
+#pragma unroll 1
+            for (int side = 0; side < sides; ++side) {  // the row's own values, then the partner's
+                const int64_t row = side ? j : i, es = side ? e2 : e, as = side ? at2 : at;
+                const uint32_t f = side ? fl2 : fl, m = side ? it.mm >> 8 : it.mm & 0xffu;
+#pragma unroll
+                for (int c = 0; c < 9; ++c) {
+                    const ff v = s[c / 3][c % 3];
+                    const float g = c / 3 == 1 ? 1.0f : sgn;
+                    store[spring_at(aos, c, as, stride)] = make_float2(g * v.hi, g * v.lo);
+                }
+                const f3 fo = fm(sgn * o.force.x, sgn * o.force.y, sgn * o.force.z);
+                const f3 roll = fm(sgn * o.roll.x, sgn * o.roll.y, sgn * o.roll.z);
+                const f3 twist = fm(sgn * o.twist.x, sgn * o.twist.y, sgn * o.twist.z);
+                const f3 tau = torque_of(roll, o.slide, twist, o.rr, o.rp);
+                put(row, m, make_float4(fo.x * MX.bin_im, fo.y * MX.bin_im, fo.z * MX.bin_im, tau.x * MX.bin_iI),
+                    make_float4(tau.y * MX.bin_iI, tau.z * MX.bin_iI, 0.f, 0.f));
+                if (breaks) {
+                    const float st = (float)BV.strength[as];
+                    if (f2 > st * st) {
+                        BV.intact[as] = 0;
+                        PV.flags[es] = f & ~(kBonded | (0xffu << 8));
+                    }
+                } else if (!(f & (kBonded | kXiLive))) {
+                    PV.flags[es] = f | kXiLive;
+                }
+                sgn = -1.0f;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Contact part of row i's accelerations from its entries' records: T running sums over entries 0, T, ...
+// and 1, T + 1, ..., then added in order (the order in which contact_rows with T lanes per row adds them).
+template <int T>
+__device__ __forceinline__ void contact_sums(const PairView &PV, const NearScratch &R, int64_t n, int64_t i,
+                                             ff (&a)[3], ff (&al)[3]) {
+    ff acc[T][6];
+#pragma unroll
+    for (int t = 0; t < T; ++t)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) acc[t][c] = ff{0.f, 0.f};
+    constexpr int kAhead = 4;  // entries loaded with the row's count, before it is known (every row has them)
+    float4 p[kAhead], q[kAhead];
+    const int len = PV.near_len[i];
+    const bool ahead = PV.cap >= kAhead;
+    for (int m = 0; m == 0 || m < len; m += kAhead) {
+#pragma unroll
+        for (int t = 0; t < kAhead; ++t) {
+            if (m == 0 ? ahead || t < len : m + t < len) {
+                const float4 *rec = R.rec + 2 * ((int64_t)(m + t) * n + i);
+                p[t] = rec[0];
+                q[t] = rec[1];
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < kAhead; ++t) {
+            if (m + t < len) {
+                ff(&s)[6] = acc[t % T];
+                ff_acc(s[0], p[t].x);
+                ff_acc(s[1], p[t].y);
+                ff_acc(s[2], p[t].z);
+                ff_acc(s[3], p[t].w);
+                ff_acc(s[4], q[t].x);
+                ff_acc(s[5], q[t].y);
             }
         }
     }
-    if (!active) return;
-    MX.hsum[2 * i] = make_float4(acch[0].hi, acch[0].lo, acch[1].hi, acch[1].lo);
-    MX.hsum[2 * i + 1] = make_float4(acch[2].hi, acch[2].lo, 0.f, 0.f);
+#pragma unroll
+    for (int t = 1; t < T; ++t)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+            ff_acc(acc[0][c], acc[t][c].hi);
+            ff_acc(acc[0][c], acc[t][c].lo);
+        }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        a[c] = acc[0][c];
+        al[c] = acc[0][3 + c];
+    }
+}
+
+// The contact part of row i: from the records (R.rec) or from the contact kernel's sums (MX.csum).
+__device__ __forceinline__ void contact_part(const PairView &PV, const NearScratch &R, const MixedExtra &MX, int64_t n,
+                                             int64_t i, ff (&a)[3], ff (&al)[3]) {
+    if (R.rec) {
+        if (R.lanes == 2) contact_sums<2>(PV, R, n, i, a, al);
+        else contact_sums<1>(PV, R, n, i, a, al);
+        return;
+    }
+    const float4 c0 = MX.csum[3 * i], c1 = MX.csum[3 * i + 1], c2 = MX.csum[3 * i + 2];
+    a[0] = ff{c0.x, c0.y};
+    a[1] = ff{c0.z, c0.w};
+    a[2] = ff{c1.x, c1.y};
+    al[0] = ff{c1.z, c1.w};
+    al[1] = ff{c2.x, c2.y};
+    al[2] = ff{c2.z, c2.w};
+}
+
+// Hamaker pairs: hsum receives the Hamaker part of the row's acceleration as a float-float sum. L lanes
+// per row, lane l taking windows l, l + L, ... of kWin slots and evaluating their pairs from registers
+// (the partner indices of its next window are loaded meanwhile). The windows' sums are added in the order
+// that SL slices define, whatever L is: slice s adds windows s, s + SL, ... one after another, then the
+// slices are added in order.
+template <bool VERLET, int HM, int L, int SL>
+__global__ void __launch_bounds__(kHThreads, L == 1 ? 6 : 7) forces_hamaker_mixed(Params P, PairView PV, MixedExtra MX) {
+    static_assert(L % SL == 0 && 32 % L == 0, "a row's lanes hold whole slices");
+    const int lane = threadIdx.x & 31, l = lane % L, base = lane - l;
+    const int64_t n = P.n;
+    const int64_t i = ((int64_t)blockIdx.x * kHThreads + threadIdx.x) / L;
+    const bool active = i < n;
+    int32_t len = 0;
+    float4 xh = make_float4(0.f, 0.f, 0.f, 0.f), xl = xh;
+    if (active) {
+        len = VERLET ? PV.row_len[i] : (int32_t)(n - 1);
+        xh = MX.x32[2 * i];
+        xl = MX.x32[2 * i + 1];
+    }
+    const int32_t maxlen = (int32_t)__reduce_max_sync(0xffffffffu, (unsigned)len);
+    ff acc[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};  // of slice l % SL
+    int32_t jn[kWin];
+    window_partners<VERLET>(PV, n, i, len, l * kWin, jn);
+    for (int32_t k0 = 0; k0 < maxlen; k0 += L * kWin) {
+        int32_t j[kWin];
+#pragma unroll
+        for (int u = 0; u < kWin; ++u) j[u] = jn[u];
+        window_partners<VERLET>(PV, n, i, len, k0 + (L + l) * kWin, jn);
+        const f3 w = window_sum<HM>(MX, xh, xl, j);
+        if (L == SL) {
+            ff_acc(acc[0], w.x);
+            ff_acc(acc[1], w.y);
+            ff_acc(acc[2], w.z);
+        } else {
+#pragma unroll
+            for (int t = 0; t < L / SL; ++t) {
+                const int src = base + l % SL + t * SL;
+                ff_acc(acc[0], __shfl_sync(0xffffffffu, w.x, src));
+                ff_acc(acc[1], __shfl_sync(0xffffffffu, w.y, src));
+                ff_acc(acc[2], __shfl_sync(0xffffffffu, w.z, src));
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 1; q < SL; ++q) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float hi = __shfl_sync(0xffffffffu, acc[c].hi, base + q), lo = __shfl_sync(0xffffffffu, acc[c].lo, base + q);
+            if (l == 0) {
+                ff_acc(acc[c], hi);
+                ff_acc(acc[c], lo);
+            }
+        }
+    }
+    if (!active || l != 0) return;
+    MX.hsum[2 * i] = make_float4(acc[0].hi, acc[0].lo, acc[1].hi, acc[1].lo);
+    MX.hsum[2 * i + 1] = make_float4(acc[2].hi, acc[2].lo, 0.f, 0.f);
 }
 
 // Completion of row i in FP64: contact part (csum when `contacts`) plus the Hamaker part (hsum when
@@ -124,11 +368,12 @@ __global__ void __launch_bounds__(ShapeH<SL>::kWarps * 32, ShapeH<SL>::kMinBlock
 // the next step's opening half kick and drift, and the float-float copies of the new state.
 template <bool FACETS>
 __device__ __forceinline__ void finish_fp64_row(const Params &P, const StateView &S, int64_t i, double hdt, double dt,
-                                                int contacts, int hamaker, int kick, const MixedExtra &MX) {
+                                                int contacts, int hamaker, int kick, const MixedExtra &MX,
+                                                const PairView &PV, const NearScratch &R) {
     // every input is loaded before anything is stored (the buffers are distinct)
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 c0 = contacts ? MX.csum[3 * i] : z4, c1 = contacts ? MX.csum[3 * i + 1] : z4,
-                 c2 = contacts ? MX.csum[3 * i + 2] : z4;
+    ff ac[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}}, alc[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+    if (contacts) contact_part(PV, R, MX, P.n, i, ac, alc);
     const float4 h0 = hamaker ? MX.hsum[2 * i] : z4, h1 = hamaker ? MX.hsum[2 * i + 1] : z4;
     const d3 vi = ld4(S.v, i), wi = ld4(S.w, i);
     d3 xo = zero3(), tho = zero3();
@@ -137,8 +382,8 @@ __device__ __forceinline__ void finish_fp64_row(const Params &P, const StateView
         tho = ld4(S.th, i);
     }
     // contact part (float-float pairs hi, lo), then the Hamaker part
-    d3 a_tot = mk3((double)c0.x + (double)c0.y, (double)c0.z + (double)c0.w, (double)c1.x + (double)c1.y);
-    d3 al_tot = mk3((double)c1.z + (double)c1.w, (double)c2.x + (double)c2.y, (double)c2.z + (double)c2.w);
+    d3 a_tot = mk3(ff_to_d(ac[0]), ff_to_d(ac[1]), ff_to_d(ac[2]));
+    d3 al_tot = mk3(ff_to_d(alc[0]), ff_to_d(alc[1]), ff_to_d(alc[2]));
     if (hamaker) {
         const d3 ah = mk3((double)h0.x + (double)h0.y, (double)h0.z + (double)h0.w, (double)h1.x + (double)h1.y);
         a_tot = contacts ? add(a_tot, ah) : ah;
@@ -163,11 +408,11 @@ __device__ __forceinline__ void finish_fp64_row(const Params &P, const StateView
 template <bool FACETS>
 __global__ void __launch_bounds__(64) forces_finish_mixed(Params P, StateView S, double hdt, double dt,
                                                           int move_facets, int contacts, int hamaker, int kick,
-                                                          MixedExtra MX) {
+                                                          MixedExtra MX, PairView PV, NearScratch R) {
     if (move_facets && blockIdx.x == 0 && threadIdx.x == 0) compact::move_facets(P, S, dt);
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= P.n || inactive_of(P.hold, i)) return;
-    finish_fp64_row<FACETS>(P, S, i, hdt, dt, contacts, hamaker, kick, MX);
+    finish_fp64_row<FACETS>(P, S, i, hdt, dt, contacts, hamaker, kick, MX, PV, R);
 }
 
 // Completion of a step of a run (no facets, no body term), integrating in float-float on the FP32
@@ -185,22 +430,21 @@ __global__ void __launch_bounds__(64) forces_finish_mixed(Params P, StateView S,
 // rotation hi / lo.
 template <bool LAST>
 __global__ void __launch_bounds__(64) forces_finish_ff(Params P, StateView S, int contacts, int hamaker, ff hdt, ff dt,
-                                                       double hdt_d, double dt_d, MixedExtra MX) {
+                                                       double hdt_d, double dt_d, MixedExtra MX, PairView PV,
+                                                       NearScratch R) {
     const int64_t n = P.n;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t h = hold_of(P.hold, i);
     if (h & kHoldInactive) return;  // takes no part
     if (h) {  // a held particle keeps its FP64 state current (a held value stays exactly as it was)
-        finish_fp64_row<false>(P, S, i, hdt_d, dt_d, contacts, hamaker, LAST ? 0 : 1, MX);
+        finish_fp64_row<false>(P, S, i, hdt_d, dt_d, contacts, hamaker, LAST ? 0 : 1, MX, PV, R);
         return;
     }
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 c0 = contacts ? MX.csum[3 * i] : z4, c1 = contacts ? MX.csum[3 * i + 1] : z4,
-                 c2 = contacts ? MX.csum[3 * i + 2] : z4;
     const float4 h0 = hamaker ? MX.hsum[2 * i] : z4, h1 = hamaker ? MX.hsum[2 * i + 1] : z4;
-    ff a[3] = {{c0.x, c0.y}, {c0.z, c0.w}, {c1.x, c1.y}};
-    const ff al[3] = {{c1.z, c1.w}, {c2.x, c2.y}, {c2.z, c2.w}};
+    ff a[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}}, al[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+    if (contacts) contact_part(PV, R, MX, n, i, a, al);
     if (hamaker) {
         const ff ah[3] = {{h0.x, h0.y}, {h0.z, h0.w}, {h1.x, h1.y}};
 #pragma unroll
@@ -226,22 +470,15 @@ void launch_contacts(const Params &P, const StateView &S, const PairView &PV, co
         forces_contacts_mixed<NEAR, T, LG_CONTACT_MIN_BLOCKS_ALONE><<<blocks, kCWarps * 32, smem, st>>>(P, S, PV, BV, MX);
 }
 
-template <bool VERLET, int SL>
+template <bool VERLET, int L, int SL>
 void launch_hamaker(const Params &P, const PairView &PV, const MixedExtra &MX, cudaStream_t st) {
-    using Sh = ShapeH<SL>;
-    const size_t smem = sizeof(HamakerSmem) * Sh::kWarps;
-    const int64_t rows_per_block = Sh::kRowWarps * 32;
-    const unsigned blocks = (unsigned)((P.n + rows_per_block - 1) / rows_per_block);
-    if (smem > 48 * 1024) {  // above the default dynamic shared-memory limit: opt in, once per device
-        static thread_local int attr_device = -1;
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (attr_device != dev) {
-            cudaFuncSetAttribute(forces_hamaker_mixed<VERLET, SL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            attr_device = dev;
-        }
-    }
-    forces_hamaker_mixed<VERLET, SL><<<blocks, Sh::kWarps * 32, smem, st>>>(P, PV, MX);
+    const unsigned blocks = (unsigned)((P.n * L + kHThreads - 1) / kHThreads);
+    if (P.hamaker_model == LG_HAMAKER_LIMITED)
+        forces_hamaker_mixed<VERLET, LG_HAMAKER_LIMITED, L, SL><<<blocks, kHThreads, 0, st>>>(P, PV, MX);
+    else if (P.hamaker_model == LG_HAMAKER_SIMPLIFIED)
+        forces_hamaker_mixed<VERLET, LG_HAMAKER_SIMPLIFIED, L, SL><<<blocks, kHThreads, 0, st>>>(P, PV, MX);
+    else
+        forces_hamaker_mixed<VERLET, LG_HAMAKER_FULL, L, SL><<<blocks, kHThreads, 0, st>>>(P, PV, MX);
 }
 
 }  // namespace
@@ -268,10 +505,20 @@ static int mixed_hamaker_slices_all_pairs(int64_t n) {
     return 1;
 }
 
+// Rows per block of owned contact candidates (about 1.8 a row in an aggregate, somewhat more than half of
+// them touching): a block's candidates are about two per thread of 128, 64 or 32, and its touching pairs
+// one per thread.
+int32_t near_block_rows(int64_t n) { return n >= 32768 ? 128 : n >= 8192 ? 64 : 32; }
+
+void launch_near_owners(int64_t n, const PairView &PV, const NearScratch &R, cudaStream_t st) {
+    const unsigned blocks = (unsigned)((n + R.rb - 1) / R.rb);
+    if (blocks) near_owners<<<blocks, 4 * (unsigned)R.rb, 0, st>>>(n, PV, R);  // four lanes per row
+}
+
 int launch_forces_compact_mixed(const Params &P, const StateView &S, const PairView &PV, const BondView &BV, double hdt,
                                 double dt, int move_facets, bool kick, bool prev_fused, const MixedExtra &MX,
                                 cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int slices,
-                                int contact_lanes) {
+                                int contact_lanes, NearScratch R) {
     const bool ver = P.pairs == LG_PAIRS_VERLET;
     const int contacts = P.binary_model != LG_BINARY_NONE ? 1 : 0;
     const int hamaker = P.hamaker_model != LG_HAMAKER_NONE ? 1 : 0;
@@ -282,7 +529,14 @@ int launch_forces_compact_mixed(const Params &P, const StateView &S, const PairV
         // the FP64 positions are current unless the step before integrated in float-float
         MixedExtra MC = MX;
         MC.x64 = prev_fused ? nullptr : S.x;
-        if (ver && PV.near_len && contact_lanes == 1)
+        if (!(ver && PV.near_len)) R.rec = nullptr;
+        R.lanes = contact_lanes == 1 ? 1 : 2;
+        if (R.rec) {
+            const unsigned nb = (unsigned)((P.n + R.rb - 1) / R.rb);
+            if (R.rb == 128) mixed_contacts<128><<<nb, 128, 0, side>>>(P, PV, BV, MC, R);
+            else if (R.rb == 64) mixed_contacts<64><<<nb, 64, 0, side>>>(P, PV, BV, MC, R);
+            else mixed_contacts<32><<<nb, 32, 0, side>>>(P, PV, BV, MC, R);
+        } else if (ver && PV.near_len && contact_lanes == 1)
             launch_contacts<true, 1>(P, S, PV, BV, MC, side, hamaker != 0);
         else if (ver && PV.near_len)
             launch_contacts<true, kContactLanes>(P, S, PV, BV, MC, side, hamaker != 0);
@@ -293,24 +547,24 @@ int launch_forces_compact_mixed(const Params &P, const StateView &S, const PairV
     if (hamaker) {
         switch (slices > 0 ? slices : ver ? mixed_hamaker_slices(P.n) : mixed_hamaker_slices_all_pairs(P.n)) {
             case 16:
-                if (ver) launch_hamaker<true, 16>(P, PV, MX, st);
-                else launch_hamaker<false, 16>(P, PV, MX, st);
+                if (ver) launch_hamaker<true, 16, 16>(P, PV, MX, st);
+                else launch_hamaker<false, 32, 16>(P, PV, MX, st);
                 break;
             case 8:
-                if (ver) launch_hamaker<true, 8>(P, PV, MX, st);
-                else launch_hamaker<false, 8>(P, PV, MX, st);
+                if (ver) launch_hamaker<true, 8, 8>(P, PV, MX, st);
+                else launch_hamaker<false, 32, 8>(P, PV, MX, st);
                 break;
             case 4:
-                if (ver) launch_hamaker<true, 4>(P, PV, MX, st);
-                else launch_hamaker<false, 4>(P, PV, MX, st);
+                if (ver) launch_hamaker<true, 4, 4>(P, PV, MX, st);
+                else launch_hamaker<false, 16, 4>(P, PV, MX, st);
                 break;
             case 2:
-                if (ver) launch_hamaker<true, 2>(P, PV, MX, st);
-                else launch_hamaker<false, 2>(P, PV, MX, st);
+                if (ver) launch_hamaker<true, 2, 2>(P, PV, MX, st);
+                else launch_hamaker<false, 8, 2>(P, PV, MX, st);
                 break;
             default:
-                if (ver) launch_hamaker<true, 1>(P, PV, MX, st);
-                else launch_hamaker<false, 1>(P, PV, MX, st);
+                if (ver) launch_hamaker<true, 1, 1>(P, PV, MX, st);
+                else launch_hamaker<false, 8, 1>(P, PV, MX, st);
         }
         ++kernels;
     }
@@ -324,17 +578,17 @@ int launch_forces_compact_mixed(const Params &P, const StateView &S, const PairV
     const bool plain = P.n_facets == 0 && !P.ext_a && MX.s32;
     auto split = [](double d) { const float hi = (float)d; return ff{hi, (float)(d - (double)hi)}; };
     if (plain && kick) {
-        forces_finish_ff<false><<<blocks, 64, 0, st>>>(P, S, contacts, hamaker, split(hdt), split(dt), hdt, dt, MX);
+        forces_finish_ff<false><<<blocks, 64, 0, st>>>(P, S, contacts, hamaker, split(hdt), split(dt), hdt, dt, MX, PV, R);
         return kernels;
     }
     if (plain && prev_fused) {
-        forces_finish_ff<true><<<blocks, 64, 0, st>>>(P, S, contacts, hamaker, split(hdt), split(dt), hdt, dt, MX);
+        forces_finish_ff<true><<<blocks, 64, 0, st>>>(P, S, contacts, hamaker, split(hdt), split(dt), hdt, dt, MX, PV, R);
         return kernels;
     }
     if (P.n_facets > 0 || P.ext_a)
-        forces_finish_mixed<true><<<blocks, 64, 0, st>>>(P, S, hdt, dt, move_facets, contacts, hamaker, kick ? 1 : 0, MX);
+        forces_finish_mixed<true><<<blocks, 64, 0, st>>>(P, S, hdt, dt, move_facets, contacts, hamaker, kick ? 1 : 0, MX, PV, R);
     else
-        forces_finish_mixed<false><<<blocks, 64, 0, st>>>(P, S, hdt, dt, 0, contacts, hamaker, kick ? 1 : 0, MX);
+        forces_finish_mixed<false><<<blocks, 64, 0, st>>>(P, S, hdt, dt, 0, contacts, hamaker, kick ? 1 : 0, MX, PV, R);
     return kernels;
 }
 

@@ -9,7 +9,7 @@ namespace lg {
 
 struct GridDev {
     double lo[3];
-    double edge;
+    float inv_edge;  // 1 / cell edge
     int64_t dim[3];
     int64_t ncell;
     float rv2_lo, rv2_hi;  // FP32 accept / reject bounds of the squared list radius
@@ -30,10 +30,10 @@ struct ListScratch {
     GridDev *grid;     // device grid description
     int32_t *cell_of;  // [n]
     int32_t *count;    // [max_cells]
-    int32_t *start;    // [max_cells]
-    int32_t *fill;     // [max_cells]
+    int32_t *start;    // [max_cells] begin of every cell in the sorted list, then its end
     int32_t *sorted;   // [n]
-    int32_t *tile;     // [max_cells / 4096 + 1] cell-scan tile totals, then their offsets
+    unsigned *ticket;  // finished blocks of the bounding-box pass (zero between builds)
+    int32_t *cursor;   // places of the sorted list taken so far
     float4 *x32;       // [n] positions relative to the grid origin, FP32 (candidate filter)
     int32_t *max_row;  // [1] longest row found by the last build (before truncation)
 };
@@ -169,6 +169,19 @@ int launch_step_mixed(const Params &P, const StateView &S, const PairView &PV, c
                       const MixedExtra &MX, const StepArgs &A, cudaStream_t st, cudaStream_t side = nullptr,
                       cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr);
 
+// Scratch of the mixed contact kernel that evaluates a pair once for both rows (rec null: the kernel that
+// evaluates it from each row's side runs instead).
+struct NearScratch {
+    float4 *rec;     // [cap * n][2] per contact candidate: accelerations a (3), alpha (3)
+    uint4 *own;      // [cap * n] owned candidates of each block of rb rows (the block's from row0 * cap on)
+    int32_t *own_n;  // [ceil(n / rb)] owned candidates per block
+    int32_t rb;
+    int32_t lanes;   // running sums per row (1 or 2), as the other kernel's lanes per row add them
+};
+int32_t near_block_rows(int64_t n);
+// Lists the owned contact candidates of every block (after each list build).
+void launch_near_owners(int64_t n, const PairView &PV, const NearScratch &R, cudaStream_t st);
+
 // Warp-compacted mixed-precision kernels (lg_forces_compact_mixed.cu): the contact/bond kernel (if the system has a binary model) on `side`, beside the
 // Hamaker kernel on `st` (fork / join through the two events), then the completion kernel on `st`;
 // returns the number of kernels launched.
@@ -180,8 +193,8 @@ int launch_step_mixed(const Params &P, const StateView &S, const PairView &PV, c
 // row of the contact kernel over candidate lists (1 or 2; all pairs take a warp per row).
 int launch_forces_compact_mixed(const Params &P, const StateView &S, const PairView &PV, const BondView &BV, double hdt,
                                 double dt, int move_facets, bool kick, bool prev_fused, const MixedExtra &MX,
-                                cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int slices = 0,
-                                int contact_lanes = 2);
+                                cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int slices,
+                                int contact_lanes, NearScratch R);
 
 // Layout conversion between a caller's [n][3] doubles (already in device memory) and the padded
 // device layout (lg_reduce.cu).

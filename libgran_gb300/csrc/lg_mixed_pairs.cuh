@@ -22,7 +22,6 @@
 namespace lg {
 namespace mixed {
 
-using compact::kHCap;
 using compact::kWin;
 
 // ---- contact / bond items ----
@@ -45,15 +44,6 @@ struct ContactSmem {
     float4 vh[32], vl[32];  // the rows' own velocities (float-float)
     float4 wh[32];          // the rows' own spins (FP32)
 };
-
-// ---- Hamaker items ----
-struct HamakerSmem {
-    float4 hhi[kHCap];     // queued Hamaker partners: high part of the position, w = owner lane
-    float4 hlo[kHCap];     // low part of the position
-    float hres[kHCap][3];  // their accelerations
-    float4 xh[32], xl[32];  // the rows' own positions (float-float)
-};
-static_assert(sizeof(HamakerSmem::hhi) >= 6 * 32 * sizeof(float), "slice partial sums reuse hhi");
 
 struct f3 {
     float x, y, z;
@@ -179,6 +169,79 @@ __device__ __forceinline__ SepFF separation_ff(float4 hi, float4 lo, float4 hj, 
     return SepFF{fm(tx.hi + lx, ty.hi + ly, tz.hi + lz), s3 + rest};
 }
 
+// One contact or bond pair (contact_force.h:57-147, alt_sinter_bridge.h:103-156) from the two particles'
+// float-float positions and velocities and FP32 spins: the force on i, and the three parts of its torque
+// (rr n x f_r, rp n x f_t, rr f_o). The springs s (xi_t, xi_r, xi_o) are updated. Returns false, with
+// nothing done, when the pair does not touch.
+//
+// Seen from j (everything swapped) the normal, the slip and the torsion change sign and the rolling
+// velocity does not, in every intermediate value and to the last bit (each operation rounds
+// symmetrically, and the two rotation terms are added to each other before anything else): the force is
+// the negative, xi_t and xi_o are the negatives, xi_r is the same, n x f_r and f_o are the negatives and
+// n x f_t is the same. mixed_contacts evaluates a pair once on that ground.
+struct Body {
+    float4 xh, xl, vh, vl, w;
+};
+struct ContactOut {
+    f3 force, roll, slide, twist;  // force; n x f_r, n x f_t, f_o
+    float rr, rp;
+};
+__device__ __forceinline__ Body body_of(const MixedExtra &M, int64_t n, int64_t i) {
+    return Body{M.x32[2 * i], M.x32[2 * i + 1], M.v32[i], M.v32[n + i], M.v32[2 * n + i]};
+}
+__device__ __forceinline__ f3 torque_of(const f3 &roll, const f3 &slide, const f3 &twist, float rr, float rp) {
+    return fadd(fsub(fscl(rr, roll), fscl(rp, slide)), fscl(rr, twist));
+}
+__device__ __forceinline__ bool contact_pair(const Params &P, const MixedExtra &M, bool bonded, int64_t i, int64_t j,
+                                             const Body &bi, const Body &bj, ff (&s)[3][3], ContactOut &o) {
+    const SepFF sp = separation_ff(bi.xh, bi.xl, bj.xh, bj.xl, bonded ? M.b_fr_hi : M.c_fr_hi,
+                                   bonded ? M.b_fr_lo : M.c_fr_lo);
+    const f3 dxf = sp.d;
+    const float d2f = fdot(dxf, dxf);
+    const float rr = bonded ? M.b_r : M.c_r;
+    const float rsd = rsqrtf(d2f);
+    // 2r - |d|, from |d|^2 - (2r)^2 (the product rounds on its own in every kernel: the same bits)
+    const float overlap = -sp.q / __fadd_rn(__fmul_rn(d2f, rsd), 2.0f * rr);
+    bool touching = bonded || overlap > 0.0f;
+    // spheres at the contact distance to within rounding (a seeded aggregate places touching
+    // monomers there): the FP64 path's overlap decides whether they touch
+    if (!bonded && M.x64 && fabsf(sp.q) <= M.q_marg) touching = overlap_fp64(M.x64, i, j, (double)P.contact.r_part) > 0.0;
+    if (!touching) return false;
+    const f3 n3 = fscl(rsd, dxf);
+    // relative velocity v_i - v_j from the float-float copies (exact high-part difference)
+    const ff tx = two_sum(bi.vh.x, -bj.vh.x), ty = two_sum(bi.vh.y, -bj.vh.y), tz = two_sum(bi.vh.z, -bj.vh.z);
+    const f3 vij0 = fm(tx.hi + (tx.lo + (bi.vl.x - bj.vl.x)), ty.hi + (ty.lo + (bi.vl.y - bj.vl.y)),
+                       tz.hi + (tz.lo + (bi.vl.z - bj.vl.z)));
+    const f3 wfi = fm(bi.w.x, bi.w.y, bi.w.z), wfj = fm(bj.w.x, bj.w.y, bj.w.z);
+    const float kn = bonded ? M.b_k : M.c_k, gn = bonded ? M.b_gn : M.c_gn;
+    const float rp = rr - 0.5f * overlap;
+    const float v_n = -fdot(vij0, n3);
+    const float f_n = kn * overlap + gn * v_n;
+    const f3 nwi = fcrs(n3, wfi), nwj = fcrs(n3, wfj);
+    const f3 v_ij = fadd(vij0, fscl(rp, fadd(nwi, nwj)));
+    const f3 v_t = fsub(v_ij, fscl(fdot(v_ij, n3), n3));
+    const f3 v_r = fscl(-rp, fsub(nwi, nwj));
+    const f3 v_o = fscl(rr * (fdot(n3, wfi) - fdot(n3, wfj)), n3);
+    f3 f_t, f_r, f_o;
+    if (bonded) {
+        f_t = shear_ff(s[0], n3, M.b_kt, M.b_gt, f_n, 0.f, 0.f, v_t, M.b_dt, false);
+        f_r = shear_ff(s[1], n3, M.b_kr, M.b_gr, f_n, 0.f, 0.f, v_r, M.b_dt, false);
+        f_o = shear_ff(s[2], n3, M.b_ko, M.b_go, f_n, 0.f, 0.f, v_o, M.b_dt, false);
+    } else {
+        f_t = shear_ff(s[0], n3, M.c_kt, M.c_gt, f_n, M.c_mus, M.c_phid, v_t, M.c_dt, true);
+        f_r = shear_ff(s[1], n3, M.c_kr, M.c_gr, f_n, M.c_mur, M.c_phir, v_r, M.c_dt, true);
+        f_o = shear_ff(s[2], n3, M.c_ko, M.c_go, f_n, M.c_muo, M.c_phio, v_o, M.c_dt, true);
+    }
+    o.force = fadd(fscl(f_n, n3), f_t);
+    o.roll = fcrs(n3, f_r);
+    o.slide = fcrs(n3, f_t);
+    o.twist = f_o;
+    o.rr = rr;
+    o.rp = rp;
+    return true;
+}
+
+// Entry q of a warp's contact queue (contact_rows): evaluates the pair from the row's side.
 __device__ __forceinline__ void contact_item(const Params &P, const PairView &PV, const BondView &BV,
                                              const MixedExtra &M, ContactSmem &W, int q, int64_t row0, int64_t n,
                                              int64_t xs, int64_t bs) {
@@ -188,23 +251,12 @@ __device__ __forceinline__ void contact_item(const Params &P, const PairView &PV
     const int32_t j = W.cj[q];
     const uint32_t fl = W.cfl[q];
     const bool bonded = (fl & kBonded) != 0;
-    int64_t base, stride;
-    float2 *store;
-    int32_t aos;
-    if (bonded) {
-        base = (int64_t)bond_slot_of(fl) * n + io;
-        stride = bs;
-        store = reinterpret_cast<float2 *>(BV.xi);
-        aos = BV.aos;
-    } else {
-        base = e;
-        stride = xs;
-        store = reinterpret_cast<float2 *>(PV.xi);
-        aos = PV.aos;
-    }
+    const int64_t base = bonded ? (int64_t)bond_slot_of(fl) * n + io : e, stride = bonded ? bs : xs;
+    float2 *store = reinterpret_cast<float2 *>(bonded ? BV.xi : PV.xi);
+    const int32_t aos = bonded ? BV.aos : PV.aos;
     // every load the pair may need is issued before any arithmetic (one memory round trip): the
     // partner's low position part, velocities and spin, and the springs of a live slot or bond
-    const float4 lj = M.x32[2 * j + 1], vhj = M.v32[j], vlj = M.v32[n + j], wj4 = M.v32[2 * n + j];
+    const Body bj{W.chj[q], M.x32[2 * j + 1], M.v32[j], M.v32[n + j], M.v32[2 * n + j]};
     ff s[3][3] = {};  // springs of a slot that is not live are zero
     if (bonded || (fl & kXiLive))
 #pragma unroll
@@ -212,51 +264,15 @@ __device__ __forceinline__ void contact_item(const Params &P, const PairView &PV
             const float2 v = store[spring_at(aos, c, base, stride)];
             s[c / 3][c % 3] = ff{v.x, v.y};
         }
-    const SepFF sp = separation_ff(W.xh[own], W.xl[own], W.chj[q], lj, bonded ? M.b_fr_hi : M.c_fr_hi,
-                                   bonded ? M.b_fr_lo : M.c_fr_lo);
-    const f3 dxf = sp.d;
-    const float d2f = fdot(dxf, dxf);
-    const float rr = bonded ? M.b_r : M.c_r;
-    const float rsd = rsqrtf(d2f);
-    const float overlap = -sp.q / (d2f * rsd + 2.0f * rr);  // 2r - |d|, from |d|^2 - (2r)^2
-    bool touching = bonded || overlap > 0.0f;
-    // spheres at the contact distance to within rounding (a seeded aggregate places touching
-    // monomers there): the FP64 path's overlap decides whether they touch
-    if (!bonded && M.x64 && fabsf(sp.q) <= M.q_marg) touching = overlap_fp64(M.x64, io, j, (double)P.contact.r_part) > 0.0;
+    const Body bi{W.xh[own], W.xl[own], W.vh[own], W.vl[own], W.wh[own]};
+    ContactOut o;
     f3 force = fm(0.f, 0.f, 0.f), torque = fm(0.f, 0.f, 0.f);
-    if (touching) {
-        const f3 n3 = fscl(rsd, dxf);
-        // relative velocity v_i - v_j from the float-float copies (exact high-part difference)
-        const float4 vhi = W.vh[own], vlo = W.vl[own];
-        const ff tx = two_sum(vhi.x, -vhj.x), ty = two_sum(vhi.y, -vhj.y), tz = two_sum(vhi.z, -vhj.z);
-        const f3 vij0 = fm(tx.hi + (tx.lo + (vlo.x - vlj.x)), ty.hi + (ty.lo + (vlo.y - vlj.y)),
-                           tz.hi + (tz.lo + (vlo.z - vlj.z)));
-        const float4 wo4 = W.wh[own];
-        const f3 wfi = fm(wo4.x, wo4.y, wo4.z), wfj = fm(wj4.x, wj4.y, wj4.z);
-        const float kn = bonded ? M.b_k : M.c_k, gn = bonded ? M.b_gn : M.c_gn;
-        const float rp = rr - 0.5f * overlap;
-        const float v_n = -fdot(vij0, n3);
-        const float f_n = kn * overlap + gn * v_n;
-        const f3 nwi = fcrs(n3, wfi), nwj = fcrs(n3, wfj);
-        const f3 v_ij = fadd(vij0, fscl(rp, fadd(nwi, nwj)));
-        const f3 v_t = fsub(v_ij, fscl(fdot(v_ij, n3), n3));
-        const f3 v_r = fscl(-rp, fsub(nwi, nwj));
-        const f3 v_o = fscl(rr * (fdot(n3, wfi) - fdot(n3, wfj)), n3);
-        f3 f_t, f_r, f_o;
-        if (bonded) {
-            f_t = shear_ff(s[0], n3, M.b_kt, M.b_gt, f_n, 0.f, 0.f, v_t, M.b_dt, false);
-            f_r = shear_ff(s[1], n3, M.b_kr, M.b_gr, f_n, 0.f, 0.f, v_r, M.b_dt, false);
-            f_o = shear_ff(s[2], n3, M.b_ko, M.b_go, f_n, 0.f, 0.f, v_o, M.b_dt, false);
-        } else {
-            f_t = shear_ff(s[0], n3, M.c_kt, M.c_gt, f_n, M.c_mus, M.c_phid, v_t, M.c_dt, true);
-            f_r = shear_ff(s[1], n3, M.c_kr, M.c_gr, f_n, M.c_mur, M.c_phir, v_r, M.c_dt, true);
-            f_o = shear_ff(s[2], n3, M.c_ko, M.c_go, f_n, M.c_muo, M.c_phio, v_o, M.c_dt, true);
-        }
+    if (contact_pair(P, M, bonded, io, j, bi, bj, s, o)) {
 #pragma unroll
         for (int c = 0; c < 9; ++c)
             store[spring_at(aos, c, base, stride)] = make_float2(s[c / 3][c % 3].hi, s[c / 3][c % 3].lo);
-        force = fadd(fscl(f_n, n3), f_t);
-        torque = fadd(fsub(fscl(rr, fcrs(n3, f_r)), fscl(rp, fcrs(n3, f_t))), fscl(rr, f_o));
+        force = o.force;
+        torque = torque_of(o.roll, o.slide, o.twist, o.rr, o.rp);
         if (bonded) {
             if (P.binary_model == LG_BINARY_BREAKING_SINTER) {
                 const float st = (float)BV.strength[base];
@@ -281,27 +297,72 @@ __device__ __forceinline__ void contact_item(const Params &P, const PairView &PV
     W.cres[q][5] = torque.z * M.bin_iI;
 }
 
-// One queued Hamaker pair (hamaker_force.h:28-44; limited form hamaker_force.h:86-93): partner
-// position from the queue, owner position from the warp's row data.
-__device__ __forceinline__ void hamaker_item(const Params &P, const MixedExtra &M, HamakerSmem &W, int q) {
-    const float4 ph = W.hhi[q];
-    const int own = __float_as_int(ph.w);
-    const SepFF sp = separation_ff(W.xh[own], W.xl[own], ph, W.hlo[q], M.h_fr_hi, M.h_fr_lo);
-    f3 a = fm(0.f, 0.f, 0.f);
-    if (!(P.hamaker_model == LG_HAMAKER_LIMITED && sp.q > M.h_qcut)) {
-        const f3 dxf = sp.d;
-        const float d2f = fdot(dxf, dxf);
-        const float rsd = rsqrtf(d2f);
-        float h = sp.q / (d2f * rsd + 2.0f * M.h_r);  // |d| - 2r to FP32 precision
-        h = fmaxf(h, M.h_h0);
-        const float sfac = ham_factor(P.hamaker_model, M.h_A, M.h_r, h) * M.inv_mass_h * rsd;
-        a = fscl(-sfac, dxf);  // along x_j - x_i
-    }
-    W.hres[q][0] = a.x;
-    W.hres[q][1] = a.y;
-    W.hres[q][2] = a.z;
+// The Hamaker acceleration of a row's particle towards one partner (hamaker_force.h:28-44; limited form
+// hamaker_force.h:86-93). Its last product and the sums over it round on their own (no fused add), so
+// that every kernel that adds these terms gives the same bits.
+__device__ __forceinline__ f3 hamaker_pair(int hm, const MixedExtra &M, float4 xh, float4 xl, float4 ph, float4 pl) {
+    const SepFF sp = separation_ff(xh, xl, ph, pl, M.h_fr_hi, M.h_fr_lo);
+    const f3 dxf = sp.d;
+    const float d2f = fdot(dxf, dxf);
+    const float rsd = rsqrtf(d2f);
+    float h = sp.q / (d2f * rsd + 2.0f * M.h_r);  // |d| - 2r to FP32 precision
+    h = fmaxf(h, M.h_h0);
+    const float sfac = ham_factor(hm, M.h_A, M.h_r, h) * M.inv_mass_h * rsd;
+    if (hm == LG_HAMAKER_LIMITED && sp.q > M.h_qcut) return fm(0.f, 0.f, 0.f);
+    return fm(__fmul_rn(-sfac, dxf.x), __fmul_rn(-sfac, dxf.y), __fmul_rn(-sfac, dxf.z));  // along x_j - x_i
 }
 
+// Partners of row i in the window of kWin slots from slot k0 on (-1: past the row's end).
+template <bool VERLET>
+__device__ __forceinline__ void window_partners(const PairView &PV, int64_t n, int64_t i, int32_t len, int32_t k0,
+                                                int32_t (&j)[kWin]) {
+    const char *row = VERLET ? reinterpret_cast<const char *>(PV.nbr + i) : nullptr;
+    const uint32_t pitch = 4u * (uint32_t)n;  // bytes from slot to slot (n <= 2^30)
+#pragma unroll
+    for (int u = 0; u < kWin; ++u) {
+        const int32_t k = k0 + u;
+        j[u] = -1;
+        if (k < len)
+            j[u] = VERLET ? *reinterpret_cast<const int32_t *>(row + (uint64_t)(uint32_t)k * pitch)
+                          : (k < (int32_t)i ? k : k + 1);
+    }
+}
+
+// Sum of a window's Hamaker terms in slot order (FP32; the windows' sums are added with compensation).
+// Every slot is evaluated and the ones out of range are left out of the sum: without branches the four
+// evaluations overlap.
+template <int HM>
+__device__ __forceinline__ f3 window_sum(const MixedExtra &MX, float4 xh, float4 xl, const int32_t (&j)[kWin]) {
+    float4 ph[kWin], pl[kWin];
+#pragma unroll
+    for (int u = 0; u < kWin; ++u) {
+        ph[u] = xh;
+        pl[u] = xl;
+        if (j[u] >= 0) {
+            const float4 *p = MX.x32 + 2 * (int64_t)j[u];
+            ph[u] = p[0];
+            pl[u] = p[1];
+        }
+    }
+    f3 sum = fm(0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < kWin; ++u) {
+        bool on = j[u] >= 0;
+        if (HM == LG_HAMAKER_LIMITED) {
+            const float dx = xh.x - ph[u].x, dy = xh.y - ph[u].y, dz = xh.z - ph[u].z;
+            on = on && fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= MX.near2;
+        }
+        const f3 a = hamaker_pair(HM, MX, xh, xl, ph[u], pl[u]);
+        sum = fm(on ? __fadd_rn(sum.x, a.x) : sum.x, on ? __fadd_rn(sum.y, a.y) : sum.y,
+                 on ? __fadd_rn(sum.z, a.z) : sum.z);
+    }
+    return sum;
+}
+__device__ __forceinline__ f3 window_sum(int hm, const MixedExtra &MX, float4 xh, float4 xl, const int32_t (&j)[kWin]) {
+    if (hm == LG_HAMAKER_LIMITED) return window_sum<LG_HAMAKER_LIMITED>(MX, xh, xl, j);
+    if (hm == LG_HAMAKER_SIMPLIFIED) return window_sum<LG_HAMAKER_SIMPLIFIED>(MX, xh, xl, j);
+    return window_sum<LG_HAMAKER_FULL>(MX, xh, xl, j);
+}
 
 // Float-float sum and product (the product's rounding error from an FMA; results renormalised).
 __device__ __forceinline__ ff ff_add(ff a, ff b) {
@@ -474,114 +535,24 @@ __device__ __forceinline__ void contact_rows(const Params &P, const PairView &PV
     MX.csum[3 * i + 2] = make_float4(accw[1].hi, accw[1].lo, accw[2].hi, accw[2].lo);
 }
 
-// Virtual slot v of slice sl of kSlices (its windows sl, sl + kSlices, ...) -> slot of the row; the
-// same mapping as compact::slot_of with the slice count known at run time.
-__device__ __forceinline__ int64_t slot_at(int64_t v, int sl, int kSlices) {
-    return ((v / kWin) * kSlices + sl) * kWin + (v % kWin);
-}
-
-// Hamaker pairs of rows row0 .. row0 + 31 (one warp), slice sl of kSlices: the windows sl,
-// sl + kSlices, ... of every row. acch receives the lane's row's partial sum (float-float).
+// Hamaker pairs of row row0 + lane, slice sl of kSlices: the windows sl, sl + kSlices, ... acch receives
+// the row's partial sum (float-float).
 template <bool VERLET>
-__device__ __forceinline__ void hamaker_rows(const Params &P, const PairView &PV, const MixedExtra &MX,
-                                             HamakerSmem &W, int64_t row0, int sl, int kSlices, int lane,
-                                             ff (&acch)[3]) {
-    const int64_t n = P.n;
-    const int64_t i = row0 + lane;
-    const bool active = i < n;
-    const int hm = P.hamaker_model;
-    const uint32_t lt = (1u << lane) - 1u;
-
-    int64_t len = 0;
-    float4 hi_i = make_float4(0.f, 0.f, 0.f, 0.f);
-    {
-        float4 lo_i = hi_i;
-        if (active) {
-            len = VERLET ? (int64_t)PV.row_len[i] : n - 1;
-            hi_i = MX.x32[2 * i];
-            lo_i = MX.x32[2 * i + 1];
-        }
-        W.xh[lane] = hi_i;
-        W.xl[lane] = lo_i;
-    }
-    const int64_t maxlen = (int64_t)__reduce_max_sync(0xffffffffu, (unsigned)len);
-    // this warp's windows: sl, sl + kSlices, ...; virtual slot v maps to slot_at(v, sl, kSlices)
-    const int64_t nwin = (maxlen + kWin - 1) / kWin;
-    const int64_t mywin = nwin > sl ? (nwin - sl + kSlices - 1) / kSlices : 0;
-    const int64_t vmax = mywin * kWin;
+__device__ __forceinline__ void hamaker_rows(const Params &P, const PairView &PV, const MixedExtra &MX, int64_t row0,
+                                             int sl, int kSlices, int lane, ff (&acch)[3]) {
+    const int64_t n = P.n, i = row0 + lane;
     acch[0] = acch[1] = acch[2] = ff{0.f, 0.f};
-    __syncwarp();
-
-    // partners of the lane's row in the window at virtual slot v (-1: past the row's end)
-    int32_t jn[kWin];
-    auto load_window = [&](int64_t v) {
-        const int64_t k0 = slot_at(v, sl, kSlices);
-#pragma unroll
-        for (int u = 0; u < kWin; ++u) {
-            const int64_t kk = k0 + u;
-            jn[u] = -1;
-            if (kk < len) jn[u] = VERLET ? PV.nbr[kk * n + i] : (int32_t)(kk < i ? kk : kk + 1);
-        }
-    };
-    if (vmax > 0) load_window(0);
-
-    for (int64_t k = 0; k < vmax; k += kWin) {
-        int32_t jg[kWin];
-        float4 ph[kWin], pl[kWin];
-#pragma unroll
-        for (int u = 0; u < kWin; ++u) jg[u] = jn[u];
-#pragma unroll
-        for (int u = 0; u < kWin; ++u) {
-            ph[u] = hi_i;
-            pl[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (jg[u] >= 0) {
-                ph[u] = MX.x32[2 * jg[u]];
-                pl[u] = MX.x32[2 * jg[u] + 1];
-            }
-        }
-        if (k + kWin < vmax) load_window(k + kWin);  // next window, in flight during this one
-        int hcount = 0;
-        uint32_t hbal[kWin];
-        int hbas[kWin];
-#pragma unroll
-        for (int u = 0; u < kWin; ++u) {
-            bool hb = false;
-            if (jg[u] >= 0) {
-                if (hm == LG_HAMAKER_LIMITED) {
-                    const float dx = hi_i.x - ph[u].x, dy = hi_i.y - ph[u].y, dz = hi_i.z - ph[u].z;
-                    hb = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= MX.near2;
-                } else {
-                    hb = true;
-                }
-            }
-            const uint32_t bh = __ballot_sync(0xffffffffu, hb);
-            if (hb) {
-                const int q = hcount + __popc(bh & lt);
-                W.hhi[q] = make_float4(ph[u].x, ph[u].y, ph[u].z, __int_as_float(lane));
-                W.hlo[q] = pl[u];
-            }
-            hbal[u] = bh;
-            hbas[u] = hcount;
-            hcount += __popc(bh);
-        }
-        __syncwarp();
-        for (int q = lane; q < hcount; q += 32) hamaker_item(P, MX, W, q);
-        __syncwarp();
-        {  // the window's (at most four) terms in slot order, then one compensated add
-            float wsum[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-            for (int u = 0; u < kWin; ++u)
-                if ((hbal[u] >> lane) & 1u) {
-                    const int q = hbas[u] + __popc(hbal[u] & lt);
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) wsum[c] += W.hres[q][c];
-                }
-#pragma unroll
-            for (int c = 0; c < 3; ++c) ff_acc(acch[c], wsum[c]);
-        }
-        __syncwarp();  // the next window reuses the queue
+    if (i >= n) return;
+    const int32_t len = VERLET ? PV.row_len[i] : (int32_t)(n - 1);
+    const float4 xh = MX.x32[2 * i], xl = MX.x32[2 * i + 1];
+    for (int32_t k0 = sl * kWin; k0 < len; k0 += kSlices * kWin) {
+        int32_t j[kWin];
+        window_partners<VERLET>(PV, n, i, len, k0, j);
+        const f3 w = window_sum(P.hamaker_model, MX, xh, xl, j);
+        ff_acc(acch[0], w.x);
+        ff_acc(acch[1], w.y);
+        ff_acc(acch[2], w.z);
     }
-
 }
 
 // The completion of a step of a run for a particle that no step handler holds (the body of

@@ -44,10 +44,9 @@ constexpr int kStepWarps = 4;  // warps per block; each takes its own items
 // lg_set_step_shape) picks one. In the two-launch form the budget applies to the contact launch; the
 // Hamaker launch always takes 6, which its code alone fits without spills.
 
-// per-warp shared memory: the contact queue or the Hamaker window queue
-union StepSmem {
+// per-warp shared memory: the contact queue
+struct StepSmem {
     ContactSmem c;
-    HamakerSmem h;
 };
 
 // Completion of row i of a group: contact sums (csum), then the Hamaker partials of the group's
@@ -123,7 +122,7 @@ __global__ void __launch_bounds__(kStepWarps * 32, MINB)
             if constexpr (ROLE != 1) {
                 const int sl = k - nc;
                 ff acch[3];
-                hamaker_rows<VERLET>(P, PV, MX, W.h, row0, sl, A.slices, lane, acch);
+                hamaker_rows<VERLET>(P, PV, MX, row0, sl, A.slices, lane, acch);
                 const int64_t i = row0 + lane;
                 if (i < n) {
                     float4 *hp = A.hpart + 2 * ((int64_t)sl * n + i);
