@@ -297,8 +297,9 @@ __device__ __forceinline__ d3 shear_coulomb(d3 &xi, d3 n, double stiffness, doub
 }
 
 // FP64 overlap of a contact pair exactly as the FP64 path computes it (contact_force.h:65-66:
-// n = dx / |dx|, overlap = 2r - dx.n with dx = x_i - x_j), every operation rounded on its own.
-__device__ __forceinline__ double overlap_fp64(const dbl4 *x, int64_t i, int64_t j, double r) {
+// n = dx / |dx|, overlap = 2r - dx.n with dx = x_i - x_j), every operation rounded on its own. Out of line:
+// the mixed kernels need it for few pairs, and FP64 instructions under a false predicate are still issued.
+static __device__ __noinline__ double overlap_fp64(const dbl4 *x, int64_t i, int64_t j, double r) {
     const dbl4 a = x[i], b = x[j];
     const double dx = __dsub_rn(a.x, b.x), dy = __dsub_rn(a.y, b.y), dz = __dsub_rn(a.z, b.z);
     const double z = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));

@@ -470,7 +470,7 @@ static int rebuild_list(lg_system *s) {
     PairView &newv = s->pv[1 - s->pcur];
     PairView o = oldv;
     if (!s->list_built) o.row_len = nullptr;
-    BatchView B{s->d_agg, s->d_hoff, s->P.hold};
+    BatchView B{s->n_systems > 0 ? s->d_agg : nullptr, s->d_sys_off, s->n_systems, s->P.hold};
     launch_list_build(s->P.n, s->x, B, s->P.r_verlet, s->r_near, s->max_cells, s->ls, o, newv, s->bv, s->err,
                       s->stream);
     s->launches += 5;
@@ -1005,43 +1005,16 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
         P.hold = s->d_hold;
     }
 
-    // batch segmentation: system index per particle, hashing offsets that keep systems apart
+    // batch segmentation: system index per particle
     if (s->n_systems > 0) {
         const int64_t ns = s->n_systems;
         std::vector<int32_t> agg((size_t)n);
-        std::vector<double> cen(3 * (size_t)ns), rad((size_t)ns, 0.0);
-        double rmax = 0.0;
-        for (int64_t q = 0; q < ns; ++q) {
-            const int64_t b = s->sys_off[q], e = s->sys_off[q + 1];
-            for (int k = 0; k < 3; ++k) {
-                double sum = 0.0;
-                for (int64_t i = b; i < e; ++i) sum += x0[3 * i + k];
-                cen[3 * q + k] = sum / (double)(e - b);
-            }
-            for (int64_t i = b; i < e; ++i) {
-                agg[i] = (int32_t)q;
-                double r2 = 0.0;
-                for (int k = 0; k < 3; ++k) r2 += (x0[3 * i + k] - cen[3 * q + k]) * (x0[3 * i + k] - cen[3 * q + k]);
-                rad[q] = std::max(rad[q], std::sqrt(r2));
-            }
-            rmax = std::max(rmax, rad[q]);
-        }
-        // lattice spacing: two system radii, room for growth, and two list radii
-        const double L = arena ? arena->lattice : 4.0 * rmax + 2.0 * d->r_verlet + 8.0 * d->contact.r_part + 1e-12;
-        int64_t m = 1;
-        while (m * m * m < ns) ++m;
-        std::vector<dbl4> hoff((size_t)ns);
-        for (int64_t q = 0; q < ns; ++q) {
-            const double gx = (double)(q % m) * L, gy = (double)((q / m) % m) * L, gz = (double)(q / (m * m)) * L;
-            hoff[q] = make_double4_32a(gx - cen[3 * q], gy - cen[3 * q + 1], gz - cen[3 * q + 2], 0.0);
-        }
+        for (int64_t q = 0; q < ns; ++q) std::fill(agg.begin() + s->sys_off[q], agg.begin() + s->sys_off[q + 1], (int32_t)q);
         LG_TRY(s->alloc(&s->d_agg, (size_t)n));
-        LG_TRY(s->alloc(&s->d_hoff, (size_t)ns));
         LG_TRY(s->alloc(&s->d_sys_off, (size_t)ns + 1));
         LG_TRY(s->alloc(&s->d_centres, 3 * (size_t)ns));
         LG_TRY(s->alloc(&s->d_sys_obs, 20 * (size_t)ns));
         LG_CUDA(cudaMemcpy(s->d_agg, agg.data(), sizeof(int32_t) * agg.size(), cudaMemcpyHostToDevice));
-        LG_CUDA(cudaMemcpy(s->d_hoff, hoff.data(), sizeof(dbl4) * hoff.size(), cudaMemcpyHostToDevice));
         LG_CUDA(cudaMemcpy(s->d_sys_off, s->sys_off.data(), sizeof(int64_t) * s->sys_off.size(), cudaMemcpyHostToDevice));
     }
 
@@ -1117,22 +1090,19 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
         };
         LG_TRY(alloc_rows(cap));
         s->pcur = 0;
-        s->max_cells = std::max<int64_t>(64, (s->n_systems > 0 ? 8 : 4) * n);
-        if (arena) {  // the slot lattice at cells of about r_verlet (capped at 2^25 cells)
-            int64_t m = 1;
-            while (m * m * m < s->n_systems) ++m;
-            const double per = (double)m * arena->lattice / d->r_verlet + 2.0;
-            s->max_cells = std::max<int64_t>(s->max_cells, (int64_t)std::min(per * per * per, 33554432.0));
-        }
+        // cells: four per particle; a batch: eight per particle and 64 more per system
+        s->max_cells = s->n_systems > 0 ? 8 * n + 64 * s->n_systems : std::max<int64_t>(64, 4 * n);
         s->ls.nparts = 608;
         LG_TRY(s->alloc(&s->ls.part, 6 * 608));
-        LG_TRY(s->alloc(&s->ls.grid, 1));
+        LG_TRY(s->alloc(&s->ls.grid, (size_t)std::max<int64_t>(s->n_systems, 1)));
         LG_TRY(s->alloc(&s->ls.cell_of, (size_t)n));
         LG_TRY(s->alloc(&s->ls.count, (size_t)s->max_cells));
         LG_TRY(s->alloc(&s->ls.start, (size_t)s->max_cells));
         LG_TRY(s->alloc(&s->ls.sorted, (size_t)n));
         LG_TRY(s->alloc(&s->ls.ticket, 1));
         LG_TRY(s->alloc(&s->ls.cursor, 1));
+        LG_TRY(s->alloc(&s->ls.cell_cursor, 1));
+        LG_CUDA(cudaMemset(s->ls.cell_cursor, 0, sizeof(int32_t)));
         LG_CUDA(cudaMemset(s->ls.ticket, 0, sizeof(unsigned)));
         LG_TRY(s->alloc(&s->ls.x32, (size_t)n));
         LG_TRY(s->alloc(&s->ls.max_row, 1));
@@ -2140,15 +2110,12 @@ int lg_arena_import(lg_system *A, int64_t q, lg_system *S, const double *x0) {
         LG_CUDA(cp(PA.near_len + off, PS.near_len, sizeof(int32_t) * n));
         LG_CUDA(cudaMemsetAsync(PA.near_len + off + n, 0, sizeof(int32_t) * tail, st));
     }
-    // float-float origin (the standalone handle's) and hashing offset to the slot's lattice point
+    // float-float origin (the standalone handle's)
     dbl4 orig = make_double4_32a(S->origin[0], S->origin[1], S->origin[2], S->origin[3]);
-    const dbl4 hoff = make_double4_32a(A->slot_pos[3 * q] - c[0], A->slot_pos[3 * q + 1] - c[1],
-                                       A->slot_pos[3 * q + 2] - c[2], 0.0);
     if (A->precision == LG_PRECISION_MIXED) {
         A->h_orig[(size_t)q] = orig;
         LG_CUDA(cudaMemcpyAsync(A->d_orig + q, &orig, d4, cudaMemcpyHostToDevice, st));
     }
-    LG_CUDA(cudaMemcpyAsync(A->d_hoff + q, &hoff, d4, cudaMemcpyHostToDevice, st));
     A->n_bonds_initial_sys[(size_t)q] = S->n_bonds_initial;
     LG_CUDA(cudaGetLastError());
     LG_CUDA(cudaStreamSynchronize(st));  // host buffers above are released on return
@@ -2173,8 +2140,6 @@ int lg_arena_clear(lg_system *A, int64_t q) {
         LG_CUDA(cudaMemsetAsync(pv.row_len + off, 0, sizeof(int32_t) * C, st));
         if (pv.near_len) LG_CUDA(cudaMemsetAsync(pv.near_len + off, 0, sizeof(int32_t) * C, st));
     }
-    const dbl4 zero = make_double4_32a(0.0, 0.0, 0.0, 0.0);
-    LG_CUDA(cudaMemcpyAsync(A->d_hoff + q, &zero, d4, cudaMemcpyHostToDevice, st));
     A->n_bonds_initial_sys[(size_t)q] = 0;
     LG_CUDA(cudaGetLastError());
     LG_CUDA(cudaStreamSynchronize(st));

@@ -99,7 +99,6 @@ struct lg_system {
     std::vector<int64_t> sys_off;        // host prefix offsets [n_systems + 1]
     int64_t *d_sys_off = nullptr;        // device copy
     int32_t *d_agg = nullptr;            // [n] system of every particle
-    lg::dbl4 *d_hoff = nullptr;          // [n_systems] hashing offsets
     lg::dbl4 *d_orig = nullptr;          // [n_systems] float-float origins (x, y, z; w: extent), mixed
     std::vector<lg::dbl4> h_orig;        // host copy of d_orig
     double *d_centres = nullptr;         // [3 n_systems] scratch for per-system observables
@@ -166,7 +165,7 @@ int lg_fail(int code, const char *fmt, ...);
 // occupants advance in the same launches. lg_arena_import moves a standalone handle built from the
 // same template (the request after its construction force evaluation, at a rebuild boundary) into
 // slot q: state, bonds with their springs, pair rows with their springs (partner indices moved by
-// the slot's offset), float-float origin and hashing offset; the occupant then evolves exactly as
+// the slot's offset) and float-float origin; the occupant then evolves exactly as
 // the standalone handle would. lg_arena_clear empties a slot; lg_arena_read copies an occupant's
 // state (host arrays of 3n doubles, null: skipped). The caller keeps the arena at a rebuild
 // boundary and idle (synchronised) around imports and clears.

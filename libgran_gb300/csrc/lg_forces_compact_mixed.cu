@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(512) near_owners(int64_t n, PairView PV, NearS
 // completion adds per row in entry order; the springs of both slots are written.
 // What bounds it: instruction issue and the latency of its gathers.
 template <int THREADS>
-__global__ void __launch_bounds__(THREADS, 640 / THREADS)
+__global__ void __launch_bounds__(THREADS, 512 / THREADS)
     mixed_contacts(Params P, PairView PV, BondView BV, MixedExtra MX, NearScratch R) {
     struct Item {
         int32_t i, j;

@@ -7,33 +7,36 @@
 
 namespace lg {
 
+// Cell grid of one system (a batch: one per system, their cells one after another from `base` on).
 struct GridDev {
     double lo[3];
-    float inv_edge;  // 1 / cell edge
-    int64_t dim[3];
-    int64_t ncell;
+    float edge, inv_edge;  // cell width in y and z, and its inverse (in x: a quarter)
+    float slack;           // uncertainty of the cell boundaries, in cells
+    int32_t dim[3], base;
     float rv2_lo, rv2_hi;  // FP32 accept / reject bounds of the squared list radius
     float rn2_hi;          // FP32 bound of the squared near radius (contact candidates), < 0: none
 };
 
-// Batch segmentation (null pointers for a single system): system index of every particle and the
-// spatial offset of every system used only for cell hashing.
+// Batch segmentation (null pointers for a single system): system index of every particle, and the
+// systems' prefix offsets.
 struct BatchView {
     const int32_t *agg;    // [n]
-    const dbl4 *hoff;      // [n_systems]
+    const int64_t *off;    // [n_systems + 1]
+    int64_t n_systems;
     const uint8_t *hold;   // [n] hold bits (null: none); inactive particles are left out of the list
 };
 
 struct ListScratch {
     int nparts;        // blocks of the bounding-box pass
     double *part;      // [nparts * 6]
-    GridDev *grid;     // device grid description
+    GridDev *grid;     // [1, or n_systems] device grid descriptions
     int32_t *cell_of;  // [n]
     int32_t *count;    // [max_cells]
     int32_t *start;    // [max_cells] begin of every cell in the sorted list, then its end
-    int32_t *sorted;   // [n]
+    float4 *sorted;    // [n] cell by cell: position relative to the grid origin, and the index (bits of w)
     unsigned *ticket;  // finished blocks of the bounding-box pass (zero between builds)
     int32_t *cursor;   // places of the sorted list taken so far
+    int32_t *cell_cursor;  // batch: cells taken so far (zero between builds)
     float4 *x32;       // [n] positions relative to the grid origin, FP32 (candidate filter)
     int32_t *max_row;  // [1] longest row found by the last build (before truncation)
 };

@@ -115,32 +115,29 @@ __device__ __forceinline__ f3 shear_ff(ff (&xi)[3], f3 n, float stiffness, float
     }
     const f3 xn = fadd(xf, drot);
     const f3 f0 = fsub(fscl(-stiffness, xn), fscl(damping, rel));
-    if (!coulomb) {
+    f3 f = f0;
+    bool slide = false;
+    if (coulomb) {
+        const float fs = mu_s * normal_force;
+        const float fd = mu_s * phi * normal_force;
+        const float f0n = sqrtf(fdot(f0, f0));
+        const f3 t = f0n > 0.0f ? fscl(1.0f / f0n, f0) : fm(0.f, 0.f, 0.f);
+        slide = !(f0n <= fs);
+        if (slide) {
+            const f3 nx = fscl(-1.0f / stiffness, fadd(fscl(fd, t), fscl(damping, rel)));
+            xi[0] = ff{nx.x, 0.f};
+            xi[1] = ff{nx.y, 0.f};
+            xi[2] = ff{nx.z, 0.f};
+        }
+        f = fscl(fminf(slide ? fd : fs, f0n), t);
+    }
+    if (!slide) {
         const f3 dxi = fadd(drot, fscl(dtf, rel));
         ff_add_norm(xi[0], dxi.x);
         ff_add_norm(xi[1], dxi.y);
         ff_add_norm(xi[2], dxi.z);
-        return f0;
     }
-    const float fs = mu_s * normal_force;
-    const float fd = mu_s * phi * normal_force;
-    const float f0n = sqrtf(fdot(f0, f0));
-    const f3 t = f0n > 0.0f ? fscl(1.0f / f0n, f0) : fm(0.f, 0.f, 0.f);
-    float sel;
-    if (f0n <= fs) {
-        const f3 dxi = fadd(drot, fscl(dtf, rel));
-        ff_add_norm(xi[0], dxi.x);
-        ff_add_norm(xi[1], dxi.y);
-        ff_add_norm(xi[2], dxi.z);
-        sel = fs;
-    } else {
-        const f3 nx = fscl(-1.0f / stiffness, fadd(fscl(fd, t), fscl(damping, rel)));
-        xi[0] = ff{nx.x, 0.f};
-        xi[1] = ff{nx.y, 0.f};
-        xi[2] = ff{nx.z, 0.f};
-        sel = fd;
-    }
-    return fscl(fminf(sel, f0n), t);
+    return f;
 }
 
 // Separation d = x_i - x_j (FP32) and q = |d|^2 - (2r)^2 from float-float positions. Per component
@@ -169,6 +166,13 @@ __device__ __forceinline__ SepFF separation_ff(float4 hi, float4 lo, float4 hj, 
     return SepFF{fm(tx.hi + lx, ty.hi + ly, tz.hi + lz), s3 + rest};
 }
 
+// c ? a : b as one select instruction (see contact_pair).
+__device__ __forceinline__ float pick(int c, float a, float b) {
+    float r;
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %3, 0;\n\tselp.f32 %0, %1, %2, p;\n\t}" : "=f"(r) : "f"(a), "f"(b), "r"(c));
+    return r;
+}
+
 // One contact or bond pair (contact_force.h:57-147, alt_sinter_bridge.h:103-156) from the two particles'
 // float-float positions and velocities and FP32 spins: the force on i, and the three parts of its torque
 // (rr n x f_r, rp n x f_t, rr f_o). The springs s (xi_t, xi_r, xi_o) are updated. Returns false, with
@@ -194,11 +198,13 @@ __device__ __forceinline__ f3 torque_of(const f3 &roll, const f3 &slide, const f
 }
 __device__ __forceinline__ bool contact_pair(const Params &P, const MixedExtra &M, bool bonded, int64_t i, int64_t j,
                                              const Body &bi, const Body &bj, ff (&s)[3][3], ContactOut &o) {
-    const SepFF sp = separation_ff(bi.xh, bi.xl, bj.xh, bj.xl, bonded ? M.b_fr_hi : M.c_fr_hi,
-                                   bonded ? M.b_fr_lo : M.c_fr_lo);
+    int kind = bonded ? 1 : 0;
+    asm volatile("" : "+r"(kind));  // (its value is hidden from the compiler, see pick)
+    const SepFF sp = separation_ff(bi.xh, bi.xl, bj.xh, bj.xl, pick(kind, M.b_fr_hi, M.c_fr_hi),
+                                   pick(kind, M.b_fr_lo, M.c_fr_lo));
     const f3 dxf = sp.d;
     const float d2f = fdot(dxf, dxf);
-    const float rr = bonded ? M.b_r : M.c_r;
+    const float rr = pick(kind, M.b_r, M.c_r);
     const float rsd = rsqrtf(d2f);
     // 2r - |d|, from |d|^2 - (2r)^2 (the product rounds on its own in every kernel: the same bits)
     const float overlap = -sp.q / __fadd_rn(__fmul_rn(d2f, rsd), 2.0f * rr);
@@ -213,7 +219,7 @@ __device__ __forceinline__ bool contact_pair(const Params &P, const MixedExtra &
     const f3 vij0 = fm(tx.hi + (tx.lo + (bi.vl.x - bj.vl.x)), ty.hi + (ty.lo + (bi.vl.y - bj.vl.y)),
                        tz.hi + (tz.lo + (bi.vl.z - bj.vl.z)));
     const f3 wfi = fm(bi.w.x, bi.w.y, bi.w.z), wfj = fm(bj.w.x, bj.w.y, bj.w.z);
-    const float kn = bonded ? M.b_k : M.c_k, gn = bonded ? M.b_gn : M.c_gn;
+    const float kn = pick(kind, M.b_k, M.c_k), gn = pick(kind, M.b_gn, M.c_gn);
     const float rp = rr - 0.5f * overlap;
     const float v_n = -fdot(vij0, n3);
     const float f_n = kn * overlap + gn * v_n;
@@ -222,16 +228,12 @@ __device__ __forceinline__ bool contact_pair(const Params &P, const MixedExtra &
     const f3 v_t = fsub(v_ij, fscl(fdot(v_ij, n3), n3));
     const f3 v_r = fscl(-rp, fsub(nwi, nwj));
     const f3 v_o = fscl(rr * (fdot(n3, wfi) - fdot(n3, wfj)), n3);
-    f3 f_t, f_r, f_o;
-    if (bonded) {
-        f_t = shear_ff(s[0], n3, M.b_kt, M.b_gt, f_n, 0.f, 0.f, v_t, M.b_dt, false);
-        f_r = shear_ff(s[1], n3, M.b_kr, M.b_gr, f_n, 0.f, 0.f, v_r, M.b_dt, false);
-        f_o = shear_ff(s[2], n3, M.b_ko, M.b_go, f_n, 0.f, 0.f, v_o, M.b_dt, false);
-    } else {
-        f_t = shear_ff(s[0], n3, M.c_kt, M.c_gt, f_n, M.c_mus, M.c_phid, v_t, M.c_dt, true);
-        f_r = shear_ff(s[1], n3, M.c_kr, M.c_gr, f_n, M.c_mur, M.c_phir, v_r, M.c_dt, true);
-        f_o = shear_ff(s[2], n3, M.c_ko, M.c_go, f_n, M.c_muo, M.c_phio, v_o, M.c_dt, true);
-    }
+    // (the constants are picked by select instructions: with branches the compiler makes one copy of the
+    // shear code for bonds and one for contacts, and a warp with both kinds issues both)
+    const float dt = pick(kind, M.b_dt, M.c_dt);
+    const f3 f_t = shear_ff(s[0], n3, pick(kind, M.b_kt, M.c_kt), pick(kind, M.b_gt, M.c_gt), f_n, M.c_mus, M.c_phid, v_t, dt, !bonded);
+    const f3 f_r = shear_ff(s[1], n3, pick(kind, M.b_kr, M.c_kr), pick(kind, M.b_gr, M.c_gr), f_n, M.c_mur, M.c_phir, v_r, dt, !bonded);
+    const f3 f_o = shear_ff(s[2], n3, pick(kind, M.b_ko, M.c_ko), pick(kind, M.b_go, M.c_go), f_n, M.c_muo, M.c_phio, v_o, dt, !bonded);
     o.force = fadd(fscl(f_n, n3), f_t);
     o.roll = fcrs(n3, f_r);
     o.slide = fcrs(n3, f_t);
