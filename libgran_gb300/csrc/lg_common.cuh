@@ -376,8 +376,21 @@ __device__ __forceinline__ d3 hamaker_accel_n(int mode, const lg_hamaker_params 
     return ok ? a : dvs(su, p.mass);
 }
 
-// triangular_facet.h:73-137
-__device__ __forceinline__ d3 closest_point_on_triangle(const double *vt, double area, d3 N, d3 p) {
+// A facet's edges: unit vectors and lengths (the same for every particle of an evaluation).
+struct FacetEdges {
+    d3 u[3];
+    double len[3];
+};
+__device__ __forceinline__ void facet_edge(const double *vt, int k, FacetEdges &E) {
+    const int q = (k + 1) % 3;
+    const d3 L = sub(mk3(vt[3 * q], vt[3 * q + 1], vt[3 * q + 2]), mk3(vt[3 * k], vt[3 * k + 1], vt[3 * k + 2]));
+    E.u[k] = nrmz(L);
+    E.len[k] = nrm(L);
+}
+
+// triangular_facet.h:73-137; E: the facet's edges, or null to compute them
+__device__ __forceinline__ d3 closest_point_on_triangle(const double *vt, double area, d3 N, d3 p,
+                                                        const FacetEdges *E = nullptr) {
     d3 v0 = mk3(vt[0], vt[1], vt[2]), v1 = mk3(vt[3], vt[4], vt[5]), v2 = mk3(vt[6], vt[7], vt[8]);
     d3 off = scl(dot(v0, N), N);
     d3 proj = sub(p, scl(dot(p, N), N));
@@ -393,10 +406,17 @@ __device__ __forceinline__ d3 closest_point_on_triangle(const double *vt, double
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         d3 a = vv[k], b = vv[(k + 1) % 3];
-        d3 L = sub(b, a);
-        d3 uL = nrmz(L);
+        d3 uL;
+        double len;
+        if (E) {
+            uL = E->u[k];
+            len = E->len[k];
+        } else {
+            d3 L = sub(b, a);
+            uL = nrmz(L);
+            len = nrm(L);
+        }
         d3 tp = sub(p, a);
-        double len = nrm(L);
         double pr = dot(tp, uL);
         if (pr < 0.0)
             e[k] = a;

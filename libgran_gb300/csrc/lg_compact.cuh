@@ -22,10 +22,10 @@ __device__ __forceinline__ void move_facets(const Params &P, const StateView &S,
 // folded as the reference's unary container folds its functors, f0 + (f1 + (... + body))
 // (unary_force_container.h:27-29): the last term first, each earlier one added in front. Returns
 // false when there is no unary term. Kept out of line: the common no-facet path then needs few
-// registers; static: each translation unit keeps its own copy, compiled with its own
+// registers; edges: the facets' edges, or null; static: each translation unit keeps its own copy, compiled with its own
 // floating-point flags.
 static __device__ __noinline__ bool unary_terms(const Params &P, const StateView &S, int64_t i, int64_t n, d3 vi,
-                                                d3 wi, d3 &ua, d3 &ual) {
+                                                d3 wi, d3 &ua, d3 &ual, const FacetEdges *edges = nullptr) {
     const d3 xi = ld4(S.x, i);
     bool have = false;
     if (P.ext_a) {
@@ -36,7 +36,7 @@ static __device__ __noinline__ bool unary_terms(const Params &P, const StateView
     for (int f = P.n_facets - 1; f >= 0; --f) {
         const FacetDev &fd = P.facets[f];
         d3 N = mk3(fd.normal[0], fd.normal[1], fd.normal[2]);
-        d3 xf = closest_point_on_triangle(S.facet_vert + 9 * f, fd.area, N, xi);
+        d3 xf = closest_point_on_triangle(S.facet_vert + 9 * f, fd.area, N, xi, edges ? edges + f : nullptr);
         d3 vf = mk3(fd.v[0], fd.v[1], fd.v[2]);
         d3 fa = zero3(), fal = zero3();
         bool hv = false;

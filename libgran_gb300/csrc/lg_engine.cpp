@@ -355,8 +355,10 @@ void lg_system::release() {
     if (ev1) cudaEventDestroy(ev1);
     if (fork_ev) cudaEventDestroy(fork_ev);
     if (join_ev) cudaEventDestroy(join_ev);
-    side = nullptr;
-    fork_ev = join_ev = nullptr;
+    if (unary_st) cudaStreamDestroy(unary_st);
+    if (unary_ev) cudaEventDestroy(unary_ev);
+    side = unary_st = nullptr;
+    fork_ev = join_ev = unary_ev = nullptr;
     for (cudaEvent_t e : tev) cudaEventDestroy(e);
     tev.clear();
     stream = nullptr;
@@ -436,11 +438,14 @@ static PairScratch pair_scratch(const lg_system *s) {
 // Scratch of the mixed contact kernel that evaluates each pair once, in the idle list's spring buffer (9
 // doubles a slot: two float4 of records, an owner entry). Neck strengths looked up by the reference's
 // indexing differ between a pair's two orders, so a breaking bond may then break in one order only: such
-// systems take the kernel that evaluates each order.
+// systems take the kernel that evaluates each order. From 512 monomers on beside a Hamaker kernel, whose run
+// time covers the owners' pass and the completion's sums (us a step, once per pair against once per order: 500
+// monomers 14.5 / 15.3, 4000 15.8 / 17.1, 8000 17.0 / 19.0); alone from 49152 (8000: 16.0 / 13.8, 40000: 22.4 /
+// 21.8, 65000: 27.1 / 29.1).
 static NearScratch near_scratch(const lg_system *s) {
     NearScratch R{};
     if (!s->own_n || s->precision != LG_PRECISION_MIXED || !s->pv[0].near_len) return R;
-    if (s->P.n < (getenv("LG_NM") ? atoi(getenv("LG_NM")) : 8192)) return R;
+    if (s->P.n < (s->P.hamaker_model != LG_HAMAKER_NONE ? 512 : 49152)) return R;
     if (s->P.binary_model == LG_BINARY_BREAKING_SINTER && s->P.neck_mode == LG_NECK_REFERENCE_INDEXING) return R;
     double *base = s->pv[1 - s->pcur].xi;
     const int64_t slots = s->pv[0].cap * s->P.n;
@@ -602,7 +607,8 @@ static int launch_forces(lg_system *s, double hdt, double dt, int move_facets, b
     } else if (s->precision == LG_PRECISION_MIXED) {
         if (compact || persistent)
             kernels = launch_forces_compact_mixed(s->P, S, s->pv[s->pcur], s->bv, hdt, dt, move_facets, fuse_kick,
-                                                  prev_fused, s->mx, s->stream, s->side, s->fork_ev, s->join_ev,
+                                                  prev_fused, s->mx, s->stream,
+                                                  {s->side, s->unary_st, s->fork_ev, s->join_ev, s->unary_ev},
                                                   s->ham_slices, s->contact_lanes, near_scratch(s));
         else
             launch_forces_mixed(s->T, s->P, S, s->pv[s->pcur], s->bv, hdt, dt, move_facets, s->mx, s->stream);
@@ -725,6 +731,18 @@ static int apply_hold(lg_system *s, const uint8_t *mask) {
     return LG_OK;
 }
 
+// Buffers, stream and event of the mixed path's unary terms (systems with facets or a body term).
+static int ensure_unary(lg_system *s) {
+    if (s->precision != LG_PRECISION_MIXED || s->unary_ev) return LG_OK;
+    LG_TRY(s->alloc(&s->un_a, (size_t)s->P.n));
+    LG_TRY(s->alloc(&s->un_al, (size_t)s->P.n));
+    s->mx.un_a = s->un_a;
+    s->mx.un_al = s->un_al;
+    if (!s->unary_st) LG_CUDA(cudaStreamCreateWithFlags(&s->unary_st, cudaStreamNonBlocking));
+    LG_CUDA(cudaEventCreateWithFlags(&s->unary_ev, cudaEventDisableTiming));
+    return LG_OK;
+}
+
 // Body force or unary hook (at most one); both write the per-particle unary terms that the force
 // kernels fold after the facets.
 static int apply_unary(lg_system *s, const lg_body_force *body, lg_unary_hook hook, void *user) {
@@ -732,6 +750,7 @@ static int apply_unary(lg_system *s, const lg_body_force *body, lg_unary_hook ho
     const int model = body ? body->model : LG_BODY_NONE;
     s->drop_graphs();
     const bool on = model != LG_BODY_NONE || hook;
+    if (on || s->P.n_facets > 0) LG_TRY(ensure_unary(s));
     if (on && !s->ext_a) {
         LG_TRY(s->alloc(&s->ext_a, (size_t)s->P.n));
         LG_TRY(s->alloc(&s->ext_al, (size_t)s->P.n));

@@ -15,6 +15,10 @@ struct lg_system {
     // (fork / join events on the handle's stream; captured into the step graphs as two branches)
     cudaStream_t side = nullptr;
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
+    // and a third for the unary terms (created with them)
+    cudaStream_t unary_st = nullptr;
+    cudaEvent_t unary_ev = nullptr;
+    lg::dbl4 *un_a = nullptr, *un_al = nullptr;  // mixed: [n] unary terms of an evaluation
     lg_system_desc desc{};
     lg::Params P{};
     int precision = LG_PRECISION_FP64;

@@ -24,6 +24,7 @@
 // The per-pair and per-row pieces (and the precision scheme) are in lg_mixed_pairs.cuh, shared with
 // the persistent step kernel (lg_step_mixed.cu). Per-row sums are in an order fixed by the row
 // alone, so a system gives the same bits alone and inside a batch (with the same slicing).
+#include <algorithm>
 #include <cstddef>
 
 #include "lg_mixed_pairs.cuh"
@@ -363,6 +364,28 @@ __global__ void __launch_bounds__(kHThreads, L == 1 ? 6 : 7) forces_hamaker_mixe
     MX.hsum[2 * i + 1] = make_float4(acc[2].hi, acc[2].lo, 0.f, 0.f);
 }
 
+// Unary terms (facets, body force) of every particle, beside the pair kernels: they need the FP64 state only,
+// and the FP64 pipe, which the pair kernels leave idle (in the completion they took 105 of its 119 us for
+// 141,000 particles on a wall). The grid holds no more than sixteen warps per SM, at 64 registers: the FP64
+// pipe is nearly as busy as with more, and the rest of the register file is the pair kernels' (restructuring
+// batch of 141,000 particles, us a step: 175 with one block per 64 particles at 150 registers, 170 with six
+// such blocks per SM, 146 at 80 registers). The facets' edges are formed once per block.
+constexpr int kUnaryThreads = 64;
+constexpr int kUnaryBlocks = 152 * 8;
+__global__ void __launch_bounds__(kUnaryThreads, 16) unary_mixed(Params P, StateView S, MixedExtra MX) {
+    __shared__ FacetEdges edges[kMaxFacets];
+    if ((int)threadIdx.x < 3 * P.n_facets)
+        facet_edge(S.facet_vert + 9 * (threadIdx.x / 3), threadIdx.x % 3, edges[threadIdx.x / 3]);
+    __syncthreads();
+    for (int64_t i = blockIdx.x * (int64_t)kUnaryThreads + threadIdx.x; i < P.n; i += (int64_t)gridDim.x * kUnaryThreads) {
+        if (inactive_of(P.hold, i)) continue;
+        d3 ua = zero3(), ual = zero3();
+        compact::unary_terms(P, S, i, P.n, ld4(S.v, i), ld4(S.w, i), ua, ual, edges);
+        st4(MX.un_a, i, ua);
+        st4(MX.un_al, i, ual);
+    }
+}
+
 // Completion of row i in FP64: contact part (csum when `contacts`) plus the Hamaker part (hsum when
 // `hamaker`), both converted to FP64, then the unary terms, stores and half kick; with `kick` also
 // the next step's opening half kick and drift, and the float-float copies of the new state.
@@ -388,7 +411,11 @@ __device__ __forceinline__ void finish_fp64_row(const Params &P, const StateView
         const d3 ah = mk3((double)h0.x + (double)h0.y, (double)h0.z + (double)h0.w, (double)h1.x + (double)h1.y);
         a_tot = contacts ? add(a_tot, ah) : ah;
     }
-    compact::finish_row<FACETS>(P, S, i, P.n, a_tot, al_tot, vi, wi, hdt);
+    if (FACETS) {  // (unary_mixed's terms)
+        a_tot = add(a_tot, ld4(MX.un_a, i));
+        al_tot = add(al_tot, ld4(MX.un_al, i));
+    }
+    compact::finish_row<false>(P, S, i, P.n, a_tot, al_tot, vi, wi, hdt);
     if (kick) {  // the next step's opening half kick and drift (the end-of-step velocities are not kept)
         const uint32_t h = hold_of(P.hold, i);
         const bool hv = h & LG_HOLD_V, hw = h & LG_HOLD_OMEGA;
@@ -455,30 +482,53 @@ __global__ void __launch_bounds__(64) forces_finish_ff(Params P, StateView S, in
 
 namespace {
 
+// Launch with a share of the SM's memory set aside as shared memory (per cent; a hint).
+// An SM changes that share only while it is idle, and by default it follows the kernel's own use: kernels that
+// use none (Hamaker pairs) and some (contacts) then cannot be on one SM together, and one stream's kernel waits
+// for the other's to end: single steps of 8000 listed particles took 40 us as soon as an SM held more than one
+// contact block, and take 29 with one share for all; all pairs of 700 took 39 and take 23. (A share just large
+// enough did not help everywhere: 42 with 64 KB for all pairs of 700.) The unary terms' kernel states no
+// preference: with the others' share the restructuring batch takes 170 us a step instead of 145.
+template <typename... P, typename... A>
+void launch_shared(int share, void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t st,
+                   const A &...args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at.val.sharedMemCarveout = (unsigned)share;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(blocks);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 // Lanes per row of the contact kernel: T = 2 (or 1, a tuning choice that suits large batches) for
 // candidate lists (a few entries per row); a whole warp per row for all pairs (n - 1 candidates per
 // row: the lanes share them, and the row count no longer bounds the warps a small system can use).
 template <bool NEAR, int T>
 void launch_contacts(const Params &P, const StateView &S, const PairView &PV, const BondView &BV, const MixedExtra &MX,
-                     cudaStream_t st, bool beside_hamaker) {
+                     cudaStream_t st, bool beside_hamaker, int share) {
     const size_t smem = sizeof(ContactSmem) * kCWarps;
     const int64_t rows_per_block = (32 / T) * kCWarps;
     const unsigned blocks = (unsigned)((P.n + rows_per_block - 1) / rows_per_block);
-    if (beside_hamaker)
-        forces_contacts_mixed<NEAR, T, LG_CONTACT_MIN_BLOCKS><<<blocks, kCWarps * 32, smem, st>>>(P, S, PV, BV, MX);
+    if (NEAR && beside_hamaker)
+        launch_shared(share, forces_contacts_mixed<NEAR, T, LG_CONTACT_MIN_BLOCKS>, blocks, kCWarps * 32, smem, st, P, S, PV, BV, MX);
     else
-        forces_contacts_mixed<NEAR, T, LG_CONTACT_MIN_BLOCKS_ALONE><<<blocks, kCWarps * 32, smem, st>>>(P, S, PV, BV, MX);
+        launch_shared(share, forces_contacts_mixed<NEAR, T, LG_CONTACT_MIN_BLOCKS_ALONE>, blocks, kCWarps * 32, smem, st, P, S, PV, BV, MX);
 }
 
 template <bool VERLET, int L, int SL>
-void launch_hamaker(const Params &P, const PairView &PV, const MixedExtra &MX, cudaStream_t st) {
+void launch_hamaker(const Params &P, const PairView &PV, const MixedExtra &MX, cudaStream_t st, int share) {
     const unsigned blocks = (unsigned)((P.n * L + kHThreads - 1) / kHThreads);
     if (P.hamaker_model == LG_HAMAKER_LIMITED)
-        forces_hamaker_mixed<VERLET, LG_HAMAKER_LIMITED, L, SL><<<blocks, kHThreads, 0, st>>>(P, PV, MX);
+        launch_shared(share, forces_hamaker_mixed<VERLET, LG_HAMAKER_LIMITED, L, SL>, blocks, kHThreads, 0, st, P, PV, MX);
     else if (P.hamaker_model == LG_HAMAKER_SIMPLIFIED)
-        forces_hamaker_mixed<VERLET, LG_HAMAKER_SIMPLIFIED, L, SL><<<blocks, kHThreads, 0, st>>>(P, PV, MX);
+        launch_shared(share, forces_hamaker_mixed<VERLET, LG_HAMAKER_SIMPLIFIED, L, SL>, blocks, kHThreads, 0, st, P, PV, MX);
     else
-        forces_hamaker_mixed<VERLET, LG_HAMAKER_FULL, L, SL><<<blocks, kHThreads, 0, st>>>(P, PV, MX);
+        launch_shared(share, forces_hamaker_mixed<VERLET, LG_HAMAKER_FULL, L, SL>, blocks, kHThreads, 0, st, P, PV, MX);
 }
 
 }  // namespace
@@ -517,78 +567,91 @@ void launch_near_owners(int64_t n, const PairView &PV, const NearScratch &R, cud
 
 int launch_forces_compact_mixed(const Params &P, const StateView &S, const PairView &PV, const BondView &BV, double hdt,
                                 double dt, int move_facets, bool kick, bool prev_fused, const MixedExtra &MX,
-                                cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int slices,
-                                int contact_lanes, NearScratch R) {
+                                cudaStream_t st, const SideStreams &J, int slices, int contact_lanes, NearScratch R) {
     const bool ver = P.pairs == LG_PAIRS_VERLET;
     const int contacts = P.binary_model != LG_BINARY_NONE ? 1 : 0;
     const int hamaker = P.hamaker_model != LG_HAMAKER_NONE ? 1 : 0;
     int kernels = 1;
-    if (contacts) {  // the contact branch runs beside the Hamaker kernel
-        cudaEventRecord(fork, st);
-        cudaStreamWaitEvent(side, fork, 0);
+    const bool unary = P.n_facets > 0 || P.ext_a;
+    const unsigned blocks = (unsigned)((P.n + 63) / 64);
+    // the contact kernel runs beside the Hamaker kernel, the unary terms beside both; a lone contact kernel
+    // needs no second stream
+    const bool fork_c = contacts && (hamaker || unary);
+    if (!(ver && PV.near_len)) R.rec = nullptr;
+    // 100 KB hold the owners' blocks that the registers allow (44 KB) and seven blocks of the other contact kernel;
+    // lists that would fill the SM with more of the latter get room for twelve
+    const bool twelve = ver && !R.rec && P.n > (int64_t)7 * 152 * kCWarps * (32 / kContactLanes);
+    const int share = twelve ? 72 : 44;
+    if (fork_c || unary) cudaEventRecord(J.fork, st);
+    if (unary) {
+        cudaStreamWaitEvent(J.unary, J.fork, 0);
+        unary_mixed<<<std::min(blocks, (unsigned)kUnaryBlocks), kUnaryThreads, 0, J.unary>>>(P, S, MX);
+        cudaEventRecord(J.unary_join, J.unary);
+        ++kernels;
+    }
+    if (contacts) {
+        const cudaStream_t side = fork_c ? J.side : st;
+        if (fork_c) cudaStreamWaitEvent(side, J.fork, 0);
         // the FP64 positions are current unless the step before integrated in float-float
         MixedExtra MC = MX;
         MC.x64 = prev_fused ? nullptr : S.x;
-        if (!(ver && PV.near_len)) R.rec = nullptr;
         R.lanes = contact_lanes == 1 ? 1 : 2;
         if (R.rec) {
             const unsigned nb = (unsigned)((P.n + R.rb - 1) / R.rb);
-            if (R.rb == 128) mixed_contacts<128><<<nb, 128, 0, side>>>(P, PV, BV, MC, R);
-            else if (R.rb == 64) mixed_contacts<64><<<nb, 64, 0, side>>>(P, PV, BV, MC, R);
-            else mixed_contacts<32><<<nb, 32, 0, side>>>(P, PV, BV, MC, R);
+            if (R.rb == 128) launch_shared(share, mixed_contacts<128>, nb, 128, 0, side, P, PV, BV, MC, R);
+            else if (R.rb == 64) launch_shared(share, mixed_contacts<64>, nb, 64, 0, side, P, PV, BV, MC, R);
+            else launch_shared(share, mixed_contacts<32>, nb, 32, 0, side, P, PV, BV, MC, R);
         } else if (ver && PV.near_len && contact_lanes == 1)
-            launch_contacts<true, 1>(P, S, PV, BV, MC, side, hamaker != 0);
+            launch_contacts<true, 1>(P, S, PV, BV, MC, side, hamaker != 0, share);
         else if (ver && PV.near_len)
-            launch_contacts<true, kContactLanes>(P, S, PV, BV, MC, side, hamaker != 0);
+            launch_contacts<true, kContactLanes>(P, S, PV, BV, MC, side, hamaker != 0, share);
         else
-            launch_contacts<false, 32>(P, S, PV, BV, MC, side, hamaker != 0);
+            launch_contacts<false, 32>(P, S, PV, BV, MC, side, hamaker != 0, share);
+        if (fork_c) cudaEventRecord(J.join, side);
         ++kernels;
     }
     if (hamaker) {
         switch (slices > 0 ? slices : ver ? mixed_hamaker_slices(P.n) : mixed_hamaker_slices_all_pairs(P.n)) {
             case 16:
-                if (ver) launch_hamaker<true, 16, 16>(P, PV, MX, st);
-                else launch_hamaker<false, 32, 16>(P, PV, MX, st);
+                if (ver) launch_hamaker<true, 16, 16>(P, PV, MX, st, share);
+                else launch_hamaker<false, 32, 16>(P, PV, MX, st, share);
                 break;
             case 8:
-                if (ver) launch_hamaker<true, 8, 8>(P, PV, MX, st);
-                else launch_hamaker<false, 32, 8>(P, PV, MX, st);
+                if (ver) launch_hamaker<true, 8, 8>(P, PV, MX, st, share);
+                else launch_hamaker<false, 32, 8>(P, PV, MX, st, share);
                 break;
             case 4:
-                if (ver) launch_hamaker<true, 4, 4>(P, PV, MX, st);
-                else launch_hamaker<false, 16, 4>(P, PV, MX, st);
+                if (ver) launch_hamaker<true, 4, 4>(P, PV, MX, st, share);
+                else launch_hamaker<false, 16, 4>(P, PV, MX, st, share);
                 break;
             case 2:
-                if (ver) launch_hamaker<true, 2, 2>(P, PV, MX, st);
-                else launch_hamaker<false, 8, 2>(P, PV, MX, st);
+                if (ver) launch_hamaker<true, 2, 2>(P, PV, MX, st, share);
+                else launch_hamaker<false, 8, 2>(P, PV, MX, st, share);
                 break;
             default:
-                if (ver) launch_hamaker<true, 1, 1>(P, PV, MX, st);
-                else launch_hamaker<false, 8, 1>(P, PV, MX, st);
+                if (ver) launch_hamaker<true, 1, 1>(P, PV, MX, st, share);
+                else launch_hamaker<false, 8, 1>(P, PV, MX, st, share);
         }
         ++kernels;
     }
-    if (contacts) {
-        cudaEventRecord(join, side);
-        cudaStreamWaitEvent(st, join, 0);
-    }
-    const unsigned blocks = (unsigned)((P.n + 63) / 64);
+    if (fork_c) cudaStreamWaitEvent(st, J.join, 0);
+    if (unary) cudaStreamWaitEvent(st, J.unary_join, 0);
     // without facets or a body term the completion of a run's steps integrates in float-float; the
     // FP64 completion serves the rest (and a run's last step when the step before was not fused)
-    const bool plain = P.n_facets == 0 && !P.ext_a && MX.s32;
+    const bool plain = !unary && MX.s32;
     auto split = [](double d) { const float hi = (float)d; return ff{hi, (float)(d - (double)hi)}; };
     if (plain && kick) {
-        forces_finish_ff<false><<<blocks, 64, 0, st>>>(P, S, contacts, hamaker, split(hdt), split(dt), hdt, dt, MX, PV, R);
+        launch_shared(share, forces_finish_ff<false>, blocks, 64, 0, st, P, S, contacts, hamaker, split(hdt), split(dt), hdt, dt, MX, PV, R);
         return kernels;
     }
     if (plain && prev_fused) {
-        forces_finish_ff<true><<<blocks, 64, 0, st>>>(P, S, contacts, hamaker, split(hdt), split(dt), hdt, dt, MX, PV, R);
+        launch_shared(share, forces_finish_ff<true>, blocks, 64, 0, st, P, S, contacts, hamaker, split(hdt), split(dt), hdt, dt, MX, PV, R);
         return kernels;
     }
-    if (P.n_facets > 0 || P.ext_a)
-        forces_finish_mixed<true><<<blocks, 64, 0, st>>>(P, S, hdt, dt, move_facets, contacts, hamaker, kick ? 1 : 0, MX, PV, R);
+    if (unary)
+        launch_shared(share, forces_finish_mixed<true>, blocks, 64, 0, st, P, S, hdt, dt, move_facets, contacts, hamaker, kick ? 1 : 0, MX, PV, R);
     else
-        forces_finish_mixed<false><<<blocks, 64, 0, st>>>(P, S, hdt, dt, 0, contacts, hamaker, kick ? 1 : 0, MX, PV, R);
+        launch_shared(share, forces_finish_mixed<false>, blocks, 64, 0, st, P, S, hdt, dt, 0, contacts, hamaker, kick ? 1 : 0, MX, PV, R);
     return kernels;
 }
 

@@ -125,6 +125,7 @@ struct MixedExtra {
     // of steps integrated in float-float)
     const dbl4 *x64;
     float q_marg;
+    dbl4 *un_a, *un_al;  // [n] unary terms of the evaluation (systems with facets or a body term)
 };
 bool mixed_available();
 void launch_forces_mixed(int T, const Params &P, const StateView &S, const PairView &PV, const BondView &BV,
@@ -185,8 +186,15 @@ int32_t near_block_rows(int64_t n);
 // Lists the owned contact candidates of every block (after each list build).
 void launch_near_owners(int64_t n, const PairView &PV, const NearScratch &R, cudaStream_t st);
 
-// Warp-compacted mixed-precision kernels (lg_forces_compact_mixed.cu): the contact/bond kernel (if the system has a binary model) on `side`, beside the
-// Hamaker kernel on `st` (fork / join through the two events), then the completion kernel on `st`;
+// Streams and events of the kernels that run beside each other in a mixed evaluation: contacts, and unary
+// terms (null unless the system has some).
+struct SideStreams {
+    cudaStream_t side, unary;
+    cudaEvent_t fork, join, unary_join;
+};
+
+// Warp-compacted mixed-precision kernels (lg_forces_compact_mixed.cu): the contact/bond kernel (if the system has a binary model) on J.side, beside the
+// Hamaker kernel on `st` and the unary terms on J.unary, then the completion kernel on `st`;
 // returns the number of kernels launched.
 // With `kick`, the completion kernel goes on to the next step's opening half kick and drift (and the
 // float-float copies), exactly as launch_kick_drift_mixed would.
@@ -196,8 +204,7 @@ void launch_near_owners(int64_t n, const PairView &PV, const NearScratch &R, cud
 // row of the contact kernel over candidate lists (1 or 2; all pairs take a warp per row).
 int launch_forces_compact_mixed(const Params &P, const StateView &S, const PairView &PV, const BondView &BV, double hdt,
                                 double dt, int move_facets, bool kick, bool prev_fused, const MixedExtra &MX,
-                                cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int slices,
-                                int contact_lanes, NearScratch R);
+                                cudaStream_t st, const SideStreams &J, int slices, int contact_lanes, NearScratch R);
 
 // Layout conversion between a caller's [n][3] doubles (already in device memory) and the padded
 // device layout (lg_reduce.cu).

@@ -413,8 +413,10 @@ __device__ __forceinline__ void contact_rows(const Params &P, const PairView &PV
     ff acc[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}}, accw[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
     __syncwarp();
 
-    // entry of iteration it: partner and slot (-1: none); loaded two iterations ahead, and its flags
-    // and partner position one iteration ahead of its classification
+    // entry of iteration it: partner and slot (-1: none). Candidate lists are loaded two iterations ahead, and
+    // their entries' flags and partner positions one iteration ahead of the classification; with all pairs,
+    // where the partner follows from the slot, kDeep iterations of flags and positions are in flight.
+    constexpr int kDeep = NEAR ? 1 : 4;
     int32_t jn = -1, kn = 0;
     auto load_entry = [&](int64_t it) {
         const int64_t m = it * T + sub;
@@ -429,37 +431,46 @@ __device__ __forceinline__ void contact_rows(const Params &P, const PairView &PV
             }
         }
     };
-    int32_t jc = -1, kc = 0;  // the entry being classified, with its flags and partner position
-    uint32_t flc = 0;
-    float4 pjc = hi_i;
-    auto take_entry = [&]() {  // the loaded entry becomes the current one; its data is requested
+    int32_t jc = -1, kc = 0;  // the entry being classified (candidate lists), the flags and partner positions ahead
+    uint32_t flc[kDeep];
+    float4 pjc[kDeep];
+    auto take_entry = [&](int d) {  // the loaded entry becomes entry d; its data is requested
         jc = jn;
         kc = kn;
-        flc = 0;
-        pjc = hi_i;
-        if (jc >= 0) {
-            flc = PV.flags[(int64_t)kc * n + i];
-            pjc = MX.x32[2 * jc];
+        flc[d] = 0;
+        pjc[d] = hi_i;
+        if (jn >= 0) {
+            flc[d] = PV.flags[(int64_t)kn * n + i];
+            pjc[d] = MX.x32[2 * jn];
         }
     };
-    if (itmax > 0) {
-        load_entry(0);
-        take_entry();
-        if (itmax > 1) load_entry(1);
+#pragma unroll
+    for (int d = 0; d < kDeep; ++d) {
+        load_entry(d);
+        take_entry(d);
     }
+    if (NEAR) load_entry(1);
     for (int64_t it0 = 0; it0 < itmax;) {
         int ccount = 0, cdone = 0;
         int64_t it = it0;
         for (;;) {
             const bool take = it < itmax && it - it0 < kCRound && ccount + 32 <= kCQ;
             if (take) {
-                const int32_t j = jc, k = kc;
-                const uint32_t fl = flc;
-                const float4 pj = pjc;
-                if (it + 1 < itmax) {
-                    take_entry();
-                    if (it + 2 < itmax) load_entry(it + 2);
+                int32_t j = jc, k = kc;
+                if (!NEAR) {
+                    k = (int32_t)(it * T) + sub;
+                    j = k < len ? (k < i ? k : k + 1) : -1;
                 }
+                const uint32_t fl = flc[0];
+                const float4 pj = pjc[0];
+#pragma unroll
+                for (int d = 0; d + 1 < kDeep; ++d) {
+                    flc[d] = flc[d + 1];
+                    pjc[d] = pjc[d + 1];
+                }
+                if (!NEAR) load_entry(it + kDeep);
+                take_entry(kDeep - 1);
+                if (NEAR) load_entry(it + 2);
                 bool cb = false;
                 if (j >= 0) {
                     const float dx = hi_i.x - pj.x, dy = hi_i.y - pj.y, dz = hi_i.z - pj.z;
@@ -514,8 +525,21 @@ __device__ __forceinline__ void contact_rows(const Params &P, const PairView &PV
     }
     if (T > 1) {  // the row's partial sums, in lane order, onto its first lane
         const int base = lane - sub;
+        // a lane without a touching pair adds zeros, which change nothing: with a warp per row such lanes, nearly
+        // all of them, are passed over
+        uint32_t some = 0xffffffffu;
+        if (T == 32) {
+            bool any = false;
 #pragma unroll
+            for (int c = 0; c < 3; ++c) any = any || acc[c].hi != 0.f || acc[c].lo != 0.f || accw[c].hi != 0.f || accw[c].lo != 0.f;
+            some = __ballot_sync(0xffffffffu, any);
+        }
+#pragma unroll(T == 32 ? 1 : T)
         for (int t = 1; t < T; ++t) {
+            if (T == 32) {
+                t = __ffs(some & (0xffffffffu << t)) - 1;
+                if (t < 0) break;
+            }
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const float ah = __shfl_sync(0xffffffffu, acc[c].hi, base + t);
