@@ -90,7 +90,28 @@ int lg_detect_bonds(const double *x0, int64_t n, double r, double dc, bool cycle
     if (n < 2) return LG_OK;
     const double reach = 2.0 * r + dc;
     std::vector<std::pair<int32_t, int32_t>> cand;
-    if (n <= 2048) {
+    bool finite = std::isfinite(reach);
+    for (int64_t q = 0; q < 3 * n; ++q) finite = finite && std::isfinite(x0[q]);
+    // up to 8192 particles a sweep along x: a bonded pair is no further apart than the reach (1000 particles 630 us
+    // by the double loop, about 60 so; the hashed grid wins where the sweep's window holds several hundred)
+    if (n <= 8192 && finite) {
+        const double far = reach > 0 ? reach * (1.0 + 1e-9) : 0.0, far2 = far * far;
+        std::vector<int32_t> order((size_t)n);
+        for (int64_t i = 0; i < n; ++i) order[(size_t)i] = (int32_t)i;
+        std::sort(order.begin(), order.end(), [x0](int32_t a, int32_t b) { return x0[3 * a] < x0[3 * b]; });
+        std::vector<double> p(3 * (size_t)n);
+        for (int64_t q = 0; q < n; ++q)
+            for (int c = 0; c < 3; ++c) p[3 * q + c] = x0[3 * (int64_t)order[(size_t)q] + c];
+        for (int64_t a = 0; a + 1 < n; ++a)
+            for (int64_t b = a + 1; b < n && !(p[3 * b] - p[3 * a] > far); ++b) {
+                const double dx = p[3 * b] - p[3 * a], dy = p[3 * b + 1] - p[3 * a + 1], dz = p[3 * b + 2] - p[3 * a + 2];
+                if ((dx * dx + dy * dy) + dz * dz > far2) continue;
+                const int32_t i = std::min(order[(size_t)a], order[(size_t)b]), j = std::max(order[(size_t)a], order[(size_t)b]);
+                double g = nrm(sub(hld(x0, i), hld(x0, j))) - 2.0 * r;
+                if (bonded(g)) cand.emplace_back(i, j);
+            }
+        std::sort(cand.begin(), cand.end());
+    } else if (n <= 2048) {
         for (int64_t i = 0; i + 1 < n; ++i)
             for (int64_t j = i + 1; j < n; ++j) {
                 double g = nrm(sub(hld(x0, i), hld(x0, j))) - 2.0 * r;
@@ -250,14 +271,6 @@ static void to_dev4(const double *aos, int64_t n, std::vector<dbl4> &tmp) {
     for (int64_t i = 0; i < n; ++i) tmp[i] = make_double4_32a(aos[3 * i], aos[3 * i + 1], aos[3 * i + 2], 0.0);
 }
 
-static int upload4(dbl4 *dst, const double *aos, int64_t n, cudaStream_t st) {
-    std::vector<dbl4> tmp;
-    to_dev4(aos, n, tmp);
-    LG_CUDA(cudaMemcpyAsync(dst, tmp.data(), sizeof(dbl4) * (size_t)n, cudaMemcpyHostToDevice, st));
-    LG_CUDA(cudaStreamSynchronize(st));
-    return LG_OK;
-}
-
 // Origin of one system's float-float positions (mixed precision): the centroid; out[3] receives
 // the largest coordinate offset from it (at least 8 particle radii), which bounds the FP32
 // rounding of the high parts.
@@ -344,11 +357,15 @@ void lg_system::release() {
         else cudaFreeHost(h_pin);
     }
     h_pin = nullptr;
+    allocations.insert(allocations.end(), chunks.begin(), chunks.end());
     for (void *p : allocations) {
         if (pooled && stream) cudaFreeAsync(p, stream);  // in stream order, after the handle's work
         else cudaFree(p);
     }
     allocations.clear();
+    chunks.clear();
+    slab = nullptr;
+    slab_left = 0;
     if (stream) cudaStreamDestroy(stream);
     if (side) cudaStreamDestroy(side);
     if (ev0) cudaEventDestroy(ev0);
@@ -366,18 +383,39 @@ void lg_system::release() {
 
 template <typename U>
 int lg_system::alloc(U **p, size_t count) {
-    if (pooled && stream) {
-        *p = nullptr;
-        cudaError_t e = cudaMallocAsync((void **)p, sizeof(U) * std::max<size_t>(count, 1), stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);  // usable from any stream on return
+    // a pooled handle's buffers, and the small ones of any handle, are cut from chunks
+    const bool pool = pooled && stream;
+    const size_t bytes = (sizeof(U) * std::max<size_t>(count, 1) + 255) / 256 * 256;
+    if (!pool && bytes > ((size_t)256 << 10)) {
+        LG_TRY(dalloc(p, count));
+        allocations.push_back((void *)*p);
+        return LG_OK;
+    }
+    *p = nullptr;
+    if (bytes > slab_left) {
+        size_t chunk = std::max(bytes, pool ? slab_chunk : (size_t)1 << 20);
+        void *c = nullptr;
+        auto get = [&]() { return pool ? cudaMallocAsync(&c, chunk, stream) : cudaMalloc(&c, chunk); };
+        cudaError_t e = get();
+        if (e != cudaSuccess && chunk > bytes) {  // short of memory: no more than asked for
+            cudaGetLastError();
+            chunk = bytes;
+            e = get();
+        }
+        if (e == cudaSuccess && pool) e = cudaStreamSynchronize(stream);  // usable from any stream on return
         if (e != cudaSuccess) {
             cudaGetLastError();
-            return lg_fail(LG_E_NOMEM, "cudaMallocAsync of %zu bytes failed: %s", sizeof(U) * count, cudaGetErrorString(e));
+            return lg_fail(LG_E_NOMEM, "%s of %zu bytes failed: %s", pool ? "cudaMallocAsync" : "cudaMalloc", chunk,
+                           cudaGetErrorString(e));
         }
-    } else {
-        LG_TRY(dalloc(p, count));
+        chunks.push_back(c);
+        slab = (char *)c;
+        slab_left = chunk;
+        slab_chunk = (size_t)1 << 20;
     }
-    allocations.push_back((void *)*p);
+    *p = (U *)slab;
+    slab += bytes;
+    slab_left -= bytes;
     return LG_OK;
 }
 
@@ -503,7 +541,7 @@ static int ensure_step_buffers(lg_system *s) {
     const int64_t groups = (n + 31) / 32;
     const int sl = mixed_hamaker_slices(n);
     LG_TRY(s->alloc(&s->step_ctr, (size_t)(6 + groups)));
-    LG_CUDA(cudaMemset(s->step_ctr, 0, sizeof(unsigned) * (size_t)(6 + groups)));
+    LG_CUDA(cudaMemsetAsync(s->step_ctr, 0, sizeof(unsigned) * (size_t)(6 + groups), s->stream));
     LG_TRY(s->alloc(&s->hpart, 2 * (size_t)4 * (size_t)n));
     s->step_slices = sl;
     s->fstep = 0;
@@ -925,11 +963,20 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
     s->bv.bcap = bcap;
     s->bv.aos = s->precision == LG_PRECISION_MIXED ? 1 : 0;
     s->n_bonds_initial = 2 * (int64_t)bonds.size();
+    std::vector<int8_t> bint;  // host copies of the uploads below, until the stream has taken them
+    std::vector<double> bstr;
+    std::vector<dbl4> up[4];
+    struct Drain {  // also on the ways out before that
+        cudaStream_t st;
+        ~Drain() {
+            if (st) cudaStreamSynchronize(st);
+        }
+    } drain{s->stream};
     {
         const size_t bs = (size_t)bcap * (size_t)n;
         std::vector<int32_t> bj(bs, -1);
-        std::vector<int8_t> bint(bs, 0);
-        std::vector<double> bstr(bs, 0.0);
+        bint.assign(bs, 0);
+        bstr.assign(bs, 0.0);
         std::vector<double> pstr((size_t)n, 0.0);  // particle-indexed strengths of the reference
         std::vector<int32_t> fill((size_t)n, 0);
         for (size_t b = 0; b < bonds.size(); ++b) {
@@ -956,10 +1003,10 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
         LG_TRY(s->alloc(&s->bv.intact, bs));
         LG_TRY(s->alloc(&s->bv.strength, bs));
         LG_TRY(s->alloc(&s->bv.xi, 9 * bs));
-        LG_CUDA(cudaMemcpy(s->bv.j, bj.data(), sizeof(int32_t) * bs, cudaMemcpyHostToDevice));
-        LG_CUDA(cudaMemcpy(s->bv.intact, bint.data(), sizeof(int8_t) * bs, cudaMemcpyHostToDevice));
-        LG_CUDA(cudaMemcpy(s->bv.strength, bstr.data(), sizeof(double) * bs, cudaMemcpyHostToDevice));
-        LG_CUDA(cudaMemset(s->bv.xi, 0, sizeof(double) * 9 * bs));
+        LG_CUDA(cudaMemcpyAsync(s->bv.j, bj.data(), sizeof(int32_t) * bs, cudaMemcpyHostToDevice, s->stream));
+        LG_CUDA(cudaMemcpyAsync(s->bv.intact, bint.data(), sizeof(int8_t) * bs, cudaMemcpyHostToDevice, s->stream));
+        LG_CUDA(cudaMemcpyAsync(s->bv.strength, bstr.data(), sizeof(double) * bs, cudaMemcpyHostToDevice, s->stream));
+        LG_CUDA(cudaMemsetAsync(s->bv.xi, 0, sizeof(double) * 9 * bs, s->stream));
         if (connectors) {
             // the connectors of each bond, sinter_bridge.h:163-197 (evaluated in the reference's
             // order; this file is compiled without contraction)
@@ -1009,18 +1056,24 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
     LG_TRY(s->alloc(&s->a, n));
     LG_TRY(s->alloc(&s->al, n));
     LG_TRY(s->alloc(&s->err, 1));
-    LG_CUDA(cudaMemset(s->err, 0, sizeof(int32_t)));
-    LG_CUDA(cudaMemset(s->a, 0, sizeof(dbl4) * n));
-    LG_CUDA(cudaMemset(s->al, 0, sizeof(dbl4) * n));
-    LG_TRY(upload4(s->x, x0, n, s->stream));
-    LG_TRY(upload4(s->v[0], v0, n, s->stream));
-    LG_TRY(upload4(s->th, th0, n, s->stream));
-    LG_TRY(upload4(s->w[0], om0, n, s->stream));
+    LG_CUDA(cudaMemsetAsync(s->err, 0, sizeof(int32_t), s->stream));
+    LG_CUDA(cudaMemsetAsync(s->a, 0, sizeof(dbl4) * n, s->stream));
+    LG_CUDA(cudaMemsetAsync(s->al, 0, sizeof(dbl4) * n, s->stream));
+    {
+        const double *from[4] = {x0, v0, th0, om0};
+        dbl4 *to[4] = {s->x, s->v[0], s->th, s->w[0]};
+        for (int f = 0; f < 4; ++f) {
+            to_dev4(from[f], n, up[f]);
+            LG_CUDA(cudaMemcpyAsync(to[f], up[f].data(), sizeof(dbl4) * (size_t)n, cudaMemcpyHostToDevice, s->stream));
+        }
+        LG_CUDA(cudaStreamSynchronize(s->stream));
+        drain.st = nullptr;
+    }
     s->vcur = 0;
 
     if (arena) {  // every particle of an empty slot takes no part (no cell, no row, no motion)
         LG_TRY(s->alloc(&s->d_hold, (size_t)n));
-        LG_CUDA(cudaMemset(s->d_hold, (int)kHoldInactive, (size_t)n));
+        LG_CUDA(cudaMemsetAsync(s->d_hold, (int)kHoldInactive, (size_t)n, s->stream));
         P.hold = s->d_hold;
     }
 
@@ -1042,7 +1095,7 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
     LG_TRY(s->alloc(&s->fv[0], 9 * (size_t)nf));
     LG_TRY(s->alloc(&s->fv[1], 9 * (size_t)nf));
     LG_TRY(s->alloc(&s->sxi, 9 * (size_t)nf * (size_t)n));
-    LG_CUDA(cudaMemset(s->sxi, 0, sizeof(double) * 9 * (size_t)nf * (size_t)n));
+    LG_CUDA(cudaMemsetAsync(s->sxi, 0, sizeof(double) * 9 * (size_t)nf * (size_t)n, s->stream));
     if (d->n_facets > 0) {
         std::vector<double> fvh(9 * (size_t)d->n_facets);
         for (int f = 0; f < d->n_facets; ++f)
@@ -1062,7 +1115,7 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
         pv.row_len = nullptr;
         LG_TRY(s->alloc(&pv.flags, (size_t)(cap * n)));
         LG_TRY(s->alloc(&pv.xi, 9 * (size_t)(cap * n)));
-        LG_CUDA(cudaMemset(pv.xi, 0, sizeof(double) * 9 * (size_t)(cap * n)));
+        LG_CUDA(cudaMemsetAsync(pv.xi, 0, sizeof(double) * 9 * (size_t)(cap * n), s->stream));
         std::vector<uint32_t> fl((size_t)(cap * n), 0u);
         for (int64_t b = 0; b < bcap; ++b)
             for (int64_t i = 0; i < n; ++i) {
@@ -1097,12 +1150,12 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
                 LG_TRY(s->alloc(&pv.row_len, (size_t)n));
                 LG_TRY(s->alloc(&pv.flags, (size_t)(c * n)));
                 LG_TRY(s->alloc(&pv.xi, 9 * (size_t)(c * n)));
-                LG_CUDA(cudaMemset(pv.row_len, 0, sizeof(int32_t) * n));
+                LG_CUDA(cudaMemsetAsync(pv.row_len, 0, sizeof(int32_t) * n, s->stream));
                 if (s->r_near > 0) {
                     LG_TRY(s->alloc(&pv.near_j, (size_t)(c * n)));
                     LG_TRY(s->alloc(&pv.near_k, (size_t)(c * n)));
                     LG_TRY(s->alloc(&pv.near_len, (size_t)n));
-                    LG_CUDA(cudaMemset(pv.near_len, 0, sizeof(int32_t) * n));
+                    LG_CUDA(cudaMemsetAsync(pv.near_len, 0, sizeof(int32_t) * n, s->stream));
                 }
             }
             return LG_OK;
@@ -1121,33 +1174,37 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
         LG_TRY(s->alloc(&s->ls.ticket, 1));
         LG_TRY(s->alloc(&s->ls.cursor, 1));
         LG_TRY(s->alloc(&s->ls.cell_cursor, 1));
-        LG_CUDA(cudaMemset(s->ls.cell_cursor, 0, sizeof(int32_t)));
-        LG_CUDA(cudaMemset(s->ls.ticket, 0, sizeof(unsigned)));
+        LG_CUDA(cudaMemsetAsync(s->ls.cell_cursor, 0, sizeof(int32_t), s->stream));
+        LG_CUDA(cudaMemsetAsync(s->ls.ticket, 0, sizeof(unsigned), s->stream));
         LG_TRY(s->alloc(&s->ls.x32, (size_t)n));
         LG_TRY(s->alloc(&s->ls.max_row, 1));
         if (s->precision == LG_PRECISION_FP64 || s->r_near > 0) LG_TRY(s->alloc(&s->own_n, (size_t)n / 4 + 1));
-        LG_CUDA(cudaMemset(s->ls.max_row, 0, sizeof(int32_t)));
+        LG_CUDA(cudaMemsetAsync(s->ls.max_row, 0, sizeof(int32_t), s->stream));
         LG_TRY(rebuild_list(s));
         // without an explicit max_neighbors the row capacity follows the initial state: rows get
         // 1.5x the longest initial row (at most 255)
         int32_t mr = 0;
-        LG_CUDA(cudaMemcpy(&mr, s->ls.max_row, sizeof(int32_t), cudaMemcpyDeviceToHost));
+        if (d->max_neighbors == 0) {
+            LG_CUDA(cudaMemcpyAsync(&mr, s->ls.max_row, sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream));
+            LG_CUDA(cudaStreamSynchronize(s->stream));
+        }
         const int64_t want = std::min<int64_t>(255, std::max<int64_t>(8, (int64_t)(1.5 * mr) + 1));
         if (d->max_neighbors == 0 && want > cap && cap < std::max<int64_t>(n - 1, 1)) {
             for (int q = 0; q < 2; ++q) {
                 PairView &pv = s->pv[q];
                 void *old_ptrs[7] = {pv.nbr, pv.row_len, pv.flags, pv.xi, pv.near_j, pv.near_k, pv.near_len};
                 for (void *o : old_ptrs) {
-                    if (!o) continue;
+                    const auto it = std::find(s->allocations.begin(), s->allocations.end(), o);
+                    if (!o || it == s->allocations.end()) continue;  // null, or part of a chunk
                     cudaFree(o);
-                    s->allocations.erase(std::find(s->allocations.begin(), s->allocations.end(), o));
+                    s->allocations.erase(it);
                 }
             }
             cap = std::min<int64_t>(want, std::max<int64_t>(n - 1, 1));
             LG_TRY(alloc_rows(cap));
             s->list_built = false;
             s->pcur = 0;
-            LG_CUDA(cudaMemset(s->err, 0, sizeof(int32_t)));
+            LG_CUDA(cudaMemsetAsync(s->err, 0, sizeof(int32_t), s->stream));
             LG_TRY(rebuild_list(s));
         }
     }
@@ -1157,10 +1214,10 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
     LG_TRY(s->alloc(&s->obs_scratch, (size_t)obs_scratch_doubles(n)));
     if (s->precision == LG_PRECISION_FP64) {
         LG_TRY(s->alloc(&s->d_queue_n, 1));
-        LG_CUDA(cudaMemset(s->d_queue_n, 0, sizeof(int32_t)));
+        LG_CUDA(cudaMemsetAsync(s->d_queue_n, 0, sizeof(int32_t), s->stream));
     }
     LG_TRY(s->alloc(&s->d_ticket, 1));
-    LG_CUDA(cudaMemset(s->d_ticket, 0, sizeof(unsigned)));
+    LG_CUDA(cudaMemsetAsync(s->d_ticket, 0, sizeof(unsigned), s->stream));
     if (s->pooled) {  // plain host memory: freeing pinned memory can synchronise the device
         s->h_pin = (double *)std::malloc(64 * sizeof(double));
         if (!s->h_pin) return lg_fail(LG_E_NOMEM, "lg_create: host allocation failed");
@@ -1251,7 +1308,7 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
     LG_TRY(apply_unary(s, &d->body, d->unary_hook, d->unary_hook_user));
     // initial accelerations (the first half kick needs them); velocities are unchanged (hdt = 0)
     LG_TRY(launch_forces(s, 0.0, 0.0, 0));
-    LG_CUDA(cudaStreamSynchronize(s->stream));
+    if (!s->pooled) LG_CUDA(cudaStreamSynchronize(s->stream));  // a pooled handle's importer waits for it
     return LG_OK;
 }
 
@@ -2008,6 +2065,7 @@ int lg_create_staged(const lg_system_desc *desc, const double *x0, const double 
     lg_system *s = new (std::nothrow) lg_system();
     if (!s) return lg_fail(LG_E_NOMEM, "lg_create_staged: host allocation failed");
     s->pooled = true;
+    s->slab_chunk = (size_t)std::max<int64_t>(lg_estimate_device_bytes(desc, desc->n_part), 0);
     static std::mutex pool_mu;
     static std::vector<int> pool_set;  // devices whose default pool keeps freed memory for reuse
     {

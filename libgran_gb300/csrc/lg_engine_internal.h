@@ -154,6 +154,11 @@ struct lg_system {
     // device memory from the stream-ordered pool (cudaMallocAsync / cudaFreeAsync on the handle's
     // stream): releasing such a handle does not synchronise the device (serving's staging handles)
     bool pooled = false;
+    // such a handle's allocations are cut from a few chunks: slab_chunk bytes the first time (what the
+    // handle is expected to need), then 1 MiB or the allocation's own size (any handle's small ones: 1 MiB)
+    std::vector<void *> chunks;
+    char *slab = nullptr;
+    size_t slab_left = 0, slab_chunk = 0;
 
     template <typename U>
     int alloc(U **p, size_t count);

@@ -29,15 +29,25 @@ __device__ __forceinline__ double hamaker_slope(int mode, double A, double r, do
                       2.0 * r * r * (4.0 * r + 2.0 * h) / ((4.0 * r + h) * (4.0 * r + h)) / (h * h);
     return -A / 6.0 * br;
 }
-__device__ __forceinline__ double hamaker_energy(int mode, const lg_hamaker_params &p, double dist) {
-    const double r = p.r_part, h = dist - 2.0 * r;
-    double u = h < p.h0 ? hamaker_u0(mode, p.A, r, p.h0) + hamaker_slope(mode, p.A, r, p.h0) * (h - p.h0)
-                        : hamaker_u0(mode, p.A, r, h);
-    if (mode == LG_HAMAKER_LIMITED) {
-        const double hc = p.r_cutoff - 2.0 * r;
-        u -= hc < p.h0 ? hamaker_u0(mode, p.A, r, p.h0) + hamaker_slope(mode, p.A, r, p.h0) * (hc - p.h0)
-                       : hamaker_u0(mode, p.A, r, hc);
-    }
+// The pair-independent parts of the energy, the same in every lane: potential and slope at h0, and the
+// shift of the limited form. Lane parity picks the argument, so that one evaluation serves both points.
+struct HamakerAt {
+    double u_h0, slope_h0, shift;
+};
+__device__ __forceinline__ HamakerAt hamaker_at(int mode, const lg_hamaker_params &p, int lane) {
+    const double r = p.r_part, hc = p.r_cutoff - 2.0 * r;
+    const double u = hamaker_u0(mode, p.A, r, (lane & 1) ? hc : p.h0);
+    HamakerAt c;
+    c.slope_h0 = hamaker_slope(mode, p.A, r, p.h0);
+    c.u_h0 = __shfl_sync(0xffffffffu, u, 0);
+    const double u_hc = __shfl_sync(0xffffffffu, u, 1);
+    c.shift = mode != LG_HAMAKER_LIMITED ? 0.0 : hc < p.h0 ? c.u_h0 + c.slope_h0 * (hc - p.h0) : u_hc;
+    return c;
+}
+__device__ __forceinline__ double hamaker_energy(int mode, const lg_hamaker_params &p, const HamakerAt &c, double dist) {
+    const double h = dist - 2.0 * p.r_part;
+    double u = h < p.h0 ? c.u_h0 + c.slope_h0 * (h - p.h0) : hamaker_u0(mode, p.A, p.r_part, h);
+    if (mode == LG_HAMAKER_LIMITED) u -= c.shift;
     return u;
 }
 
@@ -45,13 +55,87 @@ __device__ __forceinline__ double hamaker_energy(int mode, const lg_hamaker_para
 //  0 e_tot  1 m|v|^2  2 I|w|^2  3-5 v  6-8 I w  9-11 x cross m v  12-14 x  15 potential energy
 //  16 contacts  17 intact bonds
 // Rows of particles row0 .. row0 + count - 1 into out rows 0 .. count - 1.
-__global__ void obs_rows(Params P, StateView S, PairView PV, BondView BV, double m, double I, int pairs,
-                         double *__restrict__ out, int64_t row0, int64_t count) {
+// Bound by the FP64 pipe's issue and by the length of one warp's chain of FP64 instructions (a potential
+// holds four divisions and a logarithm), so a row's slots go to eight lanes, whose energies are added in
+// slot order: a row of 23 partners fills three rounds, and the slots of 1024 rows 256 warps instead of 32 (a
+// served aggregate of 64 to 1024 monomers, with the sums' columns side by side: 440 -> 56 us).
+constexpr int kObsLanes = 8, kObsRowThreads = 64;
+__global__ void __launch_bounds__(kObsRowThreads) obs_rows(Params P, StateView S, PairView PV, BondView BV, double m,
+                                                           double I, int pairs, double *__restrict__ out, int64_t row0,
+                                                           int64_t count) {
     const int64_t n = P.n;
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= count) return;
-    const int64_t i = row0 + t;
-    const d3 v = ld4(S.v, i), w = ld4(S.w, i), x = ld4(S.x, i);
+    const int lane = threadIdx.x & 31, l = lane & (kObsLanes - 1);
+    const int64_t t = (blockIdx.x * (int64_t)kObsRowThreads + threadIdx.x) / kObsLanes;
+    const bool row = t < count;  // the lanes past the last row go along with empty rows
+    const int64_t i = row0 + (row ? t : 0);
+    const d3 x = ld4(S.x, i);
+    double pe = 0.0;
+    int ncont = 0, nbond = 0;
+    const bool ver = P.pairs == LG_PAIRS_VERLET;
+    const int64_t len = !pairs || !row ? 0 : ver ? (int64_t)PV.row_len[i] : n - 1;
+    const int64_t xs = PV.cap * n, bs = (int64_t)BV.bcap * n;
+    const bool hamaker = P.hamaker_model != LG_HAMAKER_NONE;
+    HamakerAt at{};
+    if (pairs && hamaker) at = hamaker_at(P.hamaker_model, P.hamaker, lane);
+    const int64_t longest = __reduce_max_sync(0xffffffffu, (int)len);
+    for (int64_t k0 = 0; k0 < longest; k0 += kObsLanes) {
+        const int64_t k = k0 + l;
+        double u = 0.0;
+        bool touch = false, bond = false;
+        if (k < len) {
+            const int64_t e = k * n + i;
+            const int64_t j = ver ? (int64_t)PV.nbr[e] : (k < i ? k : k + 1);
+            const uint32_t fl = PV.flags[e];
+            const double dist = nrm(sub(x, ld4(S.x, j)));
+            if ((fl & kBonded) && BV.cn) {  // 5-connector model: the connector springs
+                const int64_t be = (int64_t)bond_slot_of(fl) * n + i, ej = (int64_t)BV.rev[be] * n + j;
+                for (int k = 0; k < 5; ++k) {
+                    const d3 ci = mk3(BV.cn[(3 * k) * bs + be], BV.cn[(3 * k + 1) * bs + be], BV.cn[(3 * k + 2) * bs + be]);
+                    const d3 cj = mk3(BV.cn[(3 * k) * bs + ej], BV.cn[(3 * k + 1) * bs + ej], BV.cn[(3 * k + 2) * bs + ej]);
+                    const double dl = (k < 4 ? 2.0 * P.contact.r_part : 0.0) - nrm(sub(cj, ci));
+                    u += 0.5 * P.connector.k_d * dl * dl;
+                }
+                bond = true;
+            } else if (fl & kBonded) {
+                const int64_t be = (int64_t)bond_slot_of(fl) * n + i;
+                double dl = 2.0 * P.sinter.r_part - dist;
+                u += 0.5 * P.sinter.k * dl * dl;
+                const bool f = P.springs_ff != 0;
+                d3 s0 = mk3(spring_load(BV.xi, spring_at(BV.aos, 0, be, bs), f), spring_load(BV.xi, spring_at(BV.aos, 1, be, bs), f), spring_load(BV.xi, spring_at(BV.aos, 2, be, bs), f));
+                d3 s1 = mk3(spring_load(BV.xi, spring_at(BV.aos, 3, be, bs), f), spring_load(BV.xi, spring_at(BV.aos, 4, be, bs), f), spring_load(BV.xi, spring_at(BV.aos, 5, be, bs), f));
+                d3 s2 = mk3(spring_load(BV.xi, spring_at(BV.aos, 6, be, bs), f), spring_load(BV.xi, spring_at(BV.aos, 7, be, bs), f), spring_load(BV.xi, spring_at(BV.aos, 8, be, bs), f));
+                u += 0.5 * P.sinter.k_t * sqn(s0) + 0.5 * P.sinter.k_r * sqn(s1) + 0.5 * P.sinter.k_o * sqn(s2);
+                bond = true;
+            } else if (P.binary_model != LG_BINARY_NONE) {
+                double dl = 2.0 * P.contact.r_part - dist;
+                if (dl > 0) {
+                    u += 0.5 * P.contact.k * dl * dl;
+                    touch = true;
+                }
+                if (fl & kXiLive) {
+                    const bool f = P.springs_ff != 0;
+                    d3 s0 = mk3(spring_load(PV.xi, spring_at(PV.aos, 0, e, xs), f), spring_load(PV.xi, spring_at(PV.aos, 1, e, xs), f), spring_load(PV.xi, spring_at(PV.aos, 2, e, xs), f));
+                    d3 s1 = mk3(spring_load(PV.xi, spring_at(PV.aos, 3, e, xs), f), spring_load(PV.xi, spring_at(PV.aos, 4, e, xs), f), spring_load(PV.xi, spring_at(PV.aos, 5, e, xs), f));
+                    d3 s2 = mk3(spring_load(PV.xi, spring_at(PV.aos, 6, e, xs), f), spring_load(PV.xi, spring_at(PV.aos, 7, e, xs), f), spring_load(PV.xi, spring_at(PV.aos, 8, e, xs), f));
+                    u += 0.5 * P.contact.k_t * sqn(s0) + 0.5 * P.contact.k_r * sqn(s1) + 0.5 * P.contact.k_o * sqn(s2);
+                }
+            }
+            if (P.hamaker_model == LG_HAMAKER_FULL || P.hamaker_model == LG_HAMAKER_SIMPLIFIED ||
+                (P.hamaker_model == LG_HAMAKER_LIMITED && !(dist > P.hamaker.r_cutoff)))
+                u += hamaker_energy(P.hamaker_model, P.hamaker, at, dist);
+        }
+        const unsigned mine = 0xffu << (lane & ~(kObsLanes - 1));
+        ncont += __popc(__ballot_sync(0xffffffffu, touch) & mine);
+        nbond += __popc(__ballot_sync(0xffffffffu, bond) & mine);
+        const double half = 0.5 * u;
+#pragma unroll
+        for (int q = 0; q < kObsLanes; ++q) {
+            const double hq = __shfl_sync(0xffffffffu, half, q, kObsLanes);
+            if (k0 + q < len) pe += hq;
+        }
+    }
+    if (!row || l != 0) return;
+    const d3 v = ld4(S.v, i), w = ld4(S.w, i);
     double *o = out + t * kObs;
     o[0] = m * dot(v, v) / 2.0 + I * dot(w, w) / 2.0;
     o[1] = m * dot(v, v);
@@ -62,79 +146,32 @@ __global__ void obs_rows(Params P, StateView S, PairView PV, BondView BV, double
     d3 L = crs(x, scl(m, v));
     o[9] = L.x; o[10] = L.y; o[11] = L.z;
     o[12] = x.x; o[13] = x.y; o[14] = x.z;
-    double pe = 0.0, ncont = 0.0, nbond = 0.0;
-    const bool ver = P.pairs == LG_PAIRS_VERLET;
-    const int64_t len = !pairs ? 0 : ver ? (int64_t)PV.row_len[i] : n - 1;
-    const int64_t xs = PV.cap * n, bs = (int64_t)BV.bcap * n;
-    for (int64_t k = 0; k < len; ++k) {
-        const int64_t e = k * n + i;
-        const int64_t j = ver ? (int64_t)PV.nbr[e] : (k < i ? k : k + 1);
-        const uint32_t fl = PV.flags[e];
-        const double dist = nrm(sub(x, ld4(S.x, j)));
-        double u = 0.0;
-        if ((fl & kBonded) && BV.cn) {  // 5-connector model: the connector springs
-            const int64_t be = (int64_t)bond_slot_of(fl) * n + i, ej = (int64_t)BV.rev[be] * n + j;
-            for (int k = 0; k < 5; ++k) {
-                const d3 ci = mk3(BV.cn[(3 * k) * bs + be], BV.cn[(3 * k + 1) * bs + be], BV.cn[(3 * k + 2) * bs + be]);
-                const d3 cj = mk3(BV.cn[(3 * k) * bs + ej], BV.cn[(3 * k + 1) * bs + ej], BV.cn[(3 * k + 2) * bs + ej]);
-                const double dl = (k < 4 ? 2.0 * P.contact.r_part : 0.0) - nrm(sub(cj, ci));
-                u += 0.5 * P.connector.k_d * dl * dl;
-            }
-            nbond += 1.0;
-        } else if (fl & kBonded) {
-            const int64_t be = (int64_t)bond_slot_of(fl) * n + i;
-            double dl = 2.0 * P.sinter.r_part - dist;
-            u += 0.5 * P.sinter.k * dl * dl;
-            const bool f = P.springs_ff != 0;
-            d3 s0 = mk3(spring_load(BV.xi, spring_at(BV.aos, 0, be, bs), f), spring_load(BV.xi, spring_at(BV.aos, 1, be, bs), f), spring_load(BV.xi, spring_at(BV.aos, 2, be, bs), f));
-            d3 s1 = mk3(spring_load(BV.xi, spring_at(BV.aos, 3, be, bs), f), spring_load(BV.xi, spring_at(BV.aos, 4, be, bs), f), spring_load(BV.xi, spring_at(BV.aos, 5, be, bs), f));
-            d3 s2 = mk3(spring_load(BV.xi, spring_at(BV.aos, 6, be, bs), f), spring_load(BV.xi, spring_at(BV.aos, 7, be, bs), f), spring_load(BV.xi, spring_at(BV.aos, 8, be, bs), f));
-            u += 0.5 * P.sinter.k_t * sqn(s0) + 0.5 * P.sinter.k_r * sqn(s1) + 0.5 * P.sinter.k_o * sqn(s2);
-            nbond += 1.0;
-        } else if (P.binary_model != LG_BINARY_NONE) {
-            double dl = 2.0 * P.contact.r_part - dist;
-            if (dl > 0) {
-                u += 0.5 * P.contact.k * dl * dl;
-                ncont += 1.0;
-            }
-            if (fl & kXiLive) {
-                const bool f = P.springs_ff != 0;
-                d3 s0 = mk3(spring_load(PV.xi, spring_at(PV.aos, 0, e, xs), f), spring_load(PV.xi, spring_at(PV.aos, 1, e, xs), f), spring_load(PV.xi, spring_at(PV.aos, 2, e, xs), f));
-                d3 s1 = mk3(spring_load(PV.xi, spring_at(PV.aos, 3, e, xs), f), spring_load(PV.xi, spring_at(PV.aos, 4, e, xs), f), spring_load(PV.xi, spring_at(PV.aos, 5, e, xs), f));
-                d3 s2 = mk3(spring_load(PV.xi, spring_at(PV.aos, 6, e, xs), f), spring_load(PV.xi, spring_at(PV.aos, 7, e, xs), f), spring_load(PV.xi, spring_at(PV.aos, 8, e, xs), f));
-                u += 0.5 * P.contact.k_t * sqn(s0) + 0.5 * P.contact.k_r * sqn(s1) + 0.5 * P.contact.k_o * sqn(s2);
-            }
-        }
-        if (P.hamaker_model == LG_HAMAKER_FULL || P.hamaker_model == LG_HAMAKER_SIMPLIFIED ||
-            (P.hamaker_model == LG_HAMAKER_LIMITED && !(dist > P.hamaker.r_cutoff)))
-            u += hamaker_energy(P.hamaker_model, P.hamaker, dist);
-        pe += 0.5 * u;
-    }
     o[15] = pe;
-    o[16] = ncont;
-    o[17] = nbond;
+    o[16] = (double)ncont;
+    o[17] = (double)nbond;
     o[18] = 0.0;
     o[19] = 0.0;
 }
 
 // |x - c|^2 per particle into column 18; c = (column sums 12..14) / n, read from device memory.
-// One block of 1024 threads: thread t sums rows t, t + 1024, ... in order, then a fixed tree.
-__global__ void __launch_bounds__(1024) obs_reduce(int64_t n, const double *__restrict__ rows, int c0, int c1,
+// One block of 1024 threads per column: thread t sums rows t, t + 1024, ... in order, then a fixed tree (a
+// chain of barriers, so the columns go side by side).
+__global__ void __launch_bounds__(1024) obs_reduce(int64_t n, const double *__restrict__ rows, int c0,
                                                    double *__restrict__ out) {
     __shared__ double s[1024];
-    for (int c = c0; c < c1; ++c) {
-        double acc = 0.0;
-        for (int64_t i = threadIdx.x; i < n; i += blockDim.x) acc += rows[i * kObs + c];
-        s[threadIdx.x] = acc;
-        __syncthreads();
-        for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-            if ((int)threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[c] = s[0];
+    const int c = c0 + (int)blockIdx.x;
+    double acc = 0.0;
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) acc += rows[i * kObs + c];
+    s[threadIdx.x] = acc;
+    __syncthreads();
+    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
+        if ((int)threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
         __syncthreads();
     }
+    if (threadIdx.x == 0) out[c] = s[0];
 }
+
+static unsigned obs_row_blocks(int64_t rows) { return (unsigned)((rows * kObsLanes + kObsRowThreads - 1) / kObsRowThreads); }
 
 int64_t obs_scratch_doubles(int64_t n) { return n * kObs; }
 
@@ -273,9 +310,8 @@ void launch_observables_state(int64_t n, const dbl4 *x, const dbl4 *v, const dbl
 void launch_observables_pairs(const Params &P, const StateView &S, const PairView &PV, const BondView &BV, double mass,
                               double inertia, double *scratch, double *out, cudaStream_t st) {
     const int64_t n = P.n;
-    const unsigned blocks = (unsigned)((n + 255) / 256);
-    obs_rows<<<blocks, 256, 0, st>>>(P, S, PV, BV, mass, inertia, 1, scratch, 0, P.n);
-    obs_reduce<<<1, 1024, 0, st>>>(n, scratch, 15, 18, out);
+    obs_rows<<<obs_row_blocks(n), kObsRowThreads, 0, st>>>(P, S, PV, BV, mass, inertia, 1, scratch, 0, P.n);
+    obs_reduce<<<3, 1024, 0, st>>>(n, scratch, 15, out);
 }
 
 // out receives the column sums 0..17 (the pair columns 15..17 are zero unless `pairs`). The caller
@@ -283,38 +319,35 @@ void launch_observables_pairs(const Params &P, const StateView &S, const PairVie
 void launch_observables(const Params &P, const StateView &S, const PairView &PV, const BondView &BV, double mass,
                         double inertia, double *scratch, double *out, cudaStream_t st, bool pairs) {
     const int64_t n = P.n;
-    const unsigned blocks = (unsigned)((n + 255) / 256);
-    obs_rows<<<blocks, 256, 0, st>>>(P, S, PV, BV, mass, inertia, pairs ? 1 : 0, scratch, 0, n);
-    obs_reduce<<<1, 1024, 0, st>>>(n, scratch, 0, 18, out);
+    obs_rows<<<obs_row_blocks(n), kObsRowThreads, 0, st>>>(P, S, PV, BV, mass, inertia, pairs ? 1 : 0, scratch, 0, n);
+    obs_reduce<<<18, 1024, 0, st>>>(n, scratch, 0, out);
 }
 
 void launch_observables_range(const Params &P, const StateView &S, const PairView &PV, const BondView &BV,
                               double mass, double inertia, int64_t row0, int64_t count, double *scratch, double *out,
                               cudaStream_t st) {
     if (count <= 0) return;
-    obs_rows<<<(unsigned)((count + 255) / 256), 256, 0, st>>>(P, S, PV, BV, mass, inertia, 1, scratch, row0, count);
-    obs_reduce<<<1, 1024, 0, st>>>(count, scratch, 0, 18, out);
+    obs_rows<<<obs_row_blocks(count), kObsRowThreads, 0, st>>>(P, S, PV, BV, mass, inertia, 1, scratch, row0, count);
+    obs_reduce<<<18, 1024, 0, st>>>(count, scratch, 0, out);
 }
 
 
-// One block per system: fixed-order sums of the system's scratch rows (columns 0..17).
+// One block per system and column: fixed-order sums of the system's scratch rows (columns 0..17).
 __global__ void __launch_bounds__(256) seg_sums(const int64_t *__restrict__ off, const double *__restrict__ rows,
                                                 double *__restrict__ out) {
     __shared__ double s[256];
     const int64_t sys = blockIdx.x;
     const int64_t b = off[sys], e = off[sys + 1];
-    for (int c = 0; c < 18; ++c) {
-        double acc = 0.0;
-        for (int64_t i = b + threadIdx.x; i < e; i += blockDim.x) acc += rows[i * kObs + c];
-        s[threadIdx.x] = acc;
-        __syncthreads();
-        for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-            if ((int)threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[sys * kObs + c] = s[0];
+    const int c = (int)blockIdx.y;
+    double acc = 0.0;
+    for (int64_t i = b + threadIdx.x; i < e; i += blockDim.x) acc += rows[i * kObs + c];
+    s[threadIdx.x] = acc;
+    __syncthreads();
+    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
+        if ((int)threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
         __syncthreads();
     }
+    if (threadIdx.x == 0) out[sys * kObs + c] = s[0];
 }
 
 __global__ void __launch_bounds__(256) seg_rg(const int64_t *__restrict__ off, const dbl4 *__restrict__ x,
@@ -339,7 +372,7 @@ __global__ void __launch_bounds__(256) seg_rg(const int64_t *__restrict__ off, c
 
 void launch_segmented_sums(int64_t n_systems, const int64_t *offsets, const double *scratch, double *out,
                            cudaStream_t st) {
-    if (n_systems > 0) seg_sums<<<(unsigned)n_systems, 256, 0, st>>>(offsets, scratch, out);
+    if (n_systems > 0) seg_sums<<<dim3((unsigned)n_systems, 18), 256, 0, st>>>(offsets, scratch, out);
 }
 
 void launch_segmented_rg(int64_t n, int64_t n_systems, const int64_t *offsets, const dbl4 *x, const double *centres,

@@ -101,6 +101,8 @@ extern "C" int64_t lg_estimate_device_bytes(const lg_system_desc *d, int64_t n) 
     b += 72 * std::max(d->n_facets, 1) * n;                   // facet springs
     b += 4 * 8 * n + 4 * 4 * n;                               // list scratch
     b += 20 * 8 * n;                                          // observables scratch
+    if (d->precision == LG_PRECISION_MIXED && (d->n_facets > 0 || d->body.model != LG_BODY_NONE || d->unary_hook))
+        b += 2 * 32 * n;                                      // unary terms
     if (d->precision == LG_PRECISION_FP64 && d->pairs == LG_PAIRS_ALL)
         b += 72 * cap * n;                                    // pair kernels' records and queue
     else if (d->precision == LG_PRECISION_FP64 && cap * n <= ((int64_t)1 << 21))

@@ -187,3 +187,20 @@ def test_mixed_unary_terms_beside_the_pairs(count):
             assert np.array_equal(f[q * n:(q + 1) * n], f[:n]), q
     ref = _run(desc(n, A.LG_PRECISION_FP64), x0, v0, [], facets=[wall])
     assert H.rel_err(a[0][:n], ref[0]) <= 1e-6
+
+
+@pytest.mark.parametrize("precision", [A.LG_PRECISION_FP64, A.LG_PRECISION_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("m", [5, 7, 10])
+def test_rows_that_outgrow_their_first_capacity(m, precision):
+    """A cubic lattice at contact: 56 partners within 4.5 r, more than the 48 slots that rows start with. The handle
+    moves to longer rows at its creation; it steps as one that was given them."""
+    mat = K.Material()
+    g = np.arange(m) * 2.0 * mat.r * 0.999
+    x0 = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3)
+    v0 = generate_velocities(3, len(x0), 0.1)
+    runs = []
+    for cap in (0, 84):
+        _, d = _desc(len(x0), A.LG_BINARY_CONTACT, A.LG_HAMAKER_LIMITED, A.LG_PAIRS_VERLET, A.LG_FORCE_KERNEL_AUTO, precision,
+                     max_neighbors=cap)
+        runs.append(_run(d, x0, v0, [(1, 0), (25, 10)]))
+    _same(*runs)
