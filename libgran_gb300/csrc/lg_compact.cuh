@@ -1,7 +1,6 @@
-// lg_compact.cuh -- pieces shared by the FP64 (lg_forces_compact.cu) and mixed-precision
-// (lg_forces_compact_mixed.cu) warp-compacted force kernels: the slot windows, the slicing of a
-// row's windows over several warps, and the per-particle tail of a force evaluation (unary facet
-// terms, stores, half kick, finiteness check). Everything here is inline device code, so each
+// lg_compact.cuh -- pieces shared by the FP64 (lg_forces_pairs.cu, lg_forces_fp64.cu) and
+// mixed-precision (lg_forces_compact_mixed.cu) force kernels: the window size and the per-particle
+// tail of a force evaluation (unary facet terms, stores, half kick, finiteness check). Everything here is inline device code, so each
 // translation unit compiles it with its own floating-point flags.
 #pragma once
 #include "lg_common.cuh"

@@ -1,25 +1,25 @@
-// lg_forces_compact_mixed.cu -- force evaluation of the mixed-precision path (sm_103a): two
-// warp-compacted kernels, one lane per row (particle i), slot layout and flags shared with the FP64
-// path.
+// lg_forces_compact_mixed.cu -- force evaluation of the mixed-precision path (sm_103a): contacts,
+// Hamaker pairs and unary terms on three streams, then a completion; slot layout and flags shared
+// with the FP64 path.
 //
-//   forces_contacts_mixed  contact and bond pairs. Verlet mode walks each row's contact candidates
-//                          (PairView::near_*, listed by the list build: the slots within contact
-//                          reach plus the Verlet skin, and bonded slots); all-pairs mode walks every
-//                          slot. Candidates are queued per warp (ballot order) and evaluated 32 at a
-//                          time; the pair's linear and angular accelerations are folded per row in
-//                          slot order into float-float sums (MixedExtra::csum).
-//   forces_hamaker_mixed   Hamaker pairs over all slots, in windows of four slots: the owner lane
-//                          gathers its partners' float-float positions, the window's Hamaker pairs
-//                          are evaluated one per lane from those shared-memory copies, the next
-//                          window's partners are loaded meanwhile. For launches with few rows a
-//                          row's windows are sliced over SL warps, whose partial sums are combined
-//                          in slice order. Runs beside forces_contacts_mixed (two streams).
+//   mixed_contacts         contact and bond pairs of listed systems, each unordered pair once: the owned
+//                          contact candidates (near_owners, after each list build) are queued per block and
+//                          evaluated a warp at a time; each order's accelerations go to a record per
+//                          candidate, which the completion adds per row in entry order.
+//   forces_contacts_mixed  contact and bond pairs row by row: small lists, all pairs, and systems whose two
+//                          orders of a pair may break differently. Candidates are queued per warp (ballot
+//                          order) and evaluated 32 at a time, folded per row in slot order into
+//                          float-float sums (MixedExtra::csum).
+//   forces_hamaker_mixed   Hamaker pairs over all slots, in windows of four slots held in registers, L
+//                          lanes per row; the windows' sums are added in the order that the slicing
+//                          defines. Runs beside the contact kernel (two streams).
+//   unary_mixed            facet and body terms (FP64), on a third stream.
 //   forces_finish_ff       completion inside a run of steps (no facets, no body term): the sums, the
 //                          end-of-step half kick, the next step's half kick and drift, all in
 //                          float-float on the FP32 pipes; the run's last step writes the FP64 state.
 //   forces_finish_mixed    the FP64 completion (facets, body terms, single steps): contact part +
-//                          Hamaker part to FP64, unary terms, stores, half kick (+ next kick and
-//                          drift).
+//                          Hamaker part to FP64, the unary terms added, stores, half kick (+ next kick
+//                          and drift).
 //
 // The per-pair and per-row pieces (and the precision scheme) are in lg_mixed_pairs.cuh, shared with
 // the persistent step kernel (lg_step_mixed.cu). Per-row sums are in an order fixed by the row
@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <cstddef>
 
+#include "lg_launch.cuh"
 #include "lg_mixed_pairs.cuh"
 
 namespace lg {
@@ -47,9 +48,8 @@ constexpr int kCWarps = 2;   // warps per block
 constexpr int kHThreads = 128;  // threads per block of the Hamaker kernel
 // Resident blocks per SM the contact kernel is compiled for (its register budget): beside the Hamaker
 // kernel (two streams) a tighter budget lets more of both kernels' warps share an SM; alone, the
-// looser one avoids spills. Measured on the 32768-particle workload (graph-replayed steps): 12 blocks
-// beside the Hamaker kernel, 9.3e8 against 8.2e8 particle-steps/s with 8; contacts alone, 8 blocks,
-// 30 against 36 us per step with 12.
+// looser one avoids spills: contacts alone on 32768 particles, 8 blocks, 30 against 36 us per step
+// with 12. All pairs take the looser one in either place (a warp per row: small launches).
 #ifndef LG_CONTACT_MIN_BLOCKS
 #define LG_CONTACT_MIN_BLOCKS 12
 #endif
@@ -482,29 +482,6 @@ __global__ void __launch_bounds__(64) forces_finish_ff(Params P, StateView S, in
 
 namespace {
 
-// Launch with a share of the SM's memory set aside as shared memory (per cent; a hint).
-// An SM changes that share only while it is idle, and by default it follows the kernel's own use: kernels that
-// use none (Hamaker pairs) and some (contacts) then cannot be on one SM together, and one stream's kernel waits
-// for the other's to end: single steps of 8000 listed particles took 40 us as soon as an SM held more than one
-// contact block, and take 29 with one share for all; all pairs of 700 took 39 and take 23. (A share just large
-// enough did not help everywhere: 42 with 64 KB for all pairs of 700.) The unary terms' kernel states no
-// preference: with the others' share the restructuring batch takes 170 us a step instead of 145.
-template <typename... P, typename... A>
-void launch_shared(int share, void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t st,
-                   const A &...args) {
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
-    at.val.sharedMemCarveout = (unsigned)share;
-    cudaLaunchConfig_t c{};
-    c.gridDim = dim3(blocks);
-    c.blockDim = dim3(threads);
-    c.dynamicSmemBytes = smem;
-    c.stream = st;
-    c.attrs = &at;
-    c.numAttrs = 1;
-    cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
-}
-
 // Lanes per row of the contact kernel: T = 2 (or 1, a tuning choice that suits large batches) for
 // candidate lists (a few entries per row); a whole warp per row for all pairs (n - 1 candidates per
 // row: the lanes share them, and the row count no longer bounds the warps a small system can use).
@@ -578,6 +555,12 @@ int launch_forces_compact_mixed(const Params &P, const StateView &S, const PairV
     // needs no second stream
     const bool fork_c = contacts && (hamaker || unary);
     if (!(ver && PV.near_len)) R.rec = nullptr;
+    // The kernels of one evaluation ask for one share of shared memory: otherwise those that use none (Hamaker pairs)
+    // and those that use some (contacts) cannot be on one SM together, and one stream's kernel waits for the
+    // other's to end. Single steps of 8000 listed particles took 40 us as soon as an SM held more than one
+    // contact block, and take 29 with one share for all; all pairs of 700 took 39 and take 23. (A share just large
+    // enough did not help everywhere: 42 with 64 KB for all pairs of 700.) The unary terms' kernel states no
+    // preference: with the others' share the restructuring batch takes 170 us a step instead of 145.
     // 100 KB hold the owners' blocks that the registers allow (44 KB) and seven blocks of the other contact kernel;
     // lists that would fill the SM with more of the latter get room for twelve
     const bool twelve = ver && !R.rec && P.n > (int64_t)7 * 152 * kCWarps * (32 / kContactLanes);

@@ -10,7 +10,8 @@
 // transformations (separation_ff), so the surface gap and the overlap keep FP32 relative precision
 // however small they are; velocities come as float-float copies (MixedExtra::v32); springs are
 // float-float pairs in 8-byte slots, one 9-component record per slot or bond (spring_at), updated
-// by FP32 increments (shear_ff). No pair costs an FP64 operation, except the FP64 overlap of a pair
+// by FP32 increments (shear_ff). A pair's two orders give values that are exactly equal or opposite, so a
+// kernel may evaluate either and use it for both. No pair costs an FP64 operation, except the FP64 overlap of a pair
 // at the contact threshold (overlap_fp64). Per-row sums are float-float (compensated) FP32
 // accumulations in an order fixed by the row alone.
 #pragma once
