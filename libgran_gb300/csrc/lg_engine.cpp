@@ -434,8 +434,8 @@ static int choose_kernel(const lg_system *s, int requested) {
     if (requested == LG_FORCE_KERNEL_PAIRS) return pairs_ok ? requested : -1;
     const int64_t n = s->P.n;
     // mixed precision: the compacted kernels at every size (their float-float completion and fused
-    // runs of steps also make small systems fastest: 19 particles 13.7 against 36.9 us a step, 1000
-    // particles 15.4 against 47.7 us, on GB300 with the row-group kernel)
+    // runs of steps also make small systems fastest: 64 particles 8.6 against 57.3 us a step, 1000
+    // particles 14.8 against 47.7 us, on GB300 with the row-group kernel)
     if (s->precision == LG_PRECISION_MIXED) return LG_FORCE_KERNEL_COMPACT;
     return (int64_t)s->pv[0].cap * n <= kPairsAutoSlots ? LG_FORCE_KERNEL_PAIRS : LG_FORCE_KERNEL_COMPACT;
 }
