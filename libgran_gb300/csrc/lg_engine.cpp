@@ -1348,17 +1348,23 @@ extern "C" int lg_destroy(lg_system *s) {
 // Run `period` steps as one CUDA graph (captured on first use for this pointer parity). The host
 // bookkeeping (buffer parities, step index) advances exactly as step_once advances it.
 static int run_period_graph(lg_system *s, double dt, int64_t period, int64_t rebuild_every) {
-    lg_system::GraphKey key{dt,      period,  s->kernel, s->T, s->vcur, s->pcur, s->fcur, s->ffcur, (int)(s->fstep & 1),
-                            s->contact_lanes};
+    const int64_t rebuild = s->P.pairs == LG_PAIRS_VERLET && rebuild_every > 0 ? rebuild_every : 0;
+    lg_system::GraphKey key{dt,      period,  rebuild, s->kernel, s->T, s->vcur, s->pcur, s->fcur, s->ffcur,
+                            (int)(s->fstep & 1), s->contact_lanes};
     for (auto &g : s->graphs) {
         if (!(g.key == key)) continue;
+        // the device builds the lists that the graph was captured with: the host must count the same ones
+        int builds = 0;
+        for (int64_t k = 0; rebuild && k < period; ++k) builds += (s->step_index + k) % rebuild == 0;
+        if ((builds & 1) != g.list_flips)
+            return lg_fail(LG_E_STATE, "lg_step: a captured period and its replay disagree about the list builds");
         LG_CUDA(cudaGraphLaunch(g.exec, s->stream));
         s->ffcur ^= g.ff_flips;
         s->fstep += g.f_launches;
         set_ff_buffers(s);
         // replay the host-side state transitions of `period` steps
         for (int64_t k = 0; k < period; ++k) {
-            if (s->P.pairs == LG_PAIRS_VERLET && rebuild_every > 0 && (s->step_index % rebuild_every) == 0) {
+            if (rebuild && (s->step_index % rebuild) == 0) {
                 s->pcur = 1 - s->pcur;
                 s->list_built = true;
             }
@@ -1370,7 +1376,7 @@ static int run_period_graph(lg_system *s, double dt, int64_t period, int64_t reb
         return LG_OK;
     }
     const int64_t l0 = s->launches;
-    const int ff0 = s->ffcur;
+    const int ff0 = s->ffcur, p0 = s->pcur;
     const int64_t fs0 = s->fstep;
     LG_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
     int rc = LG_OK;
@@ -1386,7 +1392,7 @@ static int run_period_graph(lg_system *s, double dt, int64_t period, int64_t reb
     ec = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
     if (ec != cudaSuccess) return lg_fail(LG_E_CUDA, "graph instantiation failed: %s", cudaGetErrorString(ec));
-    s->graphs.push_back({key, exec, s->launches - l0, s->ffcur ^ ff0, s->fstep - fs0});
+    s->graphs.push_back({key, exec, s->launches - l0, s->ffcur ^ ff0, s->fstep - fs0, s->pcur ^ p0});
     LG_CUDA(cudaGraphLaunch(exec, s->stream));
     return LG_OK;
 }

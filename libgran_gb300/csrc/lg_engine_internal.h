@@ -112,11 +112,12 @@ struct lg_system {
     // CUDA graphs of whole rebuild periods, keyed by the state that determines their pointers
     struct GraphKey {
         double dt;
-        int64_t period;
+        int64_t period, rebuild;  // rebuild: steps between list builds (0: none); period alone does not tell
         int kernel, T, vcur, pcur, fcur, ffcur, fpar, lanes;
         bool operator==(const GraphKey &o) const {
-            return dt == o.dt && period == o.period && kernel == o.kernel && T == o.T && vcur == o.vcur &&
-                   pcur == o.pcur && fcur == o.fcur && ffcur == o.ffcur && fpar == o.fpar && lanes == o.lanes;
+            return dt == o.dt && period == o.period && rebuild == o.rebuild && kernel == o.kernel && T == o.T &&
+                   vcur == o.vcur && pcur == o.pcur && fcur == o.fcur && ffcur == o.ffcur && fpar == o.fpar &&
+                   lanes == o.lanes;
         }
     };
     struct GraphEntry {
@@ -125,6 +126,7 @@ struct lg_system {
         int64_t launches;
         int ff_flips;        // float-float buffer swaps of the period (persistent steps)
         int64_t f_launches;  // persistent step launches of the period
+        int list_flips;      // parity of the period's list builds (each makes the other list the current one)
     };
     std::vector<GraphEntry> graphs;
     bool use_graphs = true;

@@ -1,0 +1,47 @@
+"""The Verlet list's two buffers (the current list, and the idle one that holds scratch between builds) over every
+way that a handle is stepped. The same operations run in each, so the tolerance is zero."""
+import numpy as np
+import pytest
+
+from libgran_gb300 import _abi as A
+from libgran_gb300 import configs as K
+from libgran_gb300.system import System, generate_aggregate, generate_velocities
+
+import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+PRECISIONS = pytest.mark.parametrize("precision", [A.LG_PRECISION_FP64, A.LG_PRECISION_MIXED], ids=["fp64", "mixed"])
+
+
+def _system(n, precision, pairs=A.LG_PAIRS_VERLET, bm=A.LG_BINARY_CONTACT):
+    mat = K.Material()
+    x0 = generate_aggregate(21, n, mat.r)
+    v0 = generate_velocities(21, n, 0.1) - 2e7 * (x0 - x0.mean(0))
+    d = K.make_desc(n, bm, A.LG_HAMAKER_LIMITED, contact=mat.contact(), sinter=mat.sinter(), hamaker=mat.hamaker(),
+                    pairs=pairs, r_verlet=4.5 * mat.r if pairs == A.LG_PAIRS_VERLET else 0.0, precision=precision,
+                    max_neighbors=96)
+    return System(d, x0, v0)
+
+
+@PRECISIONS
+@pytest.mark.parametrize("pairs,n", [(A.LG_PAIRS_VERLET, 300), (A.LG_PAIRS_VERLET, 900), (A.LG_PAIRS_ALL, 70)],
+                         ids=["verlet-300", "verlet-900", "all-70"])
+def test_steps_without_rebuilds_between_steps_with_them(pairs, n, precision):
+    """A run without rebuilds is captured sixteen steps at a time, and so is one that rebuilds every sixteen: the
+    two graphs differ in what they do to the lists."""
+    dt = K.Material().dt
+    schedule = [(48, 0), (48, 16), (48, 0), (1, 0), (47, 16), (32, 16), (5, 0), (32, 0)]
+    runs = []
+    for graphs in (True, False):
+        s = _system(n, precision, pairs)
+        s.set_graphs(graphs)
+        out = []
+        for nst, rb in schedule:
+            s.step(dt, nst, rb)
+            out += [s.get(f) for f in H.FIELDS]
+        assert s.device_errors() == 0
+        runs.append(out)
+        s.close()
+    for a, b in zip(*runs):
+        assert np.array_equal(a, b), H.rel_err(a, b)
