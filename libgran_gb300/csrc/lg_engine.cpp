@@ -272,6 +272,14 @@ static void to_dev4(const double *aos, int64_t n, std::vector<dbl4> &tmp) {
     for (int64_t i = 0; i < n; ++i) tmp[i] = make_double4_32a(aos[3 * i], aos[3 * i + 1], aos[3 * i + 2], 0.0);
 }
 
+// Host array to device memory, complete for the handle's stream on return. (cudaMemcpy from pageable memory may
+// return before the copy has reached the device, and kernels on a non-blocking stream do not wait for it.)
+static int upload(lg_system *s, void *dst, const void *src, size_t bytes) {
+    LG_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s->stream));
+    LG_CUDA(cudaStreamSynchronize(s->stream));
+    return LG_OK;
+}
+
 // Origin of one system's float-float positions (mixed precision): the centroid; out[3] receives
 // the largest coordinate offset from it (at least 8 particle radii), which bounds the FP32
 // rounding of the high parts.
@@ -1041,8 +1049,8 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
             }
             LG_TRY(s->alloc(&s->bv.cn, 15 * bs));
             LG_TRY(s->alloc(&s->bv.rev, bs));
-            LG_CUDA(cudaMemcpy(s->bv.cn, cn.data(), sizeof(double) * cn.size(), cudaMemcpyHostToDevice));
-            LG_CUDA(cudaMemcpy(s->bv.rev, rev.data(), sizeof(int32_t) * rev.size(), cudaMemcpyHostToDevice));
+            LG_TRY(upload(s, s->bv.cn, cn.data(), sizeof(double) * cn.size()));
+            LG_TRY(upload(s, s->bv.rev, rev.data(), sizeof(int32_t) * rev.size()));
         }
         s->host_bond_j = std::move(bj);
     }
@@ -1087,8 +1095,8 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
         LG_TRY(s->alloc(&s->d_sys_off, (size_t)ns + 1));
         LG_TRY(s->alloc(&s->d_centres, 3 * (size_t)ns));
         LG_TRY(s->alloc(&s->d_sys_obs, 20 * (size_t)ns));
-        LG_CUDA(cudaMemcpy(s->d_agg, agg.data(), sizeof(int32_t) * agg.size(), cudaMemcpyHostToDevice));
-        LG_CUDA(cudaMemcpy(s->d_sys_off, s->sys_off.data(), sizeof(int64_t) * s->sys_off.size(), cudaMemcpyHostToDevice));
+        LG_TRY(upload(s, s->d_agg, agg.data(), sizeof(int32_t) * agg.size()));
+        LG_TRY(upload(s, s->d_sys_off, s->sys_off.data(), sizeof(int64_t) * s->sys_off.size()));
     }
 
     // facets
@@ -1101,8 +1109,8 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
         std::vector<double> fvh(9 * (size_t)d->n_facets);
         for (int f = 0; f < d->n_facets; ++f)
             for (int q = 0; q < 9; ++q) fvh[9 * f + q] = facets[f].vertices[q];
-        LG_CUDA(cudaMemcpy(s->fv[0], fvh.data(), sizeof(double) * fvh.size(), cudaMemcpyHostToDevice));
-        LG_CUDA(cudaMemcpy(s->fv[1], fvh.data(), sizeof(double) * fvh.size(), cudaMemcpyHostToDevice));
+        LG_TRY(upload(s, s->fv[0], fvh.data(), sizeof(double) * fvh.size()));
+        LG_TRY(upload(s, s->fv[1], fvh.data(), sizeof(double) * fvh.size()));
     }
     s->fcur = 0;
 
@@ -1125,7 +1133,7 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
                 int64_t k = j < i ? j : j - 1;
                 fl[(size_t)(k * n + i)] = kBonded | ((uint32_t)b << 8);
             }
-        LG_CUDA(cudaMemcpy(pv.flags, fl.data(), sizeof(uint32_t) * fl.size(), cudaMemcpyHostToDevice));
+        LG_TRY(upload(s, pv.flags, fl.data(), sizeof(uint32_t) * fl.size()));
         s->pv[1] = pv;
         s->pcur = 0;
     } else {

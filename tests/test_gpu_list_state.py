@@ -45,3 +45,26 @@ def test_steps_without_rebuilds_between_steps_with_them(pairs, n, precision):
         s.close()
     for a, b in zip(*runs):
         assert np.array_equal(a, b), H.rel_err(a, b)
+
+
+@PRECISIONS
+@pytest.mark.parametrize("kind", ["batch-on-a-wall", "all-pairs-bonds"])
+def test_every_creation_sees_its_uploads(kind, precision):
+    """The construction's force evaluation runs on the handle's own stream, after the copies of the systems' offsets,
+    the facets' vertices and the pair flags."""
+    mat = K.Material()
+    wall = kind == "batch-on-a-wall"
+    sizes = np.array([40, 1, 300, 7] if wall else [120])
+    x0 = np.concatenate([generate_aggregate(31 + q, n, mat.r) for q, n in enumerate(sizes)])
+    if wall:
+        x0 = K.rest_on_wall(x0, sizes, mat.r)
+    d = K.make_desc(len(x0), A.LG_BINARY_SINTER, A.LG_HAMAKER_LIMITED, contact=mat.contact(), sinter=mat.sinter(),
+                    hamaker=mat.hamaker(), pairs=A.LG_PAIRS_VERLET if wall else A.LG_PAIRS_ALL,
+                    r_verlet=4.5 * mat.r if wall else 0.0, precision=precision, max_neighbors=96, n_facets=1 if wall else 0)
+    first = None
+    for _ in range(20):
+        s = System(d, x0, sizes=sizes if wall else None, facets=[K.wall_facet(mat, 200 * mat.r)] if wall else None)
+        a = s.get(A.LG_FIELD_A)
+        first = a if first is None else first
+        assert np.array_equal(a, first)
+        s.close()
