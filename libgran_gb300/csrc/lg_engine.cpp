@@ -503,9 +503,10 @@ static NearScratch near_scratch(const lg_system *s) {
     return R;
 }
 
-// The owned slots or contact candidates of the current list (after a build, and after a restore brings an
-// older list back).
+// The owned slots or contact candidates of the current list (after a build, after a restore brings an older
+// list back, and before the next evaluation when a serving slot was emptied between two builds).
 static void list_owners(lg_system *s) {
+    s->owners_stale = false;
     const NearScratch N = near_scratch(s);
     if (N.rec) {
         launch_near_owners(s->P.n, s->pv[s->pcur], N, s->stream);
@@ -1412,6 +1413,10 @@ extern "C" int lg_step(lg_system *s, double dt, int64_t nsteps, int64_t rebuild_
     const bool verlet = s->P.pairs == LG_PAIRS_VERLET;
     const int64_t period = (verlet && rebuild_every > 0) ? rebuild_every : 16;
     int64_t k = 0;
+    if (s->owners_stale && nsteps > 0) {  // (a first step that builds the list lists its owners too)
+        if (verlet && rebuild_every > 0 && (s->step_index % rebuild_every) == 0) s->owners_stale = false;
+        else list_owners(s);
+    }
     while (k < nsteps) {
         const bool aligned = !(verlet && rebuild_every > 0) || (s->step_index % rebuild_every) == 0;
         if (s->use_graphs && !s->timing && aligned && nsteps - k >= period && s->periods_run > 0 && period <= 4096) {
@@ -2209,6 +2214,7 @@ int lg_arena_import(lg_system *A, int64_t q, lg_system *S, const double *x0) {
         LG_CUDA(cudaMemcpyAsync(A->d_orig + q, &orig, d4, cudaMemcpyHostToDevice, st));
     }
     A->n_bonds_initial_sys[(size_t)q] = S->n_bonds_initial;
+    A->owners_stale = true;
     LG_CUDA(cudaGetLastError());
     LG_CUDA(cudaStreamSynchronize(st));  // host buffers above are released on return
     return LG_OK;
@@ -2233,6 +2239,7 @@ int lg_arena_clear(lg_system *A, int64_t q) {
         if (pv.near_len) LG_CUDA(cudaMemsetAsync(pv.near_len + off, 0, sizeof(int32_t) * C, st));
     }
     A->n_bonds_initial_sys[(size_t)q] = 0;
+    A->owners_stale = true;
     LG_CUDA(cudaGetLastError());
     LG_CUDA(cudaStreamSynchronize(st));
     return LG_OK;

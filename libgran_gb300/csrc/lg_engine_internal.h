@@ -77,6 +77,7 @@ struct lg_system {
     double *pres = nullptr;
     int32_t *d_queue_n = nullptr;  // length of the contact queue (zero between evaluations)
     int32_t *own_n = nullptr;   // Verlet: owned slots per block of rows
+    bool owners_stale = false;  // rows were emptied or replaced since the owned slots were listed
     unsigned *d_ticket = nullptr;  // zeroed counter of the reductions' last-block combine
     double *h_pin = nullptr;       // pinned host buffer (64 doubles) for small results read back
     uint8_t *d_hold = nullptr;  // [n] LG_HOLD_* bits (allocated on first use)

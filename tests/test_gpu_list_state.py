@@ -1,16 +1,21 @@
 """The Verlet list's two buffers (the current list, and the idle one that holds scratch between builds) over every
 way that a handle is stepped. The same operations run in each, so the tolerance is zero."""
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
 from libgran_gb300 import _abi as A
 from libgran_gb300 import configs as K
+from libgran_gb300.serving import Server
 from libgran_gb300.system import System, generate_aggregate, generate_velocities
 
 import helpers as H
 
 pytestmark = pytest.mark.gpu
 
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 PRECISIONS = pytest.mark.parametrize("precision", [A.LG_PRECISION_FP64, A.LG_PRECISION_MIXED], ids=["fp64", "mixed"])
 
 
@@ -68,3 +73,51 @@ def test_every_creation_sees_its_uploads(kind, precision):
         first = a if first is None else first
         assert np.array_equal(a, first)
         s.close()
+
+
+def _cpp(tmp_path, name, *args):
+    """Builds tests/cpp/<name>.cpp against the engine's library and its internal header, and runs it."""
+    so, cuda = A.lib()._name, os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    exe = tmp_path / name
+    subprocess.run([os.path.join(cuda, "bin", "nvcc"), "-O2", "-std=c++17", "-I" + os.path.join(ROOT, "libgran_gb300", "csrc"),
+                    os.path.join(ROOT, "tests", "cpp", name + ".cpp"), so, "-Xlinker", "-rpath=" + os.path.dirname(so),
+                    "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)] + list(args), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout[:2000] + r.stderr
+    return r.stdout.split()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_a_slot_emptied_between_builds_owns_no_pairs(tmp_path, precision):
+    b0, b1, a0, a1, same, errs = (int(v) for v in _cpp(tmp_path, "arena_owners", precision))
+    assert b0 > 0 and b0 == b1 and a0 == 0 and a1 == b1
+    assert same and errs == 0
+
+
+@PRECISIONS
+def test_served_budgets_that_end_between_builds(precision):
+    """Requests retire between two list builds; the others, and later occupants of their slots, end as lone runs do."""
+    mat = K.Material()
+    d = K.make_desc(1, A.LG_BINARY_CONTACT, A.LG_HAMAKER_LIMITED, contact=mat.contact(), hamaker=mat.hamaker(),
+                    pairs=A.LG_PAIRS_VERLET, r_verlet=4.5 * mat.r, precision=precision, max_neighbors=96)
+    srv = Server(d, budget_bytes=4 * 10 ** 9, dt=mat.dt, rebuild_every=20)
+    srv.set_slots([128, 256, 256])
+    jobs = [(100, 7), (200, 55), (250, 40), (90, 33), (180, 61), (256, 13)]
+    states = [(generate_aggregate(40 + q, n, mat.r), generate_velocities(40 + q, n, 0.1)) for q, (n, _) in enumerate(jobs)]
+    ids = [srv.submit(x, v, steps) for (x, v), (_, steps) in zip(states, jobs)]
+    for _ in range(200):
+        active, queued, _ = srv.tick()
+        if active == 0 and queued == 0:
+            break
+    for (n, steps), (x, v), q in zip(jobs, states, ids):
+        got = srv.poll(q, want_x=True)
+        d.n_part = n
+        d.force_kernel = A.LG_FORCE_KERNEL_COMPACT
+        s = System(d, x, v)
+        s.step(mat.dt, steps, 20)
+        want = s.get(A.LG_FIELD_X)
+        s.close()
+        if precision == A.LG_PRECISION_FP64:
+            assert np.array_equal(got["x"], want), (n, steps)
+        else:  # a run's float-float state is rounded to FP64 where the run ends, at another step than the lone run's
+            assert H.rel_err(got["x"] - x, want - x) <= 1e-5, (n, steps)
