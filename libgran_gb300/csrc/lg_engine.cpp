@@ -1174,8 +1174,19 @@ static int create_impl(const lg_system_desc *d, const double *x0, const double *
         s->pcur = 0;
         // cells: four per particle; a batch: eight per particle and 64 more per system
         s->max_cells = s->n_systems > 0 ? 8 * n + 64 * s->n_systems : std::max<int64_t>(64, 4 * n);
-        s->ls.nparts = 608;
-        LG_TRY(s->alloc(&s->ls.part, 6 * 608));
+        std::vector<ListPart> parts;  // a batch's systems, shared out in proportion to their particles
+        for (int64_t q = 0; q < s->n_systems; ++q) {
+            const int64_t nq = s->sys_off[q + 1] - s->sys_off[q], k = (nq + list_part_rows() - 1) / list_part_rows();
+            for (int64_t p = 0; p < k; ++p) parts.push_back({(int32_t)q, (int32_t)p, (int32_t)k});
+        }
+        s->ls.nparts = s->n_systems > 0 ? (int)parts.size() : 608;
+        LG_TRY(s->alloc(&s->ls.part, 6 * (size_t)s->ls.nparts));
+        if (s->n_systems > 0) {
+            LG_TRY(s->alloc(&s->ls.parts, parts.size()));
+            LG_TRY(upload(s, s->ls.parts, parts.data(), sizeof(ListPart) * parts.size()));
+            LG_TRY(s->alloc(&s->ls.tickets, (size_t)s->n_systems));
+            LG_CUDA(cudaMemsetAsync(s->ls.tickets, 0, sizeof(unsigned) * (size_t)s->n_systems, s->stream));
+        }
         LG_TRY(s->alloc(&s->ls.grid, (size_t)std::max<int64_t>(s->n_systems, 1)));
         LG_TRY(s->alloc(&s->ls.cell_of, (size_t)n));
         LG_TRY(s->alloc(&s->ls.count, (size_t)s->max_cells));

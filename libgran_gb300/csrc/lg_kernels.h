@@ -26,8 +26,13 @@ struct BatchView {
     const uint8_t *hold;   // [n] hold bits (null: none); inactive particles are left out of the list
 };
 
+// A share of one system of a batch: block `part` of the `parts` that work on system `sys`.
+struct ListPart {
+    int32_t sys, part, parts;
+};
+
 struct ListScratch {
-    int nparts;        // blocks of the bounding-box pass
+    int nparts;        // blocks of the bounding-box pass (a batch: all systems' parts)
     double *part;      // [nparts * 6]
     GridDev *grid;     // [1, or n_systems] device grid descriptions
     int32_t *cell_of;  // [n]
@@ -36,6 +41,8 @@ struct ListScratch {
     float4 *sorted;    // [n] cell by cell: position relative to the grid origin, and the index (bits of w)
     unsigned *ticket;  // finished blocks of the bounding-box pass (zero between builds)
     int32_t *cursor;   // places of the sorted list taken so far
+    ListPart *parts;   // batch: [nparts] the systems' parts, each system's one after another
+    unsigned *tickets; // batch: [n_systems] finished parts of the bounding-box pass (zero between builds)
     int32_t *cell_cursor;  // batch: cells taken so far (zero between builds)
     float4 *x32;       // [n] positions relative to the grid origin, FP32 (candidate filter)
     int32_t *max_row;  // [1] longest row found by the last build (before truncation)
@@ -73,6 +80,8 @@ void launch_kick_drift_fp64(int64_t n, dbl4 *x, dbl4 *v, dbl4 *th, dbl4 *w, cons
 // each particle, null for one system); kam = k_a / mass.
 void launch_body_central(int64_t n, const dbl4 *x, const int32_t *agg, const double *centre, double kam, dbl4 *ea,
                          dbl4 *eal, cudaStream_t st);
+// Particles of one part of a batch's system (ListPart).
+int64_t list_part_rows();
 // Rebuilds the Verlet rows into newv (springs carried from oldv). With r_near > 0 it also lists each
 // row's contact candidates (newv.near_*): slots within r_near or bonded; springs of the other slots
 // are not carried (those pairs are apart, so their springs reset).

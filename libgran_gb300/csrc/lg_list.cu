@@ -17,6 +17,10 @@ namespace lg {
 namespace {
 constexpr int kBoxThreads = 256;
 constexpr int kLineThreads = 256;
+// Batch: particles of a system per block of the passes over its grid, one per thread. (With one block per system
+// a build grew with the largest: systems of 32768 + 32768 monomers 225 us, 100,000 + 500 508; now 116 and 200, and
+// 114 and 200 for one system as large.)
+constexpr int kPartRows = 256;
 constexpr int kBuildRows = 32;    // rows per block of build_rows
 constexpr int kBuildLanes = 8;    // lanes per row
 constexpr int kBuildThreads = kBuildRows * kBuildLanes;
@@ -136,6 +140,29 @@ __device__ __forceinline__ int32_t grid_of(const Box &b, GridDev *g, double rv, 
     return (int32_t)(dim[0] * dim[1] * dim[2]);
 }
 
+// Leaves the block's box (in thread 0's b) at `at`; true in the block that is the last of `blocks` to do so.
+__device__ __forceinline__ bool last_of(const Box &b, Box *at, unsigned *ticket, unsigned blocks, bool *last) {
+    if (threadIdx.x == 0) {
+        *at = b;
+        __threadfence();
+        *last = atomicAdd(ticket, 1u) == blocks - 1;
+    }
+    __syncthreads();
+    if (!*last) return false;
+    __threadfence();
+    return true;
+}
+// The box over the boxes that `count` blocks left at `part`, in thread 0.
+__device__ __forceinline__ void combine_boxes(Box &b, const Box *part, int count, Box *s) {
+    b = empty_box();
+    for (int q = threadIdx.x; q < count; q += blockDim.x) {
+        const long long *p = reinterpret_cast<const long long *>(part + q);
+        const int64_t lo[3] = {__ldcg(p), __ldcg(p + 1), __ldcg(p + 2)}, hi[3] = {__ldcg(p + 3), __ldcg(p + 4), __ldcg(p + 5)};
+        box_add(b, lo, hi);
+    }
+    block_box(b, s);
+}
+
 // One system: bounding box of the positions, and in the last block to finish the grid. Also zeroes the
 // cell counts.
 __global__ void __launch_bounds__(kBoxThreads) box_grid(int64_t n, const dbl4 *__restrict__ x, ListScratch L, double rv,
@@ -148,21 +175,8 @@ __global__ void __launch_bounds__(kBoxThreads) box_grid(int64_t n, const dbl4 *_
     for (int64_t i = t; i < n; i += step) box_point(b, x[i]);
     block_box(b, s);
     Box *part = reinterpret_cast<Box *>(L.part);
-    if (threadIdx.x == 0) {
-        part[blockIdx.x] = b;
-        __threadfence();
-        last = atomicAdd(L.ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    b = empty_box();
-    for (int q = threadIdx.x; q < (int)gridDim.x; q += blockDim.x) {
-        const long long *p = reinterpret_cast<const long long *>(part + q);
-        const int64_t lo[3] = {__ldcg(p), __ldcg(p + 1), __ldcg(p + 2)}, hi[3] = {__ldcg(p + 3), __ldcg(p + 4), __ldcg(p + 5)};
-        box_add(b, lo, hi);
-    }
-    block_box(b, s);
+    if (!last_of(b, part + blockIdx.x, L.ticket, gridDim.x, &last)) return;
+    combine_boxes(b, part, (int)gridDim.x, s);
     if (threadIdx.x != 0) return;
     *L.ticket = 0u;
     *L.cursor = 0;
@@ -170,31 +184,36 @@ __global__ void __launch_bounds__(kBoxThreads) box_grid(int64_t n, const dbl4 *_
     grid_of(b, L.grid, rv, rnear, max_cells);
 }
 
-// A batch: one block per system, each with a grid of its own over its active particles (a common grid would
-// have to span the empty space between the systems). The systems' cells lie one after another, in any
-// order; a system of n_q particles gets at most 8 n_q + 64. Zeroes the cell counts too.
+// A batch: each system has a grid of its own over its active particles (a common grid would have to span the
+// empty space between the systems). A system of n_q particles has ceil(n_q / kPartRows) blocks; the last of them
+// to finish makes the grid. The systems' cells lie one after another, in any order; a system gets at most
+// 8 n_q + 64. Also zeroes the cell counts.
 __global__ void __launch_bounds__(kBoxThreads) box_grid_batch(const dbl4 *__restrict__ x, BatchView B, ListScratch L,
-                                                              double rv, double rnear) {
+                                                              double rv, double rnear, int64_t max_cells) {
     __shared__ Box s[kBoxThreads / 32];
-    __shared__ int32_t base, cells;
-    const int64_t q = blockIdx.x, b0 = B.off[q], b1 = B.off[q + 1];
+    __shared__ bool last;
+    const ListPart w = L.parts[blockIdx.x];
+    const int64_t q = w.sys, b0 = B.off[q], b1 = B.off[q + 1];
+    for (int64_t c = blockIdx.x * (int64_t)kBoxThreads + threadIdx.x; c < max_cells; c += (int64_t)gridDim.x * kBoxThreads)
+        L.count[c] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *L.cursor = 0;
     Box b = empty_box();
-    for (int64_t i = b0 + threadIdx.x; i < b1; i += blockDim.x)
+    for (int64_t i = b0 + (int64_t)w.part * kBoxThreads + threadIdx.x; i < b1; i += (int64_t)w.parts * kBoxThreads)
         if (!inactive_of(B.hold, i)) box_point(b, x[i]);
     block_box(b, s);
-    if (threadIdx.x == 0) {
-        cells = grid_of(b, L.grid + q, rv, rnear, 8 * (b1 - b0) + 64);
-        base = atomicAdd(L.cell_cursor, cells);
-        L.grid[q].base = base;
-        if (q == 0) *L.cursor = 0;
+    if (w.parts > 1) {
+        if (!last_of(b, reinterpret_cast<Box *>(L.part) + blockIdx.x, L.tickets + q, w.parts, &last)) return;
+        combine_boxes(b, reinterpret_cast<Box *>(L.part) + (blockIdx.x - w.part), w.parts, s);
     }
-    __syncthreads();
-    for (int32_t c = threadIdx.x; c < cells; c += blockDim.x) L.count[base + c] = 0;
+    if (threadIdx.x != 0) return;
+    if (w.parts > 1) L.tickets[q] = 0u;
+    const int32_t cells = grid_of(b, L.grid + q, rv, rnear, 8 * (b1 - b0) + 64);
+    L.grid[q].base = atomicAdd(L.cell_cursor, cells);
 }
 
 __device__ __forceinline__ int32_t cell_coord(float f, float inv_edge, int32_t dim) {
     const float u = f * inv_edge;
-    const int32_t k = u < 2.0e9f ? (int32_t)u : 2000000000;  // (NaN converts to 0)
+    const int32_t k = u < 2.0e9f ? (int32_t)u : 2000000000;  // (NaN: the last cell)
     return k < 0 ? 0 : (k >= dim ? dim - 1 : k);
 }
 
@@ -218,14 +237,15 @@ __global__ void cell_count(int64_t n, const dbl4 *__restrict__ x, BatchView B, L
 }
 
 // Begin of every cell in the sorted list. Only cells next to each other in x need to be next to each other
-// there (a row's candidates are nine runs of up to three), so the lines of cells along x take their places
-// in any order: one warp per line scans its counts and claims the line's length from a cursor. One system:
-// the grid's warps share its lines; a batch: block q has system q's.
+// there (a row's candidates are nine runs of cells along x), so the lines of cells along x take their places
+// in any order: one warp per line scans its counts and claims the line's length from a cursor. The blocks of
+// a system share its lines (one system: all blocks; a batch: those of its parts).
 __global__ void __launch_bounds__(kLineThreads) line_starts(ListScratch L, int32_t batch) {
-    const GridDev *g = L.grid + (batch ? blockIdx.x : 0);
+    const ListPart part = batch ? L.parts[blockIdx.x] : ListPart{0, (int32_t)blockIdx.x, (int32_t)gridDim.x};
+    const GridDev *g = L.grid + part.sys;
     const int32_t d0 = g->dim[0], lines = g->dim[1] * g->dim[2], base = g->base;
-    const int lane = threadIdx.x & 31, warps = (batch ? 1 : gridDim.x) * (kLineThreads / 32);
-    for (int32_t w = (batch ? 0 : blockIdx.x * (kLineThreads / 32)) + (threadIdx.x >> 5); w < lines; w += warps) {
+    const int lane = threadIdx.x & 31, warps = part.parts * (kLineThreads / 32);
+    for (int32_t w = part.part * (kLineThreads / 32) + (threadIdx.x >> 5); w < lines; w += warps) {
         const int32_t *count = L.count + base + (int64_t)w * d0;
         int32_t *start = L.start + base + (int64_t)w * d0;
         int32_t total = 0;
@@ -527,13 +547,15 @@ __global__ void __launch_bounds__(kBuildThreads) build_rows(int64_t n, const dbl
     }
 }
 
+int64_t list_part_rows() { return kPartRows; }
+
 void launch_list_build(int64_t n, const dbl4 *x, BatchView B, double rv, double r_near, int64_t max_cells,
                        ListScratch &ls, PairView oldv, PairView newv, BondView BV, int32_t *err, cudaStream_t st) {
     const int threads = 256;
     const unsigned blocks = (unsigned)((n + threads - 1) / threads);
     const double rn = newv.near_len ? r_near : 0.0;
     if (B.agg) {
-        box_grid_batch<<<(unsigned)B.n_systems, kBoxThreads, 0, st>>>(x, B, ls, rv, rn);
+        box_grid_batch<<<(unsigned)ls.nparts, kBoxThreads, 0, st>>>(x, B, ls, rv, rn, max_cells);
     } else {
         // enough blocks for the cell counts to zero, at most the partials' room
         const int64_t want = (std::max<int64_t>(n, max_cells / 4) + kBoxThreads - 1) / kBoxThreads;
@@ -541,7 +563,7 @@ void launch_list_build(int64_t n, const dbl4 *x, BatchView B, double rv, double 
     }
     cell_count<<<blocks, threads, 0, st>>>(n, x, B, ls);
     const int64_t lb = std::min<int64_t>(std::max<int64_t>(max_cells / 128, 1), 152 * 8);
-    line_starts<<<B.agg ? (unsigned)B.n_systems : (unsigned)lb, kLineThreads, 0, st>>>(ls, B.agg ? 1 : 0);
+    line_starts<<<B.agg ? (unsigned)ls.nparts : (unsigned)lb, kLineThreads, 0, st>>>(ls, B.agg ? 1 : 0);
     cell_scatter<<<blocks, threads, 0, st>>>(n, B, ls);
     const size_t smem = build_smem_bytes(newv.cap, BV.bcap);
     static thread_local int attr_device = -1;

@@ -2,6 +2,7 @@
 way that a handle is stepped. The same operations run in each, so the tolerance is zero."""
 import os
 import subprocess
+import time
 
 import numpy as np
 import pytest
@@ -121,3 +122,59 @@ def test_served_budgets_that_end_between_builds(precision):
             assert np.array_equal(got["x"], want), (n, steps)
         else:  # a run's float-float state is rounded to FP64 where the run ends, at another step than the lone run's
             assert H.rel_err(got["x"] - x, want - x) <= 1e-5, (n, steps)
+
+
+@PRECISIONS
+def test_lists_of_systems_shared_by_several_blocks(precision):
+    """A batch's systems take blocks by their sizes: around one block's share, and far beyond it."""
+    sizes = np.array([255, 256, 257, 1, 513, 9000])
+    mat = K.Material()
+    xs = [generate_aggregate(60 + q, n, mat.r) for q, n in enumerate(sizes)]
+
+    def system(x, batch):
+        d = K.make_desc(len(x), A.LG_BINARY_CONTACT, A.LG_HAMAKER_LIMITED, contact=mat.contact(), hamaker=mat.hamaker(),
+                        pairs=A.LG_PAIRS_VERLET, r_verlet=4.5 * mat.r, precision=precision, max_neighbors=96,
+                        force_kernel=A.LG_FORCE_KERNEL_COMPACT)
+        s = System(d, x, generate_velocities(3, len(x), 0.1) * 0.0, sizes=sizes if batch else None)
+        for _ in range(3):
+            s.update_neighbor_list()
+        s.step(mat.dt, 1, 0)
+        out, st = s.get(A.LG_FIELD_A), s.pair_stats()
+        assert s.device_errors() == 0
+        s.close()
+        return out, st["mean_row_length"] * len(x)
+
+    got, rows = system(np.concatenate(xs), True)
+    cut = np.concatenate([[0], np.cumsum(sizes)])
+    alone = [system(x, False) for x in xs]
+    assert rows == pytest.approx(sum(r for _, r in alone), rel=1e-12)
+    for q, (want, _) in enumerate(alone):
+        if precision == A.LG_PRECISION_FP64:
+            assert np.array_equal(got[cut[q]:cut[q + 1]], want), q
+        elif np.abs(want).max() > 0:  # sums are grouped by the launch's slicing, a function of the total size
+            assert H.rel_err(got[cut[q]:cut[q + 1]], want) <= 1e-6, q
+
+
+def test_a_large_system_of_a_batch_builds_its_list_as_fast_as_alone():
+    """The build's passes are shared out by particles: a batch that is nearly all one system takes about as long as
+    that system (1.1 times, measured; with one block per system it took 2.5 times as long)."""
+    mat = K.Material()
+    n = 100000
+    x = np.concatenate([generate_aggregate(5, n, mat.r), generate_aggregate(6, 500, mat.r)])
+
+    def build_time(x, sizes):
+        d = K.make_desc(len(x), A.LG_BINARY_CONTACT, A.LG_HAMAKER_LIMITED, contact=mat.contact(), hamaker=mat.hamaker(),
+                        pairs=A.LG_PAIRS_VERLET, r_verlet=4.5 * mat.r, precision=A.LG_PRECISION_MIXED)
+        s = System(d, x, sizes=sizes)
+        best = np.inf
+        for _ in range(6):
+            s.device_errors()
+            t0 = time.perf_counter()
+            for _ in range(20):
+                s.update_neighbor_list()
+            s.device_errors()
+            best = min(best, time.perf_counter() - t0)
+        s.close()
+        return best
+
+    assert build_time(x, [n, 500]) <= 1.6 * build_time(x[:n], None)
