@@ -46,22 +46,17 @@ constexpr uint32_t kNoPartner = 255u;  // the partner's row does not list the en
 #endif
 constexpr int kCWarps = 2;   // warps per block
 constexpr int kHThreads = 128;  // threads per block of the Hamaker kernel
-// Resident blocks per SM the contact kernel is compiled for (its register budget): beside the Hamaker
-// kernel (two streams) a tighter budget lets more of both kernels' warps share an SM; alone, the
-// looser one avoids spills: contacts alone on 32768 particles, 8 blocks, 30 against 36 us per step
-// with 12. All pairs take the looser one in either place (a warp per row: small launches).
-#ifndef LG_CONTACT_MIN_BLOCKS
-#define LG_CONTACT_MIN_BLOCKS 12
-#endif
-#ifndef LG_CONTACT_MIN_BLOCKS_ALONE
-#define LG_CONTACT_MIN_BLOCKS_ALONE 8
-#endif
+// Resident blocks per SM that forces_contacts_mixed is compiled for: 8 leave it the 128 registers that it needs.
+// With 12 (80 registers, for more warps of the Hamaker kernel beside it) it spilled, and was slower at every size
+// and list length measured beside that kernel (us a step, 8 / 12 blocks, list radius 4.5 r and 6 r: 1000 monomers
+// 13.7 / 16.2 and 16.6 / 20.9, 32768 26.3 / 30.0 and 38.2 / 46.0) as well as alone.
+constexpr int kCBlocks = 8;
 }  // namespace
 
 // Contact and bond pairs of rows row0 .. row0 + 32/T - 1 per warp (contact_rows), csum receives the
 // contact part of the row's accelerations.
-template <bool NEAR, int T, int MINB>
-__global__ void __launch_bounds__(kCWarps * 32, MINB)
+template <bool NEAR, int T>
+__global__ void __launch_bounds__(kCWarps * 32, kCBlocks)
     forces_contacts_mixed(Params P, StateView S, PairView PV, BondView BV, MixedExtra MX) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int kRows = 32 / T;
@@ -487,14 +482,11 @@ namespace {
 // row: the lanes share them, and the row count no longer bounds the warps a small system can use).
 template <bool NEAR, int T>
 void launch_contacts(const Params &P, const StateView &S, const PairView &PV, const BondView &BV, const MixedExtra &MX,
-                     cudaStream_t st, bool beside_hamaker, int share) {
+                     cudaStream_t st, int share) {
     const size_t smem = sizeof(ContactSmem) * kCWarps;
     const int64_t rows_per_block = (32 / T) * kCWarps;
     const unsigned blocks = (unsigned)((P.n + rows_per_block - 1) / rows_per_block);
-    if (NEAR && beside_hamaker)
-        launch_shared(share, forces_contacts_mixed<NEAR, T, LG_CONTACT_MIN_BLOCKS>, blocks, kCWarps * 32, smem, st, P, S, PV, BV, MX);
-    else
-        launch_shared(share, forces_contacts_mixed<NEAR, T, LG_CONTACT_MIN_BLOCKS_ALONE>, blocks, kCWarps * 32, smem, st, P, S, PV, BV, MX);
+    launch_shared(share, forces_contacts_mixed<NEAR, T>, blocks, kCWarps * 32, smem, st, P, S, PV, BV, MX);
 }
 
 template <bool VERLET, int L, int SL>
@@ -561,10 +553,9 @@ int launch_forces_compact_mixed(const Params &P, const StateView &S, const PairV
     // contact block, and take 29 with one share for all; all pairs of 700 took 39 and take 23. (A share just large
     // enough did not help everywhere: 42 with 64 KB for all pairs of 700.) The unary terms' kernel states no
     // preference: with the others' share the restructuring batch takes 170 us a step instead of 145.
-    // 100 KB hold the owners' blocks that the registers allow (44 KB) and seven blocks of the other contact kernel;
-    // lists that would fill the SM with more of the latter get room for twelve
-    const bool twelve = ver && !R.rec && P.n > (int64_t)7 * 152 * kCWarps * (32 / kContactLanes);
-    const int share = twelve ? 72 : 44;
+    // 100 KB hold every block of the contact kernels that the registers allow but one of the row-by-row kernel's
+    // eight. (72 % for the latter was 1 to 5 % slower than 44 from 24000 monomers on, and the same below.)
+    const int share = 44;
     if (fork_c || unary) cudaEventRecord(J.fork, st);
     if (unary) {
         cudaStreamWaitEvent(J.unary, J.fork, 0);
@@ -585,11 +576,11 @@ int launch_forces_compact_mixed(const Params &P, const StateView &S, const PairV
             else if (R.rb == 64) launch_shared(share, mixed_contacts<64>, nb, 64, 0, side, P, PV, BV, MC, R);
             else launch_shared(share, mixed_contacts<32>, nb, 32, 0, side, P, PV, BV, MC, R);
         } else if (ver && PV.near_len && contact_lanes == 1)
-            launch_contacts<true, 1>(P, S, PV, BV, MC, side, hamaker != 0, share);
+            launch_contacts<true, 1>(P, S, PV, BV, MC, side, share);
         else if (ver && PV.near_len)
-            launch_contacts<true, kContactLanes>(P, S, PV, BV, MC, side, hamaker != 0, share);
+            launch_contacts<true, kContactLanes>(P, S, PV, BV, MC, side, share);
         else
-            launch_contacts<false, 32>(P, S, PV, BV, MC, side, hamaker != 0, share);
+            launch_contacts<false, 32>(P, S, PV, BV, MC, side, share);
         if (fork_c) cudaEventRecord(J.join, side);
         ++kernels;
     }
