@@ -485,14 +485,26 @@ static PairScratch pair_scratch(const lg_system *s) {
 // Scratch of the mixed contact kernel that evaluates each pair once, in the idle list's spring buffer (9
 // doubles a slot: two float4 of records, an owner entry). Neck strengths looked up by the reference's
 // indexing differ between a pair's two orders, so a breaking bond may then break in one order only: such
-// systems take the kernel that evaluates each order. From 512 monomers on beside a Hamaker kernel, whose run
-// time covers the owners' pass and the completion's sums (us a step, once per pair against once per order: 500
-// monomers 14.5 / 15.3, 4000 15.8 / 17.1, 8000 17.0 / 19.0); alone from 49152 (8000: 16.0 / 13.8, 40000: 22.4 /
-// 21.8, 65000: 27.1 / 29.1).
+// systems take the kernel that evaluates each order.
+// It halves the pairs evaluated, but every candidate costs a record, which the completion adds row by row: it leads
+// where the candidates' radius r_near is hardly beyond contact, or where there are enough rows to hide the sums.
+// us a step, once per pair / once per order, by r_near over the contact distance (single aggregates, list radius
+// 4.1 r to 5 r; "alone": no Hamaker kernel beside it):
+//   1.05  520 monomers 12.3 / 13.1, 16000 15.3 / 16.5, 65536 31.6 / 37.4; alone 32768 15.4 / 16.6
+//   1.25  2000 15.4 / 13.7, 18000 19.1 / 18.5, 24000 20.7 / 21.4, 65536 38.8 / 41.3; alone 40000 20.4 / 19.0,
+//         49152 21.6 / 22.5
+//   1.5   16000 23.4 / 19.0, 65536 48.7 / 47.9, 300000 209.5 / 207.9, batch of 392000 211 / 235; alone 131072
+//         57.2 / 49.7, batch of 392000 137 / 159
+//   2     32768 46.1 / 38.2, 65536 87.8 / 72.5
 static NearScratch near_scratch(const lg_system *s) {
     NearScratch R{};
     if (!s->own_n || s->precision != LG_PRECISION_MIXED || !s->pv[0].near_len) return R;
-    if (s->P.n < (s->P.hamaker_model != LG_HAMAKER_NONE ? 512 : 49152)) return R;
+    const double reach = 2.0 * (s->P.binary_model == LG_BINARY_CONTACT ? s->P.contact.r_part
+                                                                        : std::max(s->P.contact.r_part, s->P.sinter.r_part));
+    const double q = s->r_near / reach;
+    const bool ham = s->P.hamaker_model != LG_HAMAKER_NONE;
+    const int64_t from = q <= 1.06 ? (ham ? 512 : 32768) : q <= 1.45 ? (ham ? 24000 : 49152) : q <= 1.55 ? 200000 : INT64_MAX;
+    if (s->P.n < from) return R;
     if (s->P.binary_model == LG_BINARY_BREAKING_SINTER && s->P.neck_mode == LG_NECK_REFERENCE_INDEXING) return R;
     double *base = s->pv[1 - s->pcur].xi;
     const int64_t slots = s->pv[0].cap * s->P.n;

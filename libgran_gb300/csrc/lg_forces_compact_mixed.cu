@@ -526,8 +526,10 @@ static int mixed_hamaker_slices_all_pairs(int64_t n) {
 
 // Rows per block of owned contact candidates (about 1.8 a row in an aggregate, somewhat more than half of
 // them touching): a block's candidates are about two per thread of 128, 64 or 32, and its touching pairs
-// one per thread.
-int32_t near_block_rows(int64_t n) { return n >= 32768 ? 128 : n >= 8192 ? 64 : 32; }
+// one per thread. us a step, 32 / 64 / 128 rows, list radius 4.5 r: 2000 monomers 15.2 / 15.5 / 16.1, 4000 15.3 / 15.5 /
+// 16.1, 4800 19.8 / 15.7 / 16.4, 8000 20.9 / 16.6 / 17.1, 16000 23.9 / 18.9 / 18.7, 32768 29.1 / 25.0 / 24.7. (From
+// 4800 on nearly every SM has a block of one warp beside its Hamaker block; why those then end late is not known.)
+int32_t near_block_rows(int64_t n) { return n >= 32768 ? 128 : n > 4096 ? 64 : 32; }
 
 void launch_near_owners(int64_t n, const PairView &PV, const NearScratch &R, cudaStream_t st) {
     const unsigned blocks = (unsigned)((n + R.rb - 1) / R.rb);

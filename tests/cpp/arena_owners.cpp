@@ -36,7 +36,7 @@ int main(int argc, char **argv) {
     d.binary_model = LG_BINARY_SINTER;
     d.hamaker_model = LG_HAMAKER_LIMITED;
     d.pairs = LG_PAIRS_VERLET;
-    d.r_verlet = 4.5 * r;
+    d.r_verlet = (mixed ? 4.1 : 4.5) * r;  // (mixed: candidates near contact, which are evaluated once per pair)
     d.max_neighbors = 96;
     d.contact = {1e4, 3e-9, 5e3, 2e-9, 1.0, 1.0, 5e3, 2e-9, 1.0, 1.0, 5e3, 2e-9, 1.0, 1.0, r, m, I, dt};
     d.sinter = {1e4, 3e-9, 5e3, 2e-9, 5e3, 2e-9, 5e3, 2e-9, r, m, I, dt, 1e-9};

@@ -178,3 +178,28 @@ def test_a_large_system_of_a_batch_builds_its_list_as_fast_as_alone():
         return best
 
     assert build_time(x, [n, 500]) <= 1.6 * build_time(x[:n], None)
+
+
+@pytest.mark.parametrize("bm", [A.LG_BINARY_CONTACT, A.LG_BINARY_SINTER], ids=["contact", "sinter"])
+@pytest.mark.parametrize("n", [511, 512, 4096, 4097, 23999, 24001, 32769])
+def test_contacts_evaluated_once_per_pair_equal_rows(n, bm):
+    """Candidates near contact are evaluated once per pair, in blocks of 32, 64 or 128 rows; the persistent kernel
+    evaluates each order by itself."""
+    mat = K.Material()
+    x0 = generate_aggregate(70, n, mat.r)
+    v0 = generate_velocities(70, n, 0.1) - 2e7 * (x0 - x0.mean(0))
+    runs = []
+    for kernel in (A.LG_FORCE_KERNEL_PERSISTENT, A.LG_FORCE_KERNEL_COMPACT):
+        for rv in (4.1, 4.5):
+            d = K.make_desc(n, bm, A.LG_HAMAKER_LIMITED, contact=mat.contact(), sinter=mat.sinter(), hamaker=mat.hamaker(),
+                            pairs=A.LG_PAIRS_VERLET, r_verlet=rv * mat.r, precision=A.LG_PRECISION_MIXED, max_neighbors=96,
+                            force_kernel=kernel)
+            s = System(d, x0, v0)
+            s.step(mat.dt, 1, 20)
+            s.step(mat.dt, 39, 20)
+            assert s.device_errors() == 0
+            runs.append([s.get(f) for f in H.FIELDS])
+            s.close()
+    for a, b in ((runs[0], runs[2]), (runs[1], runs[3])):
+        for u, v in zip(a, b):
+            assert np.array_equal(u, v), H.rel_err(u, v)

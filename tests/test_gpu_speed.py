@@ -1,0 +1,37 @@
+"""Costs that have to stay in proportion, as ratios of times taken on the same GPU one after another. The limits lie
+well above what is measured (stated beside each) and below what a wrong choice of kernel gave."""
+import pytest
+
+from libgran_gb300 import _abi as A
+from libgran_gb300 import configs as K
+from libgran_gb300.system import System, generate_aggregate, generate_velocities
+
+pytestmark = pytest.mark.gpu
+
+
+def _us(n, bm, hm, r_list=0.0, precision=A.LG_PRECISION_MIXED, steps=20):
+    """us a step of a run without list builds; r_list in radii (0: all pairs)"""
+    mat = K.Material()
+    d = K.make_desc(n, bm, hm, contact=mat.contact(), sinter=mat.sinter(), hamaker=mat.hamaker(),
+                    pairs=A.LG_PAIRS_VERLET if r_list else A.LG_PAIRS_ALL, r_verlet=r_list * mat.r, precision=precision)
+    s = System(d, generate_aggregate(5, n, mat.r), generate_velocities(5, n, 0.1))
+    for _ in range(3):
+        s.step(mat.dt, steps, 0)
+    t = min(s.step_timed(mat.dt, steps, 0) for _ in range(7)) * 1e3 / steps
+    s.close()
+    return t
+
+
+@pytest.mark.parametrize("n", [1000, 5000])
+def test_wide_lists_cost_what_their_candidates_cost(n):
+    """A list radius of 8 r holds five times the partners of one of 4.5 r, and ten times the contact candidates: 1.8 to
+    2.1 times the time (3.6 to 3.8 when every candidate's record was added in the completion)."""
+    near = _us(n, A.LG_BINARY_CONTACT, A.LG_HAMAKER_LIMITED, 4.5)
+    wide = _us(n, A.LG_BINARY_CONTACT, A.LG_HAMAKER_LIMITED, 8.0)
+    assert wide <= 2.8 * near
+
+
+def test_steps_do_not_jump_between_neighbouring_sizes():
+    """4800 monomers take 1.02 times as long a step as 4000 (1.3 times with contact blocks of one warp each)."""
+    small = _us(4000, A.LG_BINARY_CONTACT, A.LG_HAMAKER_LIMITED, 4.1)
+    assert _us(4900, A.LG_BINARY_CONTACT, A.LG_HAMAKER_LIMITED, 4.1) <= 1.15 * small
