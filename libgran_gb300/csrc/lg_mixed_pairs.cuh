@@ -416,8 +416,10 @@ __device__ __forceinline__ void contact_rows(const Params &P, const PairView &PV
 
     // entry of iteration it: partner and slot (-1: none). Candidate lists are loaded two iterations ahead, and
     // their entries' flags and partner positions one iteration ahead of the classification; with all pairs,
-    // where the partner follows from the slot, kDeep iterations of flags and positions are in flight.
-    constexpr int kDeep = NEAR ? 1 : 4;
+    // where the partner follows from the slot, kDeep iterations of flags and positions are in flight (contacts
+    // alone, us a step with 1 / 2 / 4: 256 monomers 11.6 / 11.4 / 12.0, 2048 36.7 / 35.9 / 47.6, 8192 776 / 736 / 860;
+    // four take more registers than there are).
+    constexpr int kDeep = NEAR ? 1 : 2;
     int32_t jn = -1, kn = 0;
     auto load_entry = [&](int64_t it) {
         const int64_t m = it * T + sub;
@@ -469,9 +471,13 @@ __device__ __forceinline__ void contact_rows(const Params &P, const PairView &PV
                     flc[d] = flc[d + 1];
                     pjc[d] = pjc[d + 1];
                 }
-                if (!NEAR) load_entry(it + kDeep);
-                take_entry(kDeep - 1);
-                if (NEAR) load_entry(it + 2);
+                if (NEAR) {
+                    take_entry(0);
+                    load_entry(it + 2);
+                } else if (it + kDeep < itmax) {
+                    load_entry(it + kDeep);
+                    take_entry(kDeep - 1);
+                }
                 bool cb = false;
                 if (j >= 0) {
                     const float dx = hi_i.x - pj.x, dy = hi_i.y - pj.y, dz = hi_i.z - pj.z;
