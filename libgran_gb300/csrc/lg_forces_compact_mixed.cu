@@ -359,6 +359,33 @@ __global__ void __launch_bounds__(kHThreads, L == 1 ? 6 : 7) forces_hamaker_mixe
     MX.hsum[2 * i + 1] = make_float4(acc[2].hi, acc[2].lo, 0.f, 0.f);
 }
 
+// All pairs of large systems: a lane per row and a warp per slice, so that the lanes of a warp read the same
+// partners (one broadcast a load; with lanes along a row every lane reads a sector of its own, and those loads
+// are what takes the time). The sums are added in the same order.
+template <int HM, int SL>
+__global__ void __launch_bounds__(32 * SL, 2) forces_hamaker_all(Params P, PairView PV, MixedExtra MX) {
+    __shared__ float part[SL][6][32];
+    const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
+    const int64_t row0 = (int64_t)blockIdx.x * 32, i = row0 + lane;
+    ff acc[3];
+    hamaker_rows<false, HM, HM == LG_HAMAKER_LIMITED>(P, PV, MX, row0, sl, SL, lane, acc);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        part[sl][2 * c][lane] = acc[c].hi;
+        part[sl][2 * c + 1][lane] = acc[c].lo;
+    }
+    __syncthreads();
+    if (sl != 0 || i >= P.n) return;
+    for (int q = 1; q < SL; ++q)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            ff_acc(acc[c], part[q][2 * c][lane]);
+            ff_acc(acc[c], part[q][2 * c + 1][lane]);
+        }
+    MX.hsum[2 * i] = make_float4(acc[0].hi, acc[0].lo, acc[1].hi, acc[1].lo);
+    MX.hsum[2 * i + 1] = make_float4(acc[2].hi, acc[2].lo, 0.f, 0.f);
+}
+
 // Unary terms (facets, body force) of every particle, beside the pair kernels: they need the FP64 state only,
 // and the FP64 pipe, which the pair kernels leave idle (in the completion they took 105 of its 119 us for
 // 141,000 particles on a wall). The grid holds no more than sixteen warps per SM, at 64 registers: the FP64
@@ -489,6 +516,15 @@ void launch_contacts(const Params &P, const StateView &S, const PairView &PV, co
     launch_shared(share, forces_contacts_mixed<NEAR, T>, blocks, kCWarps * 32, smem, st, P, S, PV, BV, MX);
 }
 
+template <int SL>
+void launch_hamaker_all(const Params &P, const PairView &PV, const MixedExtra &MX, cudaStream_t st, int share) {
+    const unsigned blocks = (unsigned)((P.n + 31) / 32);
+    auto k = P.hamaker_model == LG_HAMAKER_LIMITED      ? forces_hamaker_all<LG_HAMAKER_LIMITED, SL>
+             : P.hamaker_model == LG_HAMAKER_SIMPLIFIED ? forces_hamaker_all<LG_HAMAKER_SIMPLIFIED, SL>
+                                                        : forces_hamaker_all<LG_HAMAKER_FULL, SL>;
+    launch_shared(share, k, blocks, 32 * SL, 0, st, P, PV, MX);
+}
+
 template <bool VERLET, int L, int SL>
 void launch_hamaker(const Params &P, const PairView &PV, const MixedExtra &MX, cudaStream_t st, int share) {
     const unsigned blocks = (unsigned)((P.n * L + kHThreads - 1) / kHThreads);
@@ -513,6 +549,12 @@ int mixed_hamaker_slices(int64_t n) {
     if (groups * 2 <= two_waves) return 2;
     return 1;
 }
+
+// Monomers from which all pairs go to forces_hamaker_all. us a step, lanes along a row / lanes on rows, Hamaker pairs
+// only: limited form 1400 monomers 25.7 / 32.2, 2048 41.8 / 41.7, 2500 60.2 / 46.6, 4096 128 / 63, 8192 477 / 173;
+// full form 2048 42.0 / 45.2, 2500 61.1 / 54.4, 8192 475 / 315. (The kernel before these two, which queued the
+// pairs in range in shared memory, took 47, 81 and 275 for the limited form at 2048, 4096 and 8192.)
+constexpr int64_t kHamakerAllFrom = 2304;
 
 // All pairs: every row holds n - 1 partners, so small systems slice their rows further (up to 16
 // warps per 32-row group) under the same two-wave bound.
@@ -590,6 +632,7 @@ int launch_forces_compact_mixed(const Params &P, const StateView &S, const PairV
         switch (slices > 0 ? slices : ver ? mixed_hamaker_slices(P.n) : mixed_hamaker_slices_all_pairs(P.n)) {
             case 16:
                 if (ver) launch_hamaker<true, 16, 16>(P, PV, MX, st, share);
+                else if (P.n >= kHamakerAllFrom) launch_hamaker_all<16>(P, PV, MX, st, share);
                 else launch_hamaker<false, 32, 16>(P, PV, MX, st, share);
                 break;
             case 8:

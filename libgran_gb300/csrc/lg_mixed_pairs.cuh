@@ -333,8 +333,8 @@ __device__ __forceinline__ void window_partners(const PairView &PV, int64_t n, i
 
 // Sum of a window's Hamaker terms in slot order (FP32; the windows' sums are added with compensation).
 // Every slot is evaluated and the ones out of range are left out of the sum: without branches the four
-// evaluations overlap.
-template <int HM>
+// evaluations overlap. SPARSE: a window without a partner in range of any of the warp's rows is passed over.
+template <int HM, bool SPARSE = false>
 __device__ __forceinline__ f3 window_sum(const MixedExtra &MX, float4 xh, float4 xl, const int32_t (&j)[kWin]) {
     float4 ph[kWin], pl[kWin];
 #pragma unroll
@@ -348,13 +348,20 @@ __device__ __forceinline__ f3 window_sum(const MixedExtra &MX, float4 xh, float4
         }
     }
     f3 sum = fm(0.f, 0.f, 0.f);
+    bool in[kWin], any = false;
 #pragma unroll
     for (int u = 0; u < kWin; ++u) {
-        bool on = j[u] >= 0;
+        in[u] = j[u] >= 0;
         if (HM == LG_HAMAKER_LIMITED) {
             const float dx = xh.x - ph[u].x, dy = xh.y - ph[u].y, dz = xh.z - ph[u].z;
-            on = on && fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= MX.near2;
+            in[u] = in[u] && fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= MX.near2;
         }
+        any = any || in[u];
+    }
+    if (SPARSE && !__any_sync(__activemask(), any)) return sum;
+#pragma unroll
+    for (int u = 0; u < kWin; ++u) {
+        const bool on = in[u];
         const f3 a = hamaker_pair(HM, MX, xh, xl, ph[u], pl[u]);
         sum = fm(on ? __fadd_rn(sum.x, a.x) : sum.x, on ? __fadd_rn(sum.y, a.y) : sum.y,
                  on ? __fadd_rn(sum.z, a.z) : sum.z);
@@ -569,8 +576,8 @@ __device__ __forceinline__ void contact_rows(const Params &P, const PairView &PV
 }
 
 // Hamaker pairs of row row0 + lane, slice sl of kSlices: the windows sl, sl + kSlices, ... acch receives
-// the row's partial sum (float-float).
-template <bool VERLET>
+// the row's partial sum (float-float). HM: the Hamaker form (negative: from P), SPARSE: as window_sum.
+template <bool VERLET, int HM = -1, bool SPARSE = false>
 __device__ __forceinline__ void hamaker_rows(const Params &P, const PairView &PV, const MixedExtra &MX, int64_t row0,
                                              int sl, int kSlices, int lane, ff (&acch)[3]) {
     const int64_t n = P.n, i = row0 + lane;
@@ -581,7 +588,9 @@ __device__ __forceinline__ void hamaker_rows(const Params &P, const PairView &PV
     for (int32_t k0 = sl * kWin; k0 < len; k0 += kSlices * kWin) {
         int32_t j[kWin];
         window_partners<VERLET>(PV, n, i, len, k0, j);
-        const f3 w = window_sum(P.hamaker_model, MX, xh, xl, j);
+        f3 w;
+        if constexpr (HM >= 0) w = window_sum<HM, SPARSE>(MX, xh, xl, j);
+        else w = window_sum(P.hamaker_model, MX, xh, xl, j);
         ff_acc(acch[0], w.x);
         ff_acc(acch[1], w.y);
         ff_acc(acch[2], w.z);
