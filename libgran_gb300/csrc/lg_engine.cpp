@@ -496,6 +496,8 @@ static PairScratch pair_scratch(const lg_system *s) {
 //   1.5   16000 23.4 / 19.0, 65536 48.7 / 47.9, 300000 209.5 / 207.9, batch of 392000 211 / 235; alone 131072
 //         57.2 / 49.7, batch of 392000 137 / 159
 //   2     32768 46.1 / 38.2, 65536 87.8 / 72.5
+// With facets, whose terms run beside it, the second line lies at 8192 (monomers on a wall, 4000 32.3 / 31.8, 8000
+// 33.7 / 33.7, 12000 35.5 / 36.1, 16000 37.3 / 37.9, 20000 40.3 / 41.6, 24000 40.8 / 42.0).
 static NearScratch near_scratch(const lg_system *s) {
     NearScratch R{};
     if (!s->own_n || s->precision != LG_PRECISION_MIXED || !s->pv[0].near_len) return R;
@@ -503,7 +505,8 @@ static NearScratch near_scratch(const lg_system *s) {
                                                                         : std::max(s->P.contact.r_part, s->P.sinter.r_part));
     const double q = s->r_near / reach;
     const bool ham = s->P.hamaker_model != LG_HAMAKER_NONE;
-    const int64_t from = q <= 1.06 ? (ham ? 512 : 32768) : q <= 1.45 ? (ham ? 24000 : 49152) : q <= 1.55 ? 200000 : INT64_MAX;
+    const int64_t few = ham ? 512 : 32768, some = !ham ? 49152 : s->P.n_facets > 0 ? 8192 : 24000;
+    const int64_t from = q <= 1.06 ? few : q <= 1.45 ? some : q <= 1.55 ? 200000 : INT64_MAX;
     if (s->P.n < from) return R;
     if (s->P.binary_model == LG_BINARY_BREAKING_SINTER && s->P.neck_mode == LG_NECK_REFERENCE_INDEXING) return R;
     double *base = s->pv[1 - s->pcur].xi;

@@ -595,15 +595,20 @@ int launch_forces_compact_mixed(const Params &P, const StateView &S, const PairV
     // and those that use some (contacts) cannot be on one SM together, and one stream's kernel waits for the
     // other's to end. Single steps of 8000 listed particles took 40 us as soon as an SM held more than one
     // contact block, and take 29 with one share for all; all pairs of 700 took 39 and take 23. (A share just large
-    // enough did not help everywhere: 42 with 64 KB for all pairs of 700.) The unary terms' kernel states no
-    // preference: with the others' share the restructuring batch takes 170 us a step instead of 145.
-    // 100 KB hold every block of the contact kernels that the registers allow but one of the row-by-row kernel's
-    // eight. (72 % for the latter was 1 to 5 % slower than 44 from 24000 monomers on, and the same below.)
+    // enough did not help everywhere: 42 with 64 KB for all pairs of 700; 72 % was 1 to 5 % slower than 44 from
+    // 24000 listed monomers on.)
+    // The unary terms' kernel is the exception: it is launched first, states no share, and then the SM keeps what its
+    // blocks' own use comes to at full occupancy. What can join it there, from the kernels' start and end times: with
+    // 0.4 KB a block (its own) mixed_contacts and the Hamaker kernel, not the row-by-row contacts, which wait for it to
+    // end, and the Hamaker blocks behind them; with 2 to 6 KB more all of them; with 8 KB more, or with the others'
+    // share stated, none. us a step beside the row-by-row contacts, with 0 / 4 KB more: 9000 monomers on a wall 32.3 /
+    // 24.7, 4000 31.4 / 31.8, a body force on 9000 24.6 / 22.0, on 16000 25.2 / 23.9. (Beside mixed_contacts: 9000 25.3 /
+    // 25.5, 16000 37.3 / 37.6, the restructuring batch 134.6 / 135.3; with the share stated that took 156.)
     const int share = 44;
     if (fork_c || unary) cudaEventRecord(J.fork, st);
     if (unary) {
         cudaStreamWaitEvent(J.unary, J.fork, 0);
-        unary_mixed<<<std::min(blocks, (unsigned)kUnaryBlocks), kUnaryThreads, 0, J.unary>>>(P, S, MX);
+        unary_mixed<<<std::min(blocks, (unsigned)kUnaryBlocks), kUnaryThreads, contacts && !R.rec ? 4096 : 0, J.unary>>>(P, S, MX);
         cudaEventRecord(J.unary_join, J.unary);
         ++kernels;
     }
