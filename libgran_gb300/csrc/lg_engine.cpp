@@ -2111,7 +2111,7 @@ int lg_create_staged(const lg_system_desc *desc, const double *x0, const double 
     lg_system *s = new (std::nothrow) lg_system();
     if (!s) return lg_fail(LG_E_NOMEM, "lg_create_staged: host allocation failed");
     s->pooled = true;
-    s->slab_chunk = (size_t)std::max<int64_t>(lg_estimate_device_bytes(desc, desc->n_part), 0);
+    s->slab_chunk = (size_t)lg_handle_bytes(desc, std::max<int64_t>(desc->n_part, 1));
     static std::mutex pool_mu;
     static std::vector<int> pool_set;  // devices whose default pool keeps freed memory for reuse
     {

@@ -171,6 +171,9 @@ struct lg_system {
 
 int lg_fail(int code, const char *fmt, ...);
 
+// Device memory of a standalone handle's buffers (lg_server.cpp).
+int64_t lg_handle_bytes(const lg_system_desc *d, int64_t n);
+
 // Serving slots (lg_engine.cpp), for the serving loop. An arena is a batch handle whose systems
 // are slots of fixed capacities (caps) on a lattice; a slot holds one request (its first n
 // particles) or nothing, and its other particles are inactive (no cell, no row, no motion). All

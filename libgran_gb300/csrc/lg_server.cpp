@@ -90,24 +90,27 @@ struct lg_server {
     int64_t periods = 0;
 };
 
+// Device memory of a standalone handle of n particles, allocation by allocation (create_impl in lg_engine.cpp).
+int64_t lg_handle_bytes(const lg_system_desc *d, int64_t n) {
+    const bool verlet = d->pairs == LG_PAIRS_VERLET, mixed = d->precision == LG_PRECISION_MIXED;
+    const int64_t others = std::max<int64_t>(n - 1, 1);
+    const int64_t cap = verlet ? std::min<int64_t>(d->max_neighbors > 0 ? d->max_neighbors : 64, others) : others;
+    const int64_t nbuf = verlet ? 2 : 1;
+    int64_t b = 8 * 32 * n;                                                    // x, th, v[2], w[2], a, al
+    if (mixed) b += 320 * n;                                                   // float-float state (two x32, v32; s32) and sums
+    b += nbuf * cap * n * (4 + 4 + 72 + (mixed ? 5 : 0)) + nbuf * 8 * n;       // nbr, flags, springs, near lists, row lengths
+    b += 8 * n * (4 + 1 + 8 + 72);                                             // bonds (up to 8 per particle)
+    b += 72 * std::max(d->n_facets, 1) * n;                                    // facet springs
+    if (verlet) b += (4 + 4 * 8 + 16 + 16 + 1) * n;                            // cells, sorted and grid positions, owners
+    b += 20 * 8 * n;                                                           // observables scratch
+    if (mixed && (d->n_facets > 0 || d->body.model != LG_BODY_NONE || d->unary_hook)) b += 2 * 32 * n;  // unary terms
+    if (!mixed && !verlet) b += 72 * cap * n;                                  // pair kernels' records and queue
+    return b + (64 << 10);                                                     // small buffers, rounding
+}
+
 extern "C" int64_t lg_estimate_device_bytes(const lg_system_desc *d, int64_t n) {
     if (!d || n < 1) return -1;
-    const int64_t cap = d->pairs == LG_PAIRS_VERLET ? (d->max_neighbors > 0 ? d->max_neighbors : 64) : std::max<int64_t>(n - 1, 1);
-    const int64_t nbuf = d->pairs == LG_PAIRS_VERLET ? 2 : 1;
-    int64_t b = 10 * 32 * n;                                  // x, th, v[2], w[2], a, al (+ slack)
-    b += 320 * n;                                             // float-float state (two x32, v32; s32) and partial sums
-    b += nbuf * cap * n * (4 + 4 + 72 + 5) + nbuf * 8 * n;   // nbr, flags, springs, near lists, row lengths
-    b += 8 * n * (1 + 1 + 8 + 72);                            // bonds (up to 8 per particle)
-    b += 72 * std::max(d->n_facets, 1) * n;                   // facet springs
-    b += 4 * 8 * n + 4 * 4 * n;                               // list scratch
-    b += 20 * 8 * n;                                          // observables scratch
-    if (d->precision == LG_PRECISION_MIXED && (d->n_facets > 0 || d->body.model != LG_BODY_NONE || d->unary_hook))
-        b += 2 * 32 * n;                                      // unary terms
-    if (d->precision == LG_PRECISION_FP64 && d->pairs == LG_PAIRS_ALL)
-        b += 72 * cap * n;                                    // pair kernels' records and queue
-    else if (d->precision == LG_PRECISION_FP64 && cap * n <= ((int64_t)1 << 21))
-        b += 48 * cap * n;                                    // headroom of small FP64 systems
-    return b + (4 << 20);                                     // fixed overhead
+    return lg_handle_bytes(d, n) + (4 << 20);  // and what the handle takes outside its buffers
 }
 
 static int64_t slots_bytes(const lg_server *s, const std::vector<int64_t> &caps) {
@@ -115,7 +118,11 @@ static int64_t slots_bytes(const lg_server *s, const std::vector<int64_t> &caps)
     for (int64_t c : caps) n += c;
     lg_system_desc d = s->tmpl;
     if (d.max_neighbors <= 0) d.max_neighbors = 96;
-    return lg_estimate_device_bytes(&d, std::max<int64_t>(n, 1));
+    int64_t b = lg_estimate_device_bytes(&d, std::max<int64_t>(n, 1));
+    // slots hold up to 16 bonds per particle, and cells by the system (FP64 only: mixed slots have always been
+    // charged without these 4 per cent, and a budget that fits them goes on fitting them)
+    if (d.precision == LG_PRECISION_FP64) b += n * (8 * 85 + 48) + (int64_t)caps.size() * 1024;
+    return b;
 }
 
 // Default slots that fit half the budget (the rest for standalone handles): 8 slots per size class,

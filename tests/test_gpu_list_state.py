@@ -203,3 +203,14 @@ def test_contacts_evaluated_once_per_pair_equal_rows(n, bm):
     for a, b in ((runs[0], runs[2]), (runs[1], runs[3])):
         for u, v in zip(a, b):
             assert np.array_equal(u, v), H.rel_err(u, v)
+
+
+def test_staged_handles_take_what_they_need(tmp_path):
+    """One chunk from the pool that holds every buffer of the handle (a monomer's bonds: 8 reckoned, 1 to 7 used) and
+    nothing else of note; the server charges it and a fixed 4 MiB."""
+    rows = np.array([int(v) for v in _cpp(tmp_path, "staged_bytes")]).reshape(-1, 7)
+    assert len(rows) == 24
+    for precision, model, n, chunk, used, chunks, charged in rows:
+        assert chunks == 1, (precision, model, n)
+        assert chunk - used <= 64 * 1024 + 0.05 * chunk, (precision, model, n, chunk, used)
+        assert chunk <= charged <= chunk + 2 ** 22
