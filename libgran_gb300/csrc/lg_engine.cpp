@@ -92,17 +92,42 @@ int lg_detect_bonds(const double *x0, int64_t n, double r, double dc, bool cycle
     std::vector<std::pair<int32_t, int32_t>> cand;
     bool finite = std::isfinite(reach);
     for (int64_t q = 0; q < 3 * n; ++q) finite = finite && std::isfinite(x0[q]);
-    // up to 8192 particles a sweep along x, as a bonded pair is no further apart than the reach (one x86 core, ms:
-    // 1000 particles 1.7 by the double loop, 0.43 so; by the hashed grid 5000 7.4 and 4.7, 8192 12.1 and 9.1,
-    // and the sweep's window goes on growing)
-    if (n <= 8192 && finite) {
-        const double far = reach > 0 ? reach * (1.0 + 1e-9) : 0.0, far2 = far * far;
-        std::vector<int32_t> order((size_t)n);
+    // up to 8192 particles a sweep along the widest axis, as a bonded pair is no further apart than the reach (one x86
+    // core, ms: an aggregate of 1000 1.2 by the double loop, 0.4 so; by the hashed grid 5000 5.3 and 3.5, 8192 9.4 and
+    // 8.8, and the sweep's window goes on growing). A comparison costs 3 ns and the grid 1.1 us a particle, so above
+    // 2048 particles, where the double loop ends, a sweep of more than 400 comparisons a particle (compact clusters)
+    // goes to the grid.
+    std::vector<int32_t> order;
+    const double far = reach > 0 ? reach * (1.0 + 1e-9) : 0.0, far2 = far * far;
+    int axis = 0;
+    bool sweep = n <= 8192 && finite;
+    if (sweep) {
+        double lo[3], hi[3];
+        for (int c = 0; c < 3; ++c) lo[c] = hi[c] = x0[c];
+        for (int64_t i = 0; i < n; ++i)
+            for (int c = 0; c < 3; ++c) {
+                lo[c] = std::min(lo[c], x0[3 * i + c]);
+                hi[c] = std::max(hi[c], x0[3 * i + c]);
+            }
+        for (int c = 1; c < 3; ++c)
+            if (hi[c] - lo[c] > hi[axis] - lo[axis]) axis = c;
+        order.resize((size_t)n);
         for (int64_t i = 0; i < n; ++i) order[(size_t)i] = (int32_t)i;
-        std::sort(order.begin(), order.end(), [x0](int32_t a, int32_t b) { return x0[3 * a] < x0[3 * b]; });
-        std::vector<double> p(3 * (size_t)n);
+        const double *xa = x0 + axis;
+        std::sort(order.begin(), order.end(), [xa](int32_t a, int32_t b) { return xa[3 * a] < xa[3 * b]; });
+        if (n > 2048 && reach > 0) {
+            int64_t total = 0, b = 0;
+            for (int64_t a = 0; a < n; ++a) {
+                while (b < n && !(xa[3 * order[(size_t)b]] - xa[3 * order[(size_t)a]] > far)) ++b;
+                total += b - a - 1;
+            }
+            sweep = total <= 400 * n;
+        }
+    }
+    if (sweep) {
+        std::vector<double> p(3 * (size_t)n);  // the sweep's axis first
         for (int64_t q = 0; q < n; ++q)
-            for (int c = 0; c < 3; ++c) p[3 * q + c] = x0[3 * (int64_t)order[(size_t)q] + c];
+            for (int c = 0; c < 3; ++c) p[3 * q + c] = x0[3 * (int64_t)order[(size_t)q] + (axis + c) % 3];
         for (int64_t a = 0; a + 1 < n; ++a)
             for (int64_t b = a + 1; b < n && !(p[3 * b] - p[3 * a] > far); ++b) {
                 const double dx = p[3 * b] - p[3 * a], dy = p[3 * b + 1] - p[3 * a + 1], dz = p[3 * b + 2] - p[3 * a + 2];
