@@ -214,3 +214,29 @@ def test_staged_handles_take_what_they_need(tmp_path):
         assert chunks == 1, (precision, model, n)
         assert chunk - used <= 64 * 1024 + 0.05 * chunk, (precision, model, n, chunk, used)
         assert chunk <= charged <= chunk + 2 ** 22
+
+
+@pytest.mark.parametrize("n,wall", [(3599, False), (3601, False), (8500, False), (8501, False), (22999, False),
+                                    (30001, False), (8999, True), (9001, True)], ids=str)
+def test_fp64_pair_kernels_equal_rows_at_their_launch_lines(n, wall):
+    """The row kernel at one thread per row adds each row in index order, and so do the pair kernels, whatever their block
+    shapes: the same bits."""
+    mat = K.Material()
+    x0 = generate_aggregate(90, n, mat.r)
+    v0 = generate_velocities(90, n, 0.1) - 2e7 * (x0 - x0.mean(0))
+    if wall:
+        x0 = K.rest_on_wall(x0, np.array([n]), mat.r)
+    runs = []
+    for kernel in (A.LG_FORCE_KERNEL_ROWGROUP, A.LG_FORCE_KERNEL_AUTO):
+        d = K.make_desc(n, A.LG_BINARY_CONTACT, A.LG_HAMAKER_LIMITED, contact=mat.contact(), hamaker=mat.hamaker(),
+                        pairs=A.LG_PAIRS_VERLET, r_verlet=4.5 * mat.r, max_neighbors=96, force_kernel=kernel,
+                        threads_per_row=1 if kernel == A.LG_FORCE_KERNEL_ROWGROUP else 0, n_facets=1 if wall else 0,
+                        facet_auto_move=1 if wall else 0)
+        s = System(d, x0, v0, facets=[K.wall_facet(mat, 200 * mat.r, 1.0)] if wall else None)
+        s.step(mat.dt, 1, 5)
+        s.step(mat.dt, 11, 5)
+        assert s.device_errors() == 0
+        runs.append([s.get(f) for f in H.FIELDS])
+        s.close()
+    for a, b in zip(*runs):
+        assert np.array_equal(a, b), H.rel_err(a, b)
