@@ -2607,6 +2607,7 @@ extern "C" int lg_autotune(lg_system *s, double dt, int64_t probe_steps, int64_t
     lg_tuning pick = keep;
     for (auto &c : cands) {
         int rc = apply_tuning(s, c);
+        s->drop_graphs();  // (the persistent kernel's shapes are not in the graphs' key)
         float ms = 0.f, ms2 = 0.f;
         if (rc == LG_OK) rc = lg_step(s, dt, probe_steps, rebuild_every);  // warm-up (and graph capture)
         if (rc == LG_OK) rc = snapshot_restore(s);
@@ -2616,11 +2617,13 @@ extern "C" int lg_autotune(lg_system *s, double dt, int64_t probe_steps, int64_t
         const int rc2 = snapshot_restore(s);
         if (rc != LG_OK || rc2 != LG_OK) {
             apply_tuning(s, keep);
+            s->drop_graphs();
             return rc != LG_OK ? rc : rc2;
         }
         const double t = std::min(ms, ms2) / (double)probe_steps;
         if (!(t > 0.0)) {  // an event pair that measured nothing cannot rank a candidate
             apply_tuning(s, keep);
+            s->drop_graphs();
             return lg_fail(LG_E_CUDA, "lg_autotune: a candidate timed %g ms", t);
         }
         if (t < best) {
@@ -2631,6 +2634,7 @@ extern "C" int lg_autotune(lg_system *s, double dt, int64_t probe_steps, int64_t
     }
     LG_CUDA(cudaStreamSynchronize(s->stream));
     s->launches = keep_launch;
+    s->drop_graphs();
     LG_TRY(apply_tuning(s, pick));
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);

@@ -240,3 +240,8 @@ def test_fp64_pair_kernels_equal_rows_at_their_launch_lines(n, wall):
         s.close()
     for a, b in zip(*runs):
         assert np.array_equal(a, b), H.rel_err(a, b)
+
+
+def test_tuned_handles_hold_no_graph_of_another_shape(tmp_path):
+    held, eager, replayed = (int(v) for v in _cpp(tmp_path, "tuned_graphs"))
+    assert held == 0 and eager == replayed
