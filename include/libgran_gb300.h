@@ -204,7 +204,7 @@ typedef struct lg_system_desc {
 #define LG_FORCE_KERNEL_COMPACT 2    /* mixed: one row per lane, warp-compacted pair queues; FP64: the pair
                                        kernels (every unordered pair once, queued contacts, then an ordered
                                        per-row fold in the reference's summation order) */
-#define LG_FORCE_KERNEL_PAIRS 3      /* FP64: the pair kernels, for systems of at most 2^21 pair slots */
+#define LG_FORCE_KERNEL_PAIRS 3      /* FP64: the pair kernels too, refused above 2^21 pair slots */
 #define LG_FORCE_KERNEL_PERSISTENT 4 /* mixed: every step inside a run of steps (no facets, body terms or
                                        held particles) is one persistent launch whose warps pull contact
                                        and Hamaker work items of 32-row groups from a device queue and

@@ -261,21 +261,15 @@ __device__ __forceinline__ d3 dvs_t(d3 a, double s) {
     }
     return dvs(a, s);
 }
-template <bool FAST>
-__device__ __forceinline__ d3 nrmz_t(d3 a) {
-    const double z = sqn(a);
-    return z > 0.0 ? dvs_t<FAST>(a, droot(z)) : a;
-}
 
 // contact_force.h:105-147
-template <bool FAST = false>
 __device__ __forceinline__ d3 shear_coulomb(d3 &xi, d3 n, double stiffness, double damping, double normal_force,
                                             double mu_static, double phi_dynamic, d3 rel, double dt) {
     double mu_dynamic = mu_static * phi_dynamic;
     d3 xi_new = sub(xi, scl(dot(xi, n), n));
     const double z = sqn(xi_new);
     if (z > 0.0) {  // (so is its root)
-        xi_new = dvs_t<FAST>(xi_new, droot(z));
+        xi_new = dvs(xi_new, droot(z));
         xi_new = scl(nrm(xi), xi_new);
     }
     xi = xi_new;
@@ -283,7 +277,7 @@ __device__ __forceinline__ d3 shear_coulomb(d3 &xi, d3 n, double stiffness, doub
     double static_friction = mu_static * normal_force;
     double dynamic_friction = mu_dynamic * normal_force;
     double f0n = nrm(f0);
-    d3 t = (f0n > 0.0) ? dvs_t<FAST>(f0, f0n) : zero3();
+    d3 t = (f0n > 0.0) ? dvs(f0, f0n) : zero3();
     double f_selected;
     if (f0n <= static_friction) {
         xi = add(xi, scl(dt, rel));

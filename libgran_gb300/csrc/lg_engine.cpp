@@ -453,9 +453,10 @@ int lg_system::alloc(U **p, size_t count) {
     return LG_OK;
 }
 
-// Pair slots up to which LG_FORCE_KERNEL_PAIRS may be asked for, and up to which the automatic choice
-// reports it. In FP64 it and LG_FORCE_KERNEL_COMPACT name the same pair kernels (lg_forces_pairs.cu),
-// whose block shape follows the size; both lead the row-group kernel at every size measured.
+// In FP64 LG_FORCE_KERNEL_PAIRS and LG_FORCE_KERNEL_COMPACT name the same pair kernels (lg_forces_pairs.cu), whose
+// block shapes follow the size; they lead the row-group kernel at every size measured. Both names, the number of
+// pair slots up to which PAIRS may be asked for and the one up to which the automatic choice reports it are kept for
+// callers and saved tuning records that know them.
 constexpr int64_t kPairsMaxSlots = (int64_t)1 << 21;
 constexpr int64_t kPairsAutoSlots = (int64_t)1 << 19;
 
@@ -873,8 +874,9 @@ static int64_t above_bound(double b) {
 }
 
 // A serving arena (lg_arena_create): a batch whose systems are slots that start empty -- every
-// particle inactive, no bonds -- on a lattice of the given spacing, with bond capacity bcap per
-// particle and float-float extents allowed up to ext.
+// particle inactive, no bonds -- with bond capacity bcap per particle and float-float extents allowed up to ext;
+// `lattice` is twice the radius that an occupant may have, and the list radius on either side (which keeps it within
+// ext), and the spacing at which the empty slots' particles are parked.
 struct ArenaSpec {
     int32_t bcap;
     double lattice, ext;
@@ -2185,6 +2187,7 @@ int lg_arena_import(lg_system *A, int64_t q, lg_system *S, const double *x0) {
         for (int k = 0; k < 3; ++k) r2 += (x0[3 * i + k] - c[k]) * (x0[3 * i + k] - c[k]);
         rad = std::max(rad, std::sqrt(r2));
     }
+    // the FP32 culling radii of all slots allow for an occupant of this radius (ArenaSpec::ext)
     if (rad > 0.5 * A->arena_lattice - A->P.r_verlet)
         return lg_fail(LG_E_INVALID, "lg_arena_import: the aggregate (radius %g) is too wide for the slot lattice (%g)", rad,
                        A->arena_lattice);
@@ -2389,7 +2392,9 @@ static int apply_tuning(lg_system *s, const lg_tuning &t) {
     s->step_min_blocks = t.step_min_blocks;
     s->step_slices = t.step_slices;
     s->step_assign = t.step_assign;
-    if (t.force_kernel == LG_FORCE_KERNEL_PAIRS && choose_kernel(s, LG_FORCE_KERNEL_PAIRS) < 0) return lg_fail(LG_E_INVALID, "tuning: no pair-parallel scratch");
+    if (t.force_kernel == LG_FORCE_KERNEL_PAIRS && choose_kernel(s, LG_FORCE_KERNEL_PAIRS) < 0)
+        return lg_fail(LG_E_INVALID, "tuning: the pair-parallel kernel is FP64 only and takes at most %lld pair slots",
+                       (long long)kPairsMaxSlots);
     s->kernel = t.force_kernel;
     if (compact_mixed(s, t.force_kernel))
         s->contact_lanes = t.threads_per_row == 1 ? 1 : 2;
@@ -2595,9 +2600,8 @@ extern "C" int lg_autotune(lg_system *s, double dt, int64_t probe_steps, int64_t
         cands.push_back(t);
     };
     const int sl0 = mixed_hamaker_slices(s->P.n);
-    add(LG_FORCE_KERNEL_COMPACT, s->precision == LG_PRECISION_MIXED ? 2 : 1, 4, sl0, 0);
+    add(choose_kernel(s, LG_FORCE_KERNEL_AUTO), s->precision == LG_PRECISION_MIXED ? 2 : 1, 4, sl0, 0);
     if (s->precision == LG_PRECISION_MIXED) add(LG_FORCE_KERNEL_COMPACT, 1, 4, sl0, 0);  // one contact lane per row
-    if (choose_kernel(s, LG_FORCE_KERNEL_PAIRS) > 0) add(LG_FORCE_KERNEL_PAIRS, 1, 4, sl0, 0);
     for (int T = 1; T <= 32; T *= 2) add(LG_FORCE_KERNEL_ROWGROUP, T, 4, sl0, 0);
     if (s->precision == LG_PRECISION_MIXED)
         for (int mb = 4; mb <= 6; ++mb)

@@ -63,7 +63,8 @@ struct lg_system {
     double tuned_ms = 0.0;         // the autotuner's time per step of the handle's current choice
     int ham_slices = 0;            // mixed: Hamaker slices of the two-stream kernels (0: size rule)
     int contact_lanes = 2;         // mixed: lanes per row of the two-stream contact kernel (1 or 2)
-    // serving arena (lg_arena_create): a batch whose systems are slots; lattice point of each slot
+    // serving arena (lg_arena_create): a batch whose systems are slots; arena_lattice bounds an occupant's radius,
+    // slot_pos is where an empty slot's particles are parked
     bool arena = false;
     double arena_lattice = 0.0;
     std::vector<double> slot_pos;  // [3 * slots]
@@ -175,15 +176,15 @@ int lg_fail(int code, const char *fmt, ...);
 int64_t lg_handle_bytes(const lg_system_desc *d, int64_t n);
 
 // Serving slots (lg_engine.cpp), for the serving loop. An arena is a batch handle whose systems
-// are slots of fixed capacities (caps) on a lattice; a slot holds one request (its first n
+// are slots of fixed capacities (caps); a slot holds one request (its first n
 // particles) or nothing, and its other particles are inactive (no cell, no row, no motion). All
 // occupants advance in the same launches. lg_arena_import moves a standalone handle built from the
 // same template (the request after its construction force evaluation, at a rebuild boundary) into
 // slot q: state, bonds with their springs, pair rows with their springs (partner indices moved by
 // the slot's offset) and float-float origin; the occupant then evolves exactly as
 // the standalone handle would. lg_arena_clear empties a slot; lg_arena_read copies an occupant's
-// state (host arrays of 3n doubles, null: skipped). The caller keeps the arena at a rebuild
-// boundary and idle (synchronised) around imports and clears.
+// state (host arrays of 3n doubles, null: skipped). The caller keeps the arena idle (synchronised) around
+// imports and clears, and at a rebuild boundary around imports.
 int lg_arena_create(const lg_system_desc *tmpl, int64_t n_slots, const int64_t *caps, int device, lg_system **out);
 // A standalone handle whose device memory comes from the stream-ordered pool (lg_create otherwise).
 int lg_create_staged(const lg_system_desc *desc, const double *x0, const double *v0, int device, lg_system **out);
