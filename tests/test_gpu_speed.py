@@ -1,5 +1,7 @@
 """Costs that have to stay in proportion, as ratios of times taken on the same GPU one after another. The limits lie
 well above what is measured (stated beside each) and below what a wrong choice of kernel gave."""
+import time
+
 import pytest
 
 from libgran_gb300 import _abi as A
@@ -52,3 +54,27 @@ def test_unary_terms_run_beside_the_contacts():
     contacts waited for the unary terms to end)."""
     plain = _us(9000, A.LG_BINARY_CONTACT, A.LG_HAMAKER_LIMITED, 4.5)
     assert _us(9000, A.LG_BINARY_CONTACT, A.LG_HAMAKER_LIMITED, 4.5, body=True) <= 1.49 * plain
+
+
+def test_row_capacities_are_found_before_the_rows_are_allocated():
+    """A handle that works out its rows' capacity is created in 1.1 times the time of one that is given it (1.5 when its
+    rows were allocated twice)."""
+    mat = K.Material()
+    n = 65536
+    x0 = generate_aggregate(5, n, mat.r)
+
+    def create_time(cap):
+        d = K.make_desc(n, A.LG_BINARY_CONTACT, A.LG_HAMAKER_LIMITED, contact=mat.contact(), hamaker=mat.hamaker(),
+                        pairs=A.LG_PAIRS_VERLET, r_verlet=4.5 * mat.r, precision=A.LG_PRECISION_MIXED, max_neighbors=cap)
+        best = float("inf")
+        for _ in range(12):
+            t0 = time.perf_counter()
+            s = System(d, x0)
+            best = min(best, time.perf_counter() - t0)
+            longest = s.pair_stats()["max_row_length"]
+            s.close()
+        return best, longest
+
+    own, longest = create_time(0)
+    assert longest > 32  # (so that the rows outgrow the 48 slots that they would start with)
+    assert own <= 1.3 * create_time(int(1.5 * longest) + 1)[0]
