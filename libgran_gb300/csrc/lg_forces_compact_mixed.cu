@@ -6,13 +6,15 @@
 //                          contact candidates (near_owners, after each list build) are queued per block and
 //                          evaluated a warp at a time; each order's accelerations go to a record per
 //                          candidate, which the completion adds per row in entry order.
-//   forces_contacts_mixed  contact and bond pairs row by row: small lists, all pairs, and systems whose two
-//                          orders of a pair may break differently. Candidates are queued per warp (ballot
+//   forces_contacts_mixed  contact and bond pairs row by row: the lists whose candidates are too many for that
+//                          (near_scratch in lg_engine.cpp), all pairs, and systems whose two orders of a pair
+//                          may break differently. Candidates are queued per warp (ballot
 //                          order) and evaluated 32 at a time, folded per row in slot order into
 //                          float-float sums (MixedExtra::csum).
 //   forces_hamaker_mixed   Hamaker pairs over all slots, in windows of four slots held in registers, L
 //                          lanes per row; the windows' sums are added in the order that the slicing
 //                          defines. Runs beside the contact kernel (two streams).
+//   forces_hamaker_all     the same over all pairs of large systems, a lane per row.
 //   unary_mixed            facet and body terms (FP64), on a third stream.
 //   forces_finish_ff       completion inside a run of steps (no facets, no body term): the sums, the
 //                          end-of-step half kick, the next step's half kick and drift, all in

@@ -19,10 +19,10 @@
 //   pair_fold      adds each row's slot values in ascending slot order, exactly as the sequential row loop
 //                  does, then the half kick and, inside a run of steps, the next step's kick and drift.
 // Every slot is written by one thread and every sum has a fixed order, so results do not depend on
-// scheduling. Measured (graph-replayed steps, us): 32768 monomers, contact + limited Hamaker 438 -> 135
+// scheduling. Measured (graph-replayed steps with their list builds, us): 32768 monomers, contact + limited Hamaker 445 -> 132
 // (kernels 49 / 48 / 16; the kernel before evaluated both orders of every pair, one lane per row, 389);
-// 96 sintered aggregates (35,613 monomers) 480 -> 116; 5003 monomers, breaking bonds 190 -> 41; 256
-// monomers, all pairs 84 -> 34; 40 monomers, one step per call 37 -> 31.
+// 96 sintered aggregates (35,613 monomers) 469 -> 113; 5003 monomers, breaking bonds 189 -> 41; 256
+// monomers, all pairs 86 -> 34; 40 monomers, one step per call 37 -> 31 to 34.
 #include <algorithm>
 
 #include "lg_compact.cuh"

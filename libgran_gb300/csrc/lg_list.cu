@@ -2,9 +2,9 @@
 // spring carry. Compiled with --fmad=false (the list test is the reference's FP64 expression).
 //
 // What bounds it: launch and dependency latency in the sort's small kernels, instruction issue in the row
-// build. Measured for 32768 monomers / a batch of 381,000 in 1024 systems, us: sort 41 / 77 -> 19 / 63, row
-// build 83 / 987 -> 42 / 290. The sort takes four launches instead of nine; a batch's systems have grids of
-// their own (one grid over all of them spans the space between, so its cells were three list radii wide and
+// build. Measured for 32768 monomers / a batch of 376,000 in 1024 systems (cold caches), us: sort 37 / 90 -> 26 / 69,
+// row build 83 / 987 -> 61 / 296 (80 -> 34 warm). The sort takes four launches instead of nine; a batch's systems
+// have grids of their own (one grid over all of them spans the space between, so its cells were three list radii wide and
 // held 27 times the candidates); candidates come cell by cell with their positions, one load each, in runs
 // cut to the row's reach (94 a row instead of 172); eight lanes build a row instead of 32.
 #include <algorithm>
