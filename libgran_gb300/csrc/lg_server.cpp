@@ -393,7 +393,11 @@ extern "C" int lg_server_tick(lg_server *s, int32_t *n_active, int32_t *n_queued
     retire(s, done);
     s->active.swap(still);
     const int32_t retired = (int32_t)done.size();
-    // admissions at a rebuild boundary: the occupant's rows start with the arena's next build
+    // admissions at a rebuild boundary: the occupant's rows start with the arena's next build. An arena that emptied
+    // between two boundaries has nobody to carry to the next one and goes there at once (it would not step, and admit
+    // nobody, for ever).
+    if (s->arena && s->active.empty() && s->arena->step_index % s->rebuild_every != 0)
+        s->arena->step_index += s->rebuild_every - s->arena->step_index % s->rebuild_every;
     const bool boundary = !s->arena || (s->arena->step_index % s->rebuild_every) == 0;
     if (boundary) {
         for (auto it = s->queue.begin(); it != s->queue.end();) {

@@ -245,3 +245,35 @@ def test_fp64_pair_kernels_equal_rows_at_their_launch_lines(n, wall):
 def test_tuned_handles_hold_no_graph_of_another_shape(tmp_path):
     held, eager, replayed = (int(v) for v in _cpp(tmp_path, "tuned_graphs"))
     assert held == 0 and eager == replayed
+
+
+@PRECISIONS
+def test_a_server_emptied_between_boundaries_goes_on_admitting(precision):
+    """Every request of a wave ends between two list builds, with others queued behind it, and a later wave finds the
+    server idle there: each ends as its lone run does (FP64: the same bits)."""
+    mat = K.Material()
+    d = K.make_desc(1, A.LG_BINARY_SINTER, A.LG_HAMAKER_LIMITED, contact=mat.contact(), sinter=mat.sinter(),
+                    hamaker=mat.hamaker(), pairs=A.LG_PAIRS_VERLET, r_verlet=4.5 * mat.r, precision=precision,
+                    max_neighbors=96)
+    srv = Server(d, budget_bytes=4 * 10 ** 9, dt=mat.dt, rebuild_every=20)
+    srv.set_slots([128])
+    for wave in range(2):
+        jobs = [(60 + 20 * q, 7 + 19 * q) for q in range(3)]
+        states = [(generate_aggregate(90 + q, n, mat.r), generate_velocities(90 + wave, n, 0.1)) for q, (n, _) in enumerate(jobs)]
+        ids = [srv.submit(x, v, steps) for (x, v), (_, steps) in zip(states, jobs)]
+        for _ in range(100):
+            active, queued, _ = srv.tick()
+            if active == 0 and queued == 0:
+                break
+        for (n, steps), (x, v), q in zip(jobs, states, ids):
+            got = srv.poll(q, want_x=True)
+            assert got["state"] == A.LG_REQ_DONE, (wave, n)
+            d.n_part = n
+            s = System(d, x, v)
+            s.step(mat.dt, steps, 20)
+            want = s.get(A.LG_FIELD_X)
+            s.close()
+            if precision == A.LG_PRECISION_FP64:
+                assert np.array_equal(got["x"], want), (wave, n)
+            else:
+                assert H.rel_err(got["x"] - x, want - x) <= 1e-5, (wave, n)
