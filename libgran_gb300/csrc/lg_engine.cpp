@@ -519,8 +519,10 @@ static PairScratch pair_scratch(const lg_system *s) {
 //   1.05  520 monomers 12.3 / 13.1, 16000 15.3 / 16.5, 65536 31.6 / 37.4; alone 32768 15.4 / 16.6
 //   1.25  2000 15.4 / 13.7, 18000 19.1 / 18.5, 24000 20.7 / 21.4, 65536 38.8 / 41.3; alone 40000 20.4 / 19.0,
 //         49152 21.6 / 22.5
-//   1.5   16000 23.4 / 19.0, 65536 48.7 / 47.9, 300000 209.5 / 207.9, batch of 392000 211 / 235; alone 131072
-//         57.2 / 49.7, batch of 392000 137 / 159
+//   1.5   16000 23.4 / 19.0, 65536 48.7 / 47.9, 300000 209.5 / 207.9; alone 40000 22.9 / 20.1, 49152 24.4 / 24.4, 70000
+//         28.8 / 30.0, 80000 33.6 / 32.5, 131072 57.5 / 49.2
+//   1.5, batches of aggregates of 400, whose rows hold fewer candidates: 20000 20.4 / 19.9, 40000 28.0 / 29.4, 200000
+//         107.6 / 122.9; alone 20000 16.8 / 16.4, 40000 19.3 / 22.2, 200000 64.5 / 77.6
 //   2     32768 46.1 / 38.2, 65536 87.8 / 72.5
 // With facets, whose terms run beside it, the second line lies at 8192 (monomers on a wall, 4000 32.3 / 31.8, 8000
 // 33.7 / 33.7, 12000 35.5 / 36.1, 16000 37.3 / 37.9, 20000 40.3 / 41.6, 24000 40.8 / 42.0).
@@ -531,9 +533,13 @@ static NearScratch near_scratch(const lg_system *s) {
                                                                         : std::max(s->P.contact.r_part, s->P.sinter.r_part));
     const double q = s->r_near / reach;
     const bool ham = s->P.hamaker_model != LG_HAMAKER_NONE;
-    const int64_t few = ham ? 512 : 32768, some = !ham ? 49152 : s->P.n_facets > 0 ? 8192 : 24000;
-    const int64_t from = q <= 1.06 ? few : q <= 1.45 ? some : q <= 1.55 ? 200000 : INT64_MAX;
-    if (s->P.n < from) return R;
+    const int64_t n = s->P.n;
+    const bool batch = s->n_systems > 0;
+    bool once = false;
+    if (q <= 1.06) once = n >= (ham ? 512 : 32768);
+    else if (q <= 1.45) once = n >= (!ham ? 49152 : s->P.n_facets > 0 ? 8192 : 24000);
+    else if (q <= 1.55) once = batch ? n >= 40000 : ham ? n >= 200000 : n >= 49152 && n < 75000;
+    if (!once) return R;
     if (s->P.binary_model == LG_BINARY_BREAKING_SINTER && s->P.neck_mode == LG_NECK_REFERENCE_INDEXING) return R;
     double *base = s->pv[1 - s->pcur].xi;
     const int64_t slots = s->pv[0].cap * s->P.n;

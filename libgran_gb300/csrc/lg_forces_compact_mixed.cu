@@ -553,8 +553,8 @@ int mixed_hamaker_slices(int64_t n) {
 }
 
 // Monomers from which all pairs go to forces_hamaker_all. us a step, lanes along a row / lanes on rows, Hamaker pairs
-// only: limited form 1400 monomers 25.7 / 32.2, 2048 41.8 / 41.7, 2500 60.2 / 46.6, 4096 128 / 63, 8192 477 / 173;
-// full form 2048 42.0 / 45.2, 2500 61.1 / 54.4, 8192 475 / 315. (The kernel before these two, which queued the
+// only: limited form 1400 monomers 25.7 / 32.2, 2048 41.8 / 41.7, 2500 60.9 / 50.7, 4096 128 / 70, 8192 480 / 180;
+// full form 2048 42.0 / 45.2, 2500 61.3 / 55.0, 8192 477 / 319. (The kernel before these two, which queued the
 // pairs in range in shared memory, took 47, 81 and 275 for the limited form at 2048, 4096 and 8192.)
 constexpr int64_t kHamakerAllFrom = 2304;
 

@@ -280,11 +280,11 @@ constexpr int kFoldRows = 10;    // rows per block of pair_fold: three lanes eac
 constexpr int kFoldAhead = 16;   // slots whose pair terms a lane of pair_fold has in flight
 constexpr int kRowsAhead = 4;    // the same for pair_fold_rows
 // pair_fold_rows issues 125 FP64 instructions for 32 rows, pair_fold 30 for ten, in shorter chains, so it wins until
-// the rows fill the SMs' sub-partitions. us a step, pair_fold / pair_fold_rows: 12000 rows 46.3 / 51.4, 16384 65.6 /
-// 66.7, 20000 73.0 / 73.9, 26000 84.5 / 83.2, 32768 104.2 / 101.7. A body force takes a lane of ten or of 32 rows more:
-// 14000 60.2 / 60.9, 20000 81.1 / 77.3. Facets take much more of it: 8000 66.8 / 70.5, 9000 62.6 / 62.3, 10000 80.7 /
-// 70.6, 14000 97.4 / 77.8.
-static int64_t fold_rows_from(const Params &P) { return P.n_facets > 0 ? 9000 : P.ext_a ? 16384 : 23000; }
+// the rows fill the SMs' sub-partitions, and longer the longer they are. us a step, pair_fold / pair_fold_rows: aggregate
+// 12000 rows 53.3 / 59.2, 16384 65.5 / 67.4, 20000 72.5 / 73.7, 26000 84.1 / 82.8; chain 12000 32.4 / 33.1, 16384 39.8 / 38.4,
+// 20000 41.7 / 40.0. A body force takes a lane of ten or of 32 rows more: 14000 60.2 / 60.9, 20000 81.1 / 77.3. Facets
+// take much more of it: 8000 66.8 / 70.5, 9000 62.6 / 62.3, 10000 80.7 / 70.6, 14000 97.4 / 77.8.
+static int64_t fold_rows_from(const Params &P) { return P.n_facets > 0 ? 9000 : 16384; }
 // pair_contacts_split issues about 190 FP64 instructions for ten slots instead of 300 for 32, so it wins
 // while its warps (0.2 per particle in an aggregate) leave the FP64 units time. us a step, split / not: 256 particles
 // 25.1 / 31.8, 5000 34.3 / 39.2, 7000 37.6 / 40.6, 8000 41.6 / 43.2, 9000 48.9 / 47.2 (with a body force), 10000 47.9 / 45.0.
@@ -436,10 +436,11 @@ __global__ void __launch_bounds__(32) pair_fold_rows(Params P, StateView S, Pair
 }
 
 // Rows per block of owned slots: blocks enough for every SM, yet full batches of 32, and at most the 32 rows whose
-// partners fill a tile. us a step, 4 / 8 / 16 / 32 rows: 2000 particles 28.4 / 31.4 / 29.5 / 39.2, 3000 29.4 / 32.2 / 30.7 /
-// 39.5, 4000 32.1 / 33.2 / 31.6 / 40.0, 8000 49.6 / 46.7 / 43.1 / 50.3, 16384 76.0 / 69.6 / 64.9 / 66.8, 26000 103.5 / 89.7 /
-// 80.7 / 82.6, 32768 129.9 / 112.0 / 103.0 / 101.4.
-int32_t pair_block_rows(int64_t n) { return n >= 30000 ? 32 : n >= 3600 ? 16 : 4; }
+// partners fill a tile. us a step, 4 / 8 / 16 / 32 rows: aggregates of 2000 28.4 / 31.4 / 29.5 / 39.2, 3000 29.4 / 32.2 /
+// 30.7 / 39.5, 4000 32.1 / 33.2 / 31.6 / 40.0, 8000 49.6 / 46.7 / 43.1 / 50.3; 16 / 32 rows: 12000 45.9 / 53.3, 16384 63.3 /
+// 65.5, 20000 71.9 / 72.5, 30000 96.3 / 93.5, without Hamaker forces 12000 33.3 / 33.7, 16384 43.3 / 41.0, 30000 55.8 / 52.5;
+// 4 / 16 rows: chain of 2600 23.9 / 23.2, of 3300 24.6 / 23.5.
+int32_t pair_block_rows(int64_t n) { return n >= 16384 ? 32 : n >= 2500 ? 16 : 4; }
 
 void launch_pair_owners(int64_t n, const PairView &PV, const PairScratch &R, cudaStream_t st) {
     const unsigned blocks = (unsigned)((n + R.rb - 1) / R.rb);

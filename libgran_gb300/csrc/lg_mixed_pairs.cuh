@@ -348,20 +348,22 @@ __device__ __forceinline__ f3 window_sum(const MixedExtra &MX, float4 xh, float4
         }
     }
     f3 sum = fm(0.f, 0.f, 0.f);
-    bool in[kWin], any = false;
+    if (SPARSE) {
+        bool any = false;
+#pragma unroll
+        for (int u = 0; u < kWin; ++u) {
+            const float dx = xh.x - ph[u].x, dy = xh.y - ph[u].y, dz = xh.z - ph[u].z;
+            any = any || (j[u] >= 0 && fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= MX.near2);
+        }
+        if (!__any_sync(__activemask(), any)) return sum;
+    }
 #pragma unroll
     for (int u = 0; u < kWin; ++u) {
-        in[u] = j[u] >= 0;
+        bool on = j[u] >= 0;
         if (HM == LG_HAMAKER_LIMITED) {
             const float dx = xh.x - ph[u].x, dy = xh.y - ph[u].y, dz = xh.z - ph[u].z;
-            in[u] = in[u] && fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= MX.near2;
+            on = on && fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= MX.near2;
         }
-        any = any || in[u];
-    }
-    if (SPARSE && !__any_sync(__activemask(), any)) return sum;
-#pragma unroll
-    for (int u = 0; u < kWin; ++u) {
-        const bool on = in[u];
         const f3 a = hamaker_pair(HM, MX, xh, xl, ph[u], pl[u]);
         sum = fm(on ? __fadd_rn(sum.x, a.x) : sum.x, on ? __fadd_rn(sum.y, a.y) : sum.y,
                  on ? __fadd_rn(sum.z, a.z) : sum.z);

@@ -216,8 +216,8 @@ def test_staged_handles_take_what_they_need(tmp_path):
         assert chunk <= charged <= chunk + 2 ** 22
 
 
-@pytest.mark.parametrize("n,wall", [(3599, False), (3601, False), (8500, False), (8501, False), (22999, False),
-                                    (30001, False), (8999, True), (9001, True)], ids=str)
+@pytest.mark.parametrize("n,wall", [(2499, False), (2501, False), (8500, False), (8501, False), (16383, False),
+                                    (16385, False), (8999, True), (9001, True)], ids=str)
 def test_fp64_pair_kernels_equal_rows_at_their_launch_lines(n, wall):
     """The row kernel at one thread per row adds each row in index order, and so do the pair kernels, whatever their block
     shapes: the same bits."""

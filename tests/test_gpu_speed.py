@@ -42,7 +42,7 @@ def test_steps_do_not_jump_between_neighbouring_sizes():
 
 
 def test_all_pairs_out_of_range_cost_little():
-    """Of all pairs of 8192 monomers one in 500 is within the Hamaker cutoff: 0.55 times the time of the form without one
+    """Of all pairs of 8192 monomers one in 500 is within the Hamaker cutoff: 0.57 times the time of the form without one
     (1.0 when the time went into reading the partners)."""
     full = _us(8192, A.LG_BINARY_NONE, A.LG_HAMAKER_FULL, steps=4)
     assert _us(8192, A.LG_BINARY_NONE, A.LG_HAMAKER_LIMITED, steps=4) <= 0.8 * full
