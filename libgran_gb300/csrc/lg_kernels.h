@@ -10,8 +10,9 @@ namespace lg {
 // Cell grid of one system (a batch: one per system, their cells one after another from `base` on).
 struct GridDev {
     double lo[3];
-    float edge, inv_edge;  // cell width in y and z, and its inverse (in x: a quarter)
+    float edge, inv_edge;  // cell width across the lines of cells, and its inverse (along them: a quarter)
     float slack;           // uncertainty of the cell boundaries, in cells
+    int32_t turn;          // the axis that the lines follow (0: x); dim and the stored coordinates begin with it
     int32_t dim[3], base;
     float rv2_lo, rv2_hi;  // FP32 accept / reject bounds of the squared list radius
     float rn2_hi;          // FP32 bound of the squared near radius (contact candidates), < 0: none
