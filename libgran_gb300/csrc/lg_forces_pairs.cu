@@ -286,9 +286,11 @@ constexpr int kRowsAhead = 4;    // the same for pair_fold_rows
 // take much more of it: 8000 66.8 / 70.5, 9000 62.6 / 62.3, 10000 80.7 / 70.6, 14000 97.4 / 77.8.
 static int64_t fold_rows_from(const Params &P) { return P.n_facets > 0 ? 9000 : 16384; }
 // pair_contacts_split issues about 190 FP64 instructions for ten slots instead of 300 for 32, so it wins
-// while its warps (0.2 per particle in an aggregate) leave the FP64 units time. us a step, split / not: 256 particles
-// 25.1 / 31.8, 5000 34.3 / 39.2, 7000 37.6 / 40.6, 8000 41.6 / 43.2, 9000 48.9 / 47.2 (with a body force), 10000 47.9 / 45.0.
-constexpr int64_t kSplitUpTo = 8500;
+// while its warps (0.2 per particle in an aggregate) leave the FP64 units time, less of it the more the contacts slide,
+// roll and twist. us a step, split / not, spins of v / r: contacts with Hamaker forces 6100 46.3 / 44.6, 7130 49.5 / 45.4,
+// 8300 53.8 / 49.3; bonds without 6100 37.3 / 35.5, 8300 45.3 / 39.1; short queues gain beyond the line (contacts alone,
+// which fly apart: 6100 26.7 / 33.4, 8300 27.3 / 34.3). Below it: 256 particles 25.1 / 31.8, 5000 34.3 / 39.2, no spins.
+constexpr int64_t kSplitUpTo = 6000;
 
 // Small systems: lane 3 r + c of the first warp sums force component c of the block's row r in slot order,
 // one dependent chain per lane with the loads of slots kFoldAhead ahead issued between its additions (a
